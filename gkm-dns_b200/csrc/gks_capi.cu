@@ -190,11 +190,9 @@ gks::LaunchCfg persistent(gks_ctx *ctx, int kind, int dir, int variant, int mult
     if (gks::max_resident_blocks(kind, dir, ctx->precision, variant, c.block, &per_sm) != cudaSuccess || per_sm < 1)
         per_sm = 1;
     long long g = (long long)ctx->nsm * per_sm * mult;
-    // work items: window runs (x / y reconstruction variants 0-2), warp-sized
-    // z segments of 32 threads each (z reconstruction variants 0-2), else cells
-    const long long items = (kind == gks::K_RECON && variant < 3)
-                                ? (dir < 2 ? ctx->batch.wtotal : ctx->batch.ztotal * 32)
-                                : ctx->batch.total;
+    // threads: one per window run (x / y reconstruction), 32 per z line (z
+    // reconstruction), else one per cell
+    const long long items = gks::batch_items(ctx->batch, kind, dir) * (kind == gks::K_RECON && dir == 2 ? 32 : 1);
     const long long need = (items + c.block - 1) / c.block;
     if (g > need) g = need;
     if (g < 1) g = 1;
@@ -348,6 +346,19 @@ int ensure_pipe(gks_ctx *ctx, FieldHost &h)
     return GKS_OK;
 }
 
+// Run length of the windowed reconstruction over `lines` (count, interfaces
+// per line): the longest that leaves at least kWinItemsPerSm items per SM.
+int win_run_for(const gks_ctx *ctx, const std::vector<std::pair<long long, long long>> &lines)
+{
+    int run = gks::win_run(ctx->precision == GKS_MIXED ? 1 : 0);
+    for (; run > gks::kWinRunMin; run /= 2) {
+        long long items = 0;
+        for (const auto &l : lines) items += l.first * ((l.second + run - 1) / run);
+        if (items >= (long long)gks::kWinItemsPerSm * ctx->nsm) break;
+    }
+    return run;
+}
+
 // One stage over the physical planes [p0, p1) of the single field.
 int pipe_stage(gks_ctx *ctx, const FieldDev &d, int kind, int dir, long long p0, long long p1)
 {
@@ -357,13 +368,18 @@ int pipe_stage(gks_ctx *ctx, const FieldDev &d, int kind, int dir, long long p0,
     b.one = d; // this step's descriptor (spare state, per-sweep reconstruction buffers)
     gks::LaunchCfg c = ctx->cfg[kind][dir];
     long long per_plane = nc * nc; // cells
-    if (kind == gks::K_RECON && c.variant < 3) {
-        if (dir == 0) per_plane = (long long)d.nrun * nc; // window items (j, run, k)
-        else if (dir == 2) per_plane = nc * ((nc + 31) / 32); // z segments ((j, i), segment)
-        else c = persistent(ctx, kind, dir, c.variant + 3, 1); // y windows run along y: one interface per thread
-    }
+    if (kind == gks::K_RECON && dir == 0) per_plane = (long long)d.nrun * nc; // window items (j, run, k)
+    if (kind == gks::K_RECON && dir == 2) per_plane = nc;                     // z lines (j, i)
     b.lo = p0 * per_plane;
     b.hi = p1 * per_plane;
+    if (kind == gks::K_RECON && dir == 1) { // y windows run along y: the range itself is cut into runs
+        b.wy0 = (int)p0;
+        b.wy1 = (int)p1;
+        b.wrun = win_run_for(ctx, {{nc * nc, p1 - p0}});
+        b.lo = 0;
+        b.hi = nc * nc * ((p1 - p0 + b.wrun - 1) / b.wrun);
+        c.grid = (int)std::min<long long>((b.hi + c.block - 1) / c.block, (long long)ctx->nsm * 8);
+    }
     if (kind == gks::K_RECON) CK(gks::launch_recon(b, dir, ctx->precision, c, ctx->stream));
     else if (kind == gks::K_FLUX) CK(gks::launch_flux(b, dir, ctx->precision, c, ctx->stream));
     else CK(gks::launch_update(b, c, ctx->stream));
@@ -611,15 +627,10 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
     ctx->own_stream = true;
 
     ctx->fh.resize(nfields);
-    // run length of the windowed reconstruction: the longest that leaves the
-    // batch at least kWinItemsPerSm window items per SM
-    int run = gks::win_run(precision == GKS_MIXED ? 1 : 0);
-    for (; run > gks::kWinRunMin; run /= 2) {
-        long long items = 0;
-        for (int f = 0; f < nfields; ++f)
-            items += (long long)(slab ? slab + 6 : phys[f].nc) * phys[f].nc * ((phys[f].nc + run - 1) / run);
-        if (items >= (long long)gks::kWinItemsPerSm * ctx->nsm) break;
-    }
+    std::vector<std::pair<long long, long long>> lines;
+    for (int f = 0; f < nfields; ++f)
+        lines.push_back({(long long)(slab ? slab + 6 : phys[f].nc) * phys[f].nc, phys[f].nc});
+    const int run = win_run_for(ctx, lines);
     long long base = 0, wbase = 0, zbase = 0;
     const double pi = std::atan(1.0) * 4.0; // param.h:14
     for (int f = 0; f < nfields; ++f) {
@@ -674,9 +685,8 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
         d.nwin = (long long)ny * p.nc * d.nrun;
         d.wbase = wbase;
         wbase += (d.nwin + gks::kItemAlign - 1) / gks::kItemAlign * gks::kItemAlign;
-        d.nzseg = (long long)ny * p.nc * ((p.nc + 31) / 32);
         d.zbase = zbase;
-        zbase += d.nzseg;
+        zbase += (long long)ny * p.nc;
         d.nc = p.nc;
         // magic number for x / nc (round-up method): l = ceil(log2 nc),
         // m = floor(2^32 (2^l - nc) / nc) + 1, x / nc = (umulhi(x, m) + x) >> l
@@ -1325,7 +1335,7 @@ int gks_autotune(gks_ctx *ctx, int reps)
     const int mults[2] = {1, 2};
     for (int dir = 0; dir < 3 && rc == GKS_OK; ++dir) {
         for (int kind : {int(gks::K_RECON), int(gks::K_FLUX)}) {
-            const int nvar = kind == gks::K_RECON ? gks::kReconVariants : gks::kFluxVariants;
+            const int nvar = 3; // reconstruction variants 3-5 repeat 0-2
             // every candidate is timed in two interleaved rounds and keeps its
             // faster one, so that one disturbed measurement does not decide
             std::vector<gks::LaunchCfg> cand;

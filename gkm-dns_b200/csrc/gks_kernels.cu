@@ -112,17 +112,17 @@ __device__ __forceinline__ void store_tau(const FieldDev &f, unsigned c, const d
 __device__ __forceinline__ double temperature(const double W[5], double cT)
 {
     // (gam-1)(E/rho - |m|^2/(2 rho^2))/R, update.cpp:560
-    const double ri = __drcp_rn(W[0]);
+    const double ri = rcp_cubic(W[0]);
     const double ke = fma(W[1], W[1], fma(W[2], W[2], W[3] * W[3]));
     return cT * fma(-0.5 * ke, ri * ri, W[4] * ri);
 }
 
 // rho E from the reconstructed density, momentum and temperature
-// (update.cpp:618-619): rho T R/(gam-1) + |m|^2 / (2 rho), ri = 1/rho.
-__device__ __forceinline__ double energy(const double w[5], double T, double ri, double icT)
+// (update.cpp:618-619): rho T R/(gam-1) + |m|^2 / (2 rho).
+__device__ __forceinline__ double energy(const double w[4], double T, double icT)
 {
     const double ke = fma(w[1], w[1], fma(w[2], w[2], w[3] * w[3]));
-    return fma(w[0] * T, icT, (0.5 * ke) * ri);
+    return fma(w[0] * T, icT, (0.5 * ke) * rcp_cubic(w[0]));
 }
 
 // The reconstruction record of cell c: Wl[0..4] then Wr[0..4] as five
@@ -152,133 +152,59 @@ __device__ __forceinline__ void get_record(const double *rec, unsigned c, double
 }
 
 // ---------------------------------------------------------------------------
-// WENO of one interface from its 6-cell stencil s[0..5] (LLL .. RRR) and the
-// stencil's temperatures T[0..5] (used unless GKS_DIRECT_ENERGY)
-// (update.cpp:247, 502-625 / GPUupdate.cu:917-977).
+// The five reconstructed quantities of a cell are rho, the momenta and the
+// temperature (update.cpp:560-619) or, with GKS_DIRECT_ENERGY, rho E
+// (GPUupdate.cu:917-977).
 // ---------------------------------------------------------------------------
-template <int PREC, typename SG>
-__device__ __forceinline__ void recon_point(const SG &s, const double (&T)[6], bool direct, double icT, double wl[5],
-                                            double wr[5])
-{
-    if (PREC == 0) {
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            weno_pair<double>(s(0, q), s(1, q), s(2, q), s(3, q), s(4, q), s(5, q), kWenoEps, wl[q], wr[q]);
-        if (direct) {
-            weno_pair<double>(s(0, 4), s(1, 4), s(2, 4), s(3, 4), s(4, 4), s(5, 4), kWenoEps, wl[4], wr[4]);
-        } else {
-            double tl, tr;
-            weno_pair<double>(T[0], T[1], T[2], T[3], T[4], T[5], kWenoEps, tl, tr);
-            // E from the reconstructed temperature (update.cpp:618-619)
-            const double r = __drcp_rn(wl[0] * wr[0]); // one reciprocal for both densities
-            wl[4] = energy(wl, tl, wr[0] * r, icT);
-            wr[4] = energy(wr, tr, wl[0] * r, icT);
-        }
-    } else {
-        // mixed: WENO in FP32 on differences from the left cell, added back
-        // in FP64; components (0, 1) and (2, 3) as the two lanes of paired
-        // FP32 instructions, the fifth (energy or temperature) alone
-        const float epsf = float(kWenoEps);
-#pragma unroll
-        for (int q = 0; q < 4; q += 2) {
-            const double c0 = s(2, q), c1 = s(2, q + 1);
-            f2 v[6];
-#pragma unroll
-            for (int a = 0; a < 6; ++a) v[a] = f2(float(s(a, q) - c0), float(s(a, q + 1) - c1));
-            f2 dl, dr;
-            weno_pair<f2>(v[0], v[1], f2(0.0f), v[3], v[4], v[5], f2(epsf), dl, dr);
-            wl[q] = c0 + double(dl.v.x);
-            wr[q] = c0 + double(dr.v.x);
-            wl[q + 1] = c1 + double(dl.v.y);
-            wr[q + 1] = c1 + double(dr.v.y);
-        }
-        if (direct) {
-            const double c0 = s(2, 4);
-            float dl, dr;
-            weno_pair<float>(float(s(0, 4) - c0), float(s(1, 4) - c0), 0.0f, float(s(3, 4) - c0),
-                             float(s(4, 4) - c0), float(s(5, 4) - c0), epsf, dl, dr);
-            wl[4] = c0 + double(dl);
-            wr[4] = c0 + double(dr);
-        } else {
-            float dl, dr;
-            weno_pair<float>(float(T[0] - T[2]), float(T[1] - T[2]), 0.0f, float(T[3] - T[2]),
-                             float(T[4] - T[2]), float(T[5] - T[2]), epsf, dl, dr);
-            const double tl = T[2] + double(dl), tr = T[2] + double(dr);
-            const double r = __drcp_rn(wl[0] * wr[0]); // one reciprocal for both densities
-            wl[4] = energy(wl, tl, wr[0] * r, icT);
-            wr[4] = energy(wr, tr, wl[0] * r, icT);
-        }
-    }
-}
-
-// The stencil as a 6 x 5 array in registers.
-struct StencilRegs {
-    const double (&v)[6][5];
-    __device__ double operator()(int a, int q) const { return v[a][q]; }
-};
-
-template <int PREC>
-__device__ __forceinline__ void recon_point(const double (&s)[6][5], const double (&T)[6], bool direct, double icT,
+// FP64: both states of one cell from the quantities' six differences d around
+// it and their values g at it, rho E from the temperatures.
+__device__ __forceinline__ void cell_states(const double (&d)[5][6], const double (&g)[5], bool direct, double icT,
                                             double wl[5], double wr[5])
 {
-    recon_point<PREC>(StencilRegs{s}, T, direct, icT, wl, wr);
-}
-
-// ---------------------------------------------------------------------------
-// Reconstruction: Wl, Wr at the interface between cell c and its +1
-// neighbour along DIR, one interface per work item, the stencil read
-// straight from the state (used for the z sweep, where the lanes of a warp
-// are consecutive along the sweep and L1 serves the overlapping stencils).
-// ---------------------------------------------------------------------------
-template <int DIR, int PREC, int MINB>
-__global__ void __launch_bounds__(kReconBlock, MINB) k_recon(Batch b)
-{
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < b.hi; it += stride) {
-        const FieldDev &f = b.fields[field_of(b.fields, b.nfields, it)];
-        if (it - f.base >= f.ncell) continue; // alignment padding after the field
-        const Cell x = decode(unsigned(it - f.base), f);
-        unsigned idx[6];
 #pragma unroll
-        for (int a = 0; a < 6; ++a) idx[a] = along<DIR>(x, a - 2);
-        double s[6][5];
-#pragma unroll
-        for (int a = 0; a < 6; ++a)
-#pragma unroll
-            for (int q = 0; q < 5; ++q) s[a][q] = __ldg(f.W[q] + idx[a]);
-        if (DIR == 0) store_tau(f, x.c, s[2]);
-        const bool direct = (f.flags & GKS_DIRECT_ENERGY) != 0;
-        double T[6];
-        if (!direct) {
-#pragma unroll
-            for (int a = 0; a < 6; ++a) T[a] = temperature(s[a], f.cT);
-        }
-        double wl[5], wr[5];
-        recon_point<PREC>(s, T, direct, f.icT, wl, wr);
-        put_record(f.rec[DIR], x.c, wl, wr, f.ncell);
+    for (int q = 0; q < 5; ++q) {
+        double dl, dr;
+        weno_cell(d[q], dl, dr);
+        wl[q] = g[q] + dl;
+        wr[q] = g[q] + dr;
     }
+    if (direct) return;
+    wl[4] = energy(wl, wl[4], icT);
+    wr[4] = energy(wr, wr[4], icT);
 }
 
-// Field of z-segment item `it` (the last field whose segment range starts at or before it).
-__device__ __forceinline__ int field_of_zseg(const FieldDev *f, int n, long long it)
+// Mixed: both states of one interface from its stencil's quantities s(a, q),
+// a = 0 .. 5 (LLL .. RRR).  WENO in FP32 on differences from the left cell,
+// added back in FP64; quantities (0, 1) and (2, 3) as the two lanes of paired
+// FP32 instructions, the fifth alone.
+template <typename SG>
+__device__ __forceinline__ void interface_states(const SG &s, bool direct, double icT, double wl[5], double wr[5])
 {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (f[mid].zbase <= it) lo = mid;
-        else hi = mid - 1;
+    const float epsf = float(kWenoEps);
+#pragma unroll
+    for (int q = 0; q < 4; q += 2) {
+        const double c0 = s(2, q), c1 = s(2, q + 1);
+        f2 v[6];
+#pragma unroll
+        for (int a = 0; a < 6; ++a) v[a] = f2(float(s(a, q) - c0), float(s(a, q + 1) - c1));
+        f2 dl, dr;
+        weno_pair<f2>(v[0], v[1], f2(0.0f), v[3], v[4], v[5], f2(epsf), dl, dr);
+        wl[q] = c0 + double(dl.v.x);
+        wr[q] = c0 + double(dr.v.x);
+        wl[q + 1] = c1 + double(dl.v.y);
+        wr[q + 1] = c1 + double(dr.v.y);
     }
-    return lo;
+    const double c0 = s(2, 4);
+    float dl, dr;
+    weno_pair<float>(float(s(0, 4) - c0), float(s(1, 4) - c0), 0.0f, float(s(3, 4) - c0), float(s(4, 4) - c0),
+                     float(s(5, 4) - c0), epsf, dl, dr);
+    wl[4] = c0 + double(dl);
+    wr[4] = c0 + double(dr);
+    if (direct) return;
+    wl[4] = energy(wl, wl[4], icT);
+    wr[4] = energy(wr, wr[4], icT);
 }
 
-// ---------------------------------------------------------------------------
-// Reconstruction for the z sweep with a warp-staged segment: a work item is
-// one warp's 32 consecutive interfaces along z of one (j, i) line.  The lanes
-// load the 37 cells the segment's stencils span (one coalesced load per lane
-// and component, five lanes load the upper halo), compute each cell's
-// temperature once and stage cells and temperatures in the warp's own
-// shared-memory tile; each lane then reads its six-cell stencil from there.
-// ---------------------------------------------------------------------------
 // Asynchronous 8-byte copy global -> shared (cp.async), its groups and waits.
 __device__ __forceinline__ void cp_async8(double *smem, const double *gmem)
 {
@@ -292,64 +218,119 @@ __device__ __forceinline__ void cp_async_wait()
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-constexpr int kZSegWarps = kReconBlock / 32, kZSegCells = 32 + 5;
+// Field of z line `it` (the last field whose line range starts at or before it).
+__device__ __forceinline__ int field_of_zline(const FieldDev *f, int n, long long it)
+{
+    int lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const int mid = (lo + hi + 1) >> 1;
+        if (f[mid].zbase <= it) lo = mid;
+        else hi = mid - 1;
+    }
+    return lo;
+}
+
+// ---------------------------------------------------------------------------
+// Reconstruction for the z sweep: a work item is one (j, i) line, a warp walks
+// it in segments of 32 cells, one cell per lane.  The warp's shared-memory
+// tile holds the five quantities of the segment's cells and the three cells
+// either side: each segment brings 32 new cells (loaded into registers while
+// the segment before is computed, one coalesced load per lane and component,
+// one temperature per cell) and keeps the last six of the one before.
+// Mixed: a lane forms both states of the interface above its cell.  FP64: it
+// forms the two states of its cell; its left state meets the right state of
+// the next lane's cell: lane L writes the interface below its cell with the
+// left state handed over by lane L - 1, lane 0's from the last lane of the
+// segment before; the line's last interface takes the right state of cell 0,
+// kept from the first segment.
+// ---------------------------------------------------------------------------
+constexpr int kZLineWarps = kReconBlock / 32, kZLineCells = 32 + 6;
 
 template <int PREC, int MINB>
-__global__ void __launch_bounds__(kReconBlock, MINB) k_recon_zseg(Batch b)
+__global__ void __launch_bounds__(kReconBlock, MINB) k_recon_zline(Batch b)
 {
-    __shared__ double tiles[kZSegWarps][6][kZSegCells];
+    __shared__ double tiles[kZLineWarps][5][kZLineCells];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    double (*tile)[kZSegCells] = tiles[wid];
-    const long long stride = (long long)gridDim.x * kZSegWarps;
-    for (long long it = b.lo + (long long)blockIdx.x * kZSegWarps + wid; it < b.hi; it += stride) {
-        const FieldDev &f = b.fields[field_of_zseg(b.fields, b.nfields, it)];
-        const long long loc = it - f.zbase; // < nzseg: segment ranges are contiguous
-        const int nc = f.nc, nseg = (nc + 31) >> 5;
-        const long long line = loc / nseg;
-        const int k0 = int(loc - line * nseg) << 5;
-        const unsigned lbase = unsigned(line) * unsigned(nc); // cell (j, i, 0)
+    double (*tile)[kZLineCells] = tiles[wid];
+    const long long stride = (long long)gridDim.x * kZLineWarps;
+    for (long long it = b.lo + (long long)blockIdx.x * kZLineWarps + wid; it < b.hi; it += stride) {
+        const FieldDev &f = b.fields[field_of_zline(b.fields, b.nfields, it)];
+        const int nc = f.nc;
+        const unsigned lbase = unsigned(it - f.zbase) * unsigned(nc); // cell (j, i, 0)
         const bool direct = (f.flags & GKS_DIRECT_ENERGY) != 0;
-        // stage cells k0-2 .. k0+34 (those the active lanes' stencils reach:
-        // k0-2 .. min(k0+34, nc+2), so each index wraps at most once) and their
-        // temperatures; lane l takes cells l and l + 32, all ten loads issued at once
-        const int nh = min(kZSegCells, nc - k0 + 5);
-        const int h1 = lane + 32;
-        const bool one = lane < nh, two = h1 < nh;
-        double w[5], v[5];
-        {
-            const unsigned c0 = lbase + unsigned(wrap(k0 - 2 + (one ? lane : 0), nc));
-            const unsigned c1 = lbase + unsigned(wrap(k0 - 2 + (two ? h1 : 0), nc));
+        const double cT = f.cT, icT = f.icT;
+        double w[5];
+        auto load = [&](int k) { // cell k of the line, -3 <= k < nc + 3
+            const unsigned c = lbase + unsigned(wrap(k, nc));
 #pragma unroll
-            for (int q = 0; q < 5; ++q) {
-                w[q] = one ? __ldg(f.W[q] + c0) : 0.0;
-                v[q] = two ? __ldg(f.W[q] + c1) : 0.0;
+            for (int q = 0; q < 5; ++q) w[q] = __ldg(f.W[q] + c);
+        };
+        auto put = [&](int col) {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) tile[q][col] = w[q];
+            tile[4][col] = direct ? w[4] : temperature(w, cT);
+        };
+        if (lane < 6) { // cells -3 .. 2
+            load(lane - 3);
+            put(lane);
+        }
+        if (lane < nc) load(lane + 3);
+        double first[5], carry[5]; // lane 0: right state of cell 0, left state of the cell before the segment
+#pragma unroll
+        for (int q = 0; q < 5; ++q) first[q] = carry[q] = 0.0;
+        for (int k0 = 0; k0 < nc; k0 += 32) {
+            const int k = k0 + lane; // this lane's cell, column lane + 3
+            if (k < nc) put(lane + 6);
+            __syncwarp();
+            if (k + 32 < nc) load(k + 35);
+            if constexpr (PREC == 0) {
+                double wl[5], wr[5];
+                if (k < nc) {
+                    double d[5][6], g[5];
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) {
+                        double lo = tile[q][lane];
+#pragma unroll
+                        for (int a = 0; a < 6; ++a) {
+                            const double hi = tile[q][lane + a + 1];
+                            d[q][a] = hi - lo;
+                            lo = hi;
+                            if (a == 2) g[q] = hi;
+                        }
+                    }
+                    cell_states(d, g, direct, icT, wl, wr);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) wl[q] = wr[q] = 0.0;
+                }
+                // lane L takes the left state of lane L - 1, lane 0 the segment's last
+                const int src = lane ? lane - 1 : min(31, nc - 1 - k0);
+                double left[5];
+#pragma unroll
+                for (int q = 0; q < 5; ++q) {
+                    const double t = __shfl_sync(0xffffffffu, wl[q], src);
+                    left[q] = lane ? t : carry[q];
+                    carry[q] = t;
+                }
+                if (k == 0) {
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) first[q] = wr[q];
+                } else if (k < nc) {
+                    put_record(f.rec[2], lbase + unsigned(k - 1), left, wr, f.ncell);
+                }
+            } else if (k < nc) {
+                double wl[5], wr[5];
+                interface_states([&](int a, int q) -> double { return tile[q][lane + a + 1]; }, direct, icT, wl, wr);
+                put_record(f.rec[2], lbase + unsigned(k), wl, wr, f.ncell);
             }
-        }
-        if (one) {
+            __syncwarp();
+            if (lane < 6) { // the last six cells become the first six of the next segment
 #pragma unroll
-            for (int q = 0; q < 5; ++q) tile[q][lane] = w[q];
-            tile[5][lane] = direct ? 0.0 : temperature(w, f.cT);
-        }
-        if (two) {
-#pragma unroll
-            for (int q = 0; q < 5; ++q) tile[q][h1] = v[q];
-            tile[5][h1] = direct ? 0.0 : temperature(v, f.cT);
-        }
-        __syncwarp();
-        const int k = k0 + lane;
-        if (k < nc) {
-            double s[6][5], T[6];
-#pragma unroll
-            for (int a = 0; a < 6; ++a) {
-#pragma unroll
-                for (int q = 0; q < 5; ++q) s[a][q] = tile[q][lane + a];
-                T[a] = tile[5][lane + a];
+                for (int q = 0; q < 5; ++q) tile[q][lane] = tile[q][lane + 32];
             }
-            double wl[5], wr[5];
-            recon_point<PREC>(s, T, direct, f.icT, wl, wr);
-            put_record(f.rec[2], lbase + unsigned(k), wl, wr, f.ncell);
+            __syncwarp();
         }
-        __syncwarp();
+        if (PREC == 0 && lane == 0) put_record(f.rec[2], lbase + unsigned(nc - 1), carry, first, f.ncell);
     }
 }
 
@@ -367,96 +348,168 @@ __device__ __forceinline__ int field_of_win(const FieldDev *f, int n, long long 
 
 // ---------------------------------------------------------------------------
 // Reconstruction for the x (DIR 0) and y (DIR 1) sweeps with a sliding
-// window: a work item is a run of f.run consecutive interfaces along the
-// sweep at one (transverse line, k); the lanes of a warp take consecutive
-// k, so every load is coalesced.  The window moves by one cell per
-// interface: one new cell (five loads) and one temperature per interface
-// instead of thirty loads and six temperatures.  The cells live in a ring of
+// window: a work item is a run of consecutive interfaces along the sweep at
+// one (transverse line, k); the lanes of a warp take consecutive k, so every
+// load is coalesced.  Cells arrive by asynchronous copies in a ring of
 // kWinRing slots in the thread's own part of shared memory
-// ([slot][component][thread], no bank conflicts) -- the six stencil cells and
-// the kWinPrefetch cells beyond them, which arrive by asynchronous copies so
-// that their latency overlaps the WENO of the interfaces before them -- and
-// only the six temperatures stay in registers (about 40 fewer registers than
-// with the window in registers).  Item order: k
-// fastest, then run, then the transverse line.  The loop is kept rolled
-// (FP64) or unrolled twice (mixed).
+// ([slot][component][thread], no bank conflicts) a few cells ahead of their
+// use.  Mixed: each interface reads its six-cell stencil from the ring, the
+// six temperatures stay in registers.  FP64: a run of n interfaces evaluates
+// n + 1 cells; the window is the six differences of each quantity in
+// registers, which slide by one cell (five loads, one temperature, five
+// differences per cell), and the left state of a cell waits one cell for the
+// right state of the next, with which it leaves as one record.  Item order: k
+// fastest, then run, then the transverse line.  A launch over a range of y
+// planes (Batch::wy0 .. wy1, one field) cuts that range into runs of
+// Batch::wrun interfaces.
 // ---------------------------------------------------------------------------
-constexpr int kWinPrefetch = 2; // 2, 4 and 8 measured within 1 %
-constexpr int kWinRing = 8;     // ring slots per thread: 6 stencil cells + the cells in flight
-
+constexpr int kWinRing = 8;
+// Cells in flight: the ring holds cells p .. p + 3 of the FP64 window, p - 2 ..
+// p + 3 of the mixed one, besides them.
+__host__ __device__ constexpr int win_prefetch(int prec) { return prec == 0 ? 3 : 2; }
 
 template <int DIR, int PREC, int MINB>
 __global__ void __launch_bounds__(kReconBlock, MINB) k_recon_win(Batch b)
 {
-    constexpr int PF = kWinPrefetch, NR = kWinRing;
-    static_assert(NR >= 5 + PF && (NR & (NR - 1)) == 0, "the ring holds the window and the cells in flight");
+    constexpr int PF = win_prefetch(PREC), NR = kWinRing;
+    static_assert(NR >= (PREC == 0 ? 4 : 6) + PF && (NR & (NR - 1)) == 0, "the ring holds the live cells and those in flight");
     __shared__ double ring[NR][5][kReconBlock];
     const int tid = threadIdx.x;
     static_assert(DIR == 0 || DIR == 1, "windowed reconstruction is for the x and y sweeps");
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < b.hi; it += stride) {
         const FieldDev &f = b.fields[field_of_win(b.fields, b.nfields, it)];
-        const long long loc = it - f.wbase;
-        if (loc >= f.nwin) continue; // alignment padding after the field
+        const bool ranged = DIR == 1 && b.wy1 > 0;
+        const long long loc = ranged ? it : it - f.wbase;
+        if (!ranged && loc >= f.nwin) continue; // alignment padding after the field
         const int nc = f.nc;
         const unsigned u = unsigned(loc);
         const unsigned rest = div_nc(u, f);
         const int k = int(u - rest * unsigned(nc));
-        const int line = int(rest / unsigned(f.nrun));
-        const int RUN = f.run;
-        const int s0 = int(rest - unsigned(line) * unsigned(f.nrun)) * RUN;
-        // cell (line, sweep position p, k): x sweep (j, i, k), y sweep (j = p, i = line)
+        const int run = ranged ? b.wrun : f.run;
+        const int nrun = ranged ? (b.wy1 - b.wy0 + run - 1) / run : f.nrun;
+        const int line = int(rest / unsigned(nrun));
+        const int s0 = int(rest - unsigned(line) * unsigned(nrun)) * run + (ranged ? b.wy0 : 0);
+        const int s1 = min(s0 + run, ranged ? b.wy1 : nc); // interfaces [s0, s1)
+        // cell (line, sweep position p, k): x sweep (j, i, k), y sweep (j = p, i =
+        // line).  A slab's y index does not wrap: the first cell of the first run
+        // and the last cell of the last one lie beyond its stored planes; they
+        // enter only the states that are not kept, and read the top plane instead
         const unsigned step = DIR == 0 ? unsigned(nc) : unsigned(nc) * unsigned(nc);
         const unsigned lbase = DIR == 0 ? unsigned(line) * unsigned(nc) * unsigned(nc) + unsigned(k)
                                         : unsigned(line) * unsigned(nc) + unsigned(k);
-        auto cell = [&](int p) -> unsigned { return lbase + unsigned(wrap(p, DIR == 0 ? nc : f.nyw)) * step; };
+        const int nw = DIR == 0 ? nc : f.nyw, top = DIR == 0 ? nc - 1 : f.ny - 1;
+        auto cell = [&](int p) -> unsigned { return lbase + unsigned(max(0, min(wrap(p, nw), top))) * step; };
         const bool direct = (f.flags & GKS_DIRECT_ENERGY) != 0;
-        // cells of the run's stencils: s0 - 2 .. last (unwrapped, at most nc + 2),
-        // cell pc in ring slot pc mod NR, one copy group per cell (empty past the run)
-        const int last = min(s0 + RUN, nc) + 2;
+        const double cT = f.cT, icT = f.icT;
+        // cells up to s1 + 3 (mixed: s1 + 2), cell pc in ring slot pc mod NR, one copy
+        // group per cell (empty past the run)
+        const int pend = s1 + (PREC == 0 ? 3 : 2);
         auto fetch = [&](int pc) {
-            if (pc <= last) {
+            if (pc <= pend) {
                 const unsigned c = cell(pc);
 #pragma unroll
                 for (int q = 0; q < 5; ++q) cp_async8(&ring[pc & (NR - 1)][q][tid], f.W[q] + c);
             }
             cp_async_commit();
         };
-        auto temp_of = [&](int pc) -> double {
+        // the five quantities of cell pc
+        auto quantities = [&](int pc, double (&g)[5]) {
             double w[5];
 #pragma unroll
             for (int q = 0; q < 5; ++q) w[q] = ring[pc & (NR - 1)][q][tid];
-            return temperature(w, f.cT);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) g[q] = w[q];
+            g[4] = direct ? w[4] : temperature(w, cT);
         };
+        if constexpr (PREC == 0) {
+            double d[5][6];
+            double last[5]; // quantities of cell p + 3 (the newest)
+            double T[4];    // fifth quantity of cells p .. p + 3
 #pragma unroll
-        for (int d = 0; d < 5 + PF; ++d) fetch(s0 - 2 + d);
-        cp_async_wait<PF>(); // the five first window cells have landed
-        double T[6];
+            for (int a = 0; a < 1 + PF; ++a) fetch(s0 - 3 + a);
+            cp_async_wait<PF>();
+            quantities(s0 - 3, last);
 #pragma unroll
-        for (int a = 0; a < 5; ++a) T[a + 1] = direct ? 0.0 : temp_of(s0 - 2 + a);
-        constexpr int UNROLL = PREC == 0 ? 1 : 2;
-#pragma unroll UNROLL
-        for (int r = 0; r < RUN; ++r) {
-            const int p = s0 + r;
-            if (p >= nc) break;
+            for (int a = 1; a < 6; ++a) {
+                fetch(s0 - 3 + a + PF);
+                cp_async_wait<PF>();
+                double g[5];
+                quantities(s0 - 3 + a, g);
 #pragma unroll
-            for (int a = 0; a < 5; ++a) T[a] = T[a + 1];
-            cp_async_wait<PF - 1>(); // cell p + 3 (issued PF groups ago) has landed
-            T[5] = direct ? 0.0 : temp_of(p + 3);
-            const auto sg = [&](int a, int q) -> double { return ring[(p - 2 + a) & (NR - 1)][q][tid]; };
-            double wl[5], wr[5];
-            recon_point<PREC>(sg, T, direct, f.icT, wl, wr);
-            const unsigned c = cell(p);
-            if (DIR == 0) {
-                double w[5];
-#pragma unroll
-                for (int q = 0; q < 5; ++q) w[q] = sg(2, q);
-                store_tau(f, c, w);
+                for (int q = 0; q < 5; ++q) {
+                    d[q][a] = g[q] - last[q];
+                    last[q] = g[q];
+                }
+                if (a >= 3) T[a - 2] = g[4];
             }
-            put_record(f.rec[DIR], c, wl, wr, f.ncell);
-            // cell p + 3 + PF takes the slot of cell p + 3 + PF - NR, which no
-            // stencil from here on reads (it lies below p - 2 for NR >= 5 + PF)
-            fetch(p + 3 + PF);
+            double left[5];
+#pragma unroll 1
+            for (int p = s0; p <= s1; ++p) {
+                // cell p + 3 + PF takes the slot of cell p + 3 + PF - NR, which lies below p
+                fetch(p + 3 + PF);
+                cp_async_wait<PF>(); // cell p + 3 has landed
+                double g[5];
+                quantities(p + 3, g);
+#pragma unroll
+                for (int q = 0; q < 5; ++q) {
+#pragma unroll
+                    for (int a = 0; a < 5; ++a) d[q][a] = d[q][a + 1];
+                    d[q][5] = g[q] - last[q];
+                    last[q] = g[q];
+                }
+                T[0] = T[1];
+                T[1] = T[2];
+                T[2] = T[3];
+                T[3] = g[4];
+                double wc[5];
+#pragma unroll
+                for (int q = 0; q < 4; ++q) g[q] = wc[q] = ring[p & (NR - 1)][q][tid];
+                g[4] = T[0];
+                double wl[5], wr[5];
+                cell_states(d, g, direct, icT, wl, wr);
+                if (DIR == 0 && p < s1) {
+                    wc[4] = ring[p & (NR - 1)][4][tid];
+                    store_tau(f, cell(p), wc);
+                }
+                if (p > s0) put_record(f.rec[DIR], cell(p - 1), left, wr, f.ncell);
+#pragma unroll
+                for (int q = 0; q < 5; ++q) left[q] = wl[q];
+            }
+        } else {
+#pragma unroll
+            for (int a = 0; a < 5 + PF; ++a) fetch(s0 - 2 + a);
+            cp_async_wait<PF>(); // the five first window cells have landed
+            double T[6];
+#pragma unroll
+            for (int a = 0; a < 5; ++a) {
+                double g[5];
+                quantities(s0 - 2 + a, g);
+                T[a + 1] = g[4];
+            }
+#pragma unroll 2
+            for (int p = s0; p < s1; ++p) {
+#pragma unroll
+                for (int a = 0; a < 5; ++a) T[a] = T[a + 1];
+                cp_async_wait<PF - 1>(); // cell p + 3 (issued PF groups ago) has landed
+                double g[5];
+                quantities(p + 3, g);
+                T[5] = g[4];
+                const auto sg = [&](int a, int q) -> double { return q < 4 ? ring[(p - 2 + a) & (NR - 1)][q][tid] : T[a]; };
+                double wl[5], wr[5];
+                interface_states(sg, direct, icT, wl, wr);
+                const unsigned c = cell(p);
+                if (DIR == 0) {
+                    double w[5];
+#pragma unroll
+                    for (int q = 0; q < 5; ++q) w[q] = ring[p & (NR - 1)][q][tid];
+                    store_tau(f, c, w);
+                }
+                put_record(f.rec[DIR], c, wl, wr, f.ncell);
+                // cell p + 3 + PF takes the slot of cell p + 3 + PF - NR, which no
+                // stencil from here on reads (it lies below p - 2)
+                fetch(p + 3 + PF);
+            }
         }
         cp_async_wait<0>(); // nothing in flight into the ring before the next item
     }
@@ -1119,23 +1172,23 @@ cudaError_t occ(KernelT k, int block, int *n)
 }
 
 // Register-cap variants: reconstruction blocks of 128 threads at 3 / 4 / 5
-// resident blocks per SM (launch bounds; 168 / 128 / 96 registers), each in
-// the windowed and the one-interface form; flux blocks of 64 threads at
-// explicit caps of 200 / 168 / 128 registers (5 / 6 / 8 resident blocks).  A
-// launch bound of 5 blocks of 64 threads would not give the 200: the compiler
-// rounds the resident warps up to a multiple of four and caps at 168, as for
-// 6 blocks.  The tuner picks one variant per kernel, precision and sweep.
-// Every variant gives bit-identical results.
+// resident blocks per SM (launch bounds; 168 / 128 / 96 registers), numbered
+// 0-2 and again 3-5 (pinned configurations of either number stay valid); flux
+// blocks of 64 threads at explicit caps of 200 / 168 / 128 registers (5 / 6 /
+// 8 resident blocks).  A launch bound of 5 blocks of 64 threads would not give
+// the 200: the compiler rounds the resident warps up to a multiple of four
+// and caps at 168, as for 6 blocks.  The tuner picks one variant per kernel,
+// precision and sweep.  Every variant gives bit-identical results.
 constexpr int kReconMinb[3] = {3, 4, 5};
 constexpr int kFluxRegs[kFluxVariants] = {200, 168, 128};
 
 // The item range of a launch (all items of its kind when b.hi < 0) and the
 // blocks it needs: at most cfg.grid, no more than the range fills.
-Batch resolve_range(Batch b, int kind, int dir, int variant)
+Batch resolve_range(Batch b, int kind, int dir)
 {
     if (b.hi < 0) {
         b.lo = 0;
-        b.hi = batch_items(b, kind, dir, variant);
+        b.hi = batch_items(b, kind, dir);
     }
     return b;
 }
@@ -1146,35 +1199,25 @@ int range_grid(int grid, long long items, int items_per_block)
     return int(std::max(1LL, std::min((long long)grid, need)));
 }
 
-// Reconstruction variants: 0-2 the windowed kernel (x, y sweeps) or the
-// warp-staged segment kernel (z sweep) at the three register caps, 3-5 the
-// one-interface-per-thread kernel at the same caps.
 template <int DIR, int PREC>
 cudaError_t recon_go(Batch b, LaunchCfg cfg, cudaStream_t st)
 {
-    b = resolve_range(b, K_RECON, DIR, cfg.variant);
+    b = resolve_range(b, K_RECON, DIR);
     if (b.hi <= b.lo) return cudaSuccess;
     const long long items = b.hi - b.lo;
-    if (DIR < 2 && cfg.variant < 3) {
-        const int g = range_grid(cfg.grid, items, cfg.block);
-        switch (cfg.variant) {
-        case 1: k_recon_win<DIR < 2 ? DIR : 0, PREC, kReconMinb[1]><<<g, cfg.block, 0, st>>>(b); break;
-        case 2: k_recon_win<DIR < 2 ? DIR : 0, PREC, kReconMinb[2]><<<g, cfg.block, 0, st>>>(b); break;
-        default: k_recon_win<DIR < 2 ? DIR : 0, PREC, kReconMinb[0]><<<g, cfg.block, 0, st>>>(b); break;
-        }
-    } else if (DIR == 2 && cfg.variant < 3) {
-        const int g = range_grid(cfg.grid, items, kZSegWarps);
-        switch (cfg.variant) {
-        case 1: k_recon_zseg<PREC, kReconMinb[1]><<<g, cfg.block, 0, st>>>(b); break;
-        case 2: k_recon_zseg<PREC, kReconMinb[2]><<<g, cfg.block, 0, st>>>(b); break;
-        default: k_recon_zseg<PREC, kReconMinb[0]><<<g, cfg.block, 0, st>>>(b); break;
-        }
-    } else {
+    if constexpr (DIR < 2) {
         const int g = range_grid(cfg.grid, items, cfg.block);
         switch (cfg.variant % 3) {
-        case 1: k_recon<DIR, PREC, kReconMinb[1]><<<g, cfg.block, 0, st>>>(b); break;
-        case 2: k_recon<DIR, PREC, kReconMinb[2]><<<g, cfg.block, 0, st>>>(b); break;
-        default: k_recon<DIR, PREC, kReconMinb[0]><<<g, cfg.block, 0, st>>>(b); break;
+        case 1: k_recon_win<DIR, PREC, kReconMinb[1]><<<g, cfg.block, 0, st>>>(b); break;
+        case 2: k_recon_win<DIR, PREC, kReconMinb[2]><<<g, cfg.block, 0, st>>>(b); break;
+        default: k_recon_win<DIR, PREC, kReconMinb[0]><<<g, cfg.block, 0, st>>>(b); break;
+        }
+    } else {
+        const int g = range_grid(cfg.grid, items, kZLineWarps);
+        switch (cfg.variant % 3) {
+        case 1: k_recon_zline<PREC, kReconMinb[1]><<<g, cfg.block, 0, st>>>(b); break;
+        case 2: k_recon_zline<PREC, kReconMinb[2]><<<g, cfg.block, 0, st>>>(b); break;
+        default: k_recon_zline<PREC, kReconMinb[0]><<<g, cfg.block, 0, st>>>(b); break;
         }
     }
     return cudaGetLastError();
@@ -1183,7 +1226,7 @@ cudaError_t recon_go(Batch b, LaunchCfg cfg, cudaStream_t st)
 template <int DIR, int PREC>
 cudaError_t flux_go(Batch b, LaunchCfg cfg, cudaStream_t st)
 {
-    b = resolve_range(b, K_FLUX, DIR, cfg.variant);
+    b = resolve_range(b, K_FLUX, DIR);
     if (b.hi <= b.lo) return cudaSuccess;
     const int g = range_grid(cfg.grid, b.hi - b.lo, cfg.block);
     switch (cfg.variant) {
@@ -1197,21 +1240,16 @@ cudaError_t flux_go(Batch b, LaunchCfg cfg, cudaStream_t st)
 template <int DIR, int PREC>
 cudaError_t occ_kind(int kind, int variant, int block, int *n)
 {
-    if (kind == K_RECON && DIR < 2 && variant < 3) {
-        constexpr int D = DIR < 2 ? DIR : 0;
-        if (variant == 1) return occ(k_recon_win<D, PREC, kReconMinb[1]>, block, n);
-        if (variant == 2) return occ(k_recon_win<D, PREC, kReconMinb[2]>, block, n);
-        return occ(k_recon_win<D, PREC, kReconMinb[0]>, block, n);
-    }
-    if (kind == K_RECON && DIR == 2 && variant < 3) {
-        if (variant == 1) return occ(k_recon_zseg<PREC, kReconMinb[1]>, block, n);
-        if (variant == 2) return occ(k_recon_zseg<PREC, kReconMinb[2]>, block, n);
-        return occ(k_recon_zseg<PREC, kReconMinb[0]>, block, n);
-    }
     if (kind == K_RECON) {
-        if (variant % 3 == 1) return occ(k_recon<DIR, PREC, kReconMinb[1]>, block, n);
-        if (variant % 3 == 2) return occ(k_recon<DIR, PREC, kReconMinb[2]>, block, n);
-        return occ(k_recon<DIR, PREC, kReconMinb[0]>, block, n);
+        if constexpr (DIR < 2) {
+            if (variant % 3 == 1) return occ(k_recon_win<DIR, PREC, kReconMinb[1]>, block, n);
+            if (variant % 3 == 2) return occ(k_recon_win<DIR, PREC, kReconMinb[2]>, block, n);
+            return occ(k_recon_win<DIR, PREC, kReconMinb[0]>, block, n);
+        } else {
+            if (variant % 3 == 1) return occ(k_recon_zline<PREC, kReconMinb[1]>, block, n);
+            if (variant % 3 == 2) return occ(k_recon_zline<PREC, kReconMinb[2]>, block, n);
+            return occ(k_recon_zline<PREC, kReconMinb[0]>, block, n);
+        }
     }
     if (variant == 1) return occ(k_flux<DIR, PREC, kFluxRegs[1]>, block, n);
     if (variant == 2) return occ(k_flux<DIR, PREC, kFluxRegs[2]>, block, n);
@@ -1241,7 +1279,7 @@ cudaError_t launch_flux(const Batch &b, int dir, int prec, LaunchCfg cfg, cudaSt
 
 cudaError_t launch_update(const Batch &batch, LaunchCfg cfg, cudaStream_t st)
 {
-    const Batch b = resolve_range(batch, K_UPDATE, 0, 0);
+    const Batch b = resolve_range(batch, K_UPDATE, 0);
     if (b.hi <= b.lo) return cudaSuccess;
     k_update<<<range_grid(cfg.grid, b.hi - b.lo, cfg.block), cfg.block, 0, st>>>(b);
     return cudaGetLastError();

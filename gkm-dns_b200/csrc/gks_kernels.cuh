@@ -38,8 +38,7 @@ struct FieldDev {
     long long nwin;   // window items: nc^2 * nrun
     int run;          // interfaces per window item (the same for every field of a batch)
     int nrun;         // runs per line: ceil(nc / run)
-    long long zbase;  // first z-segment item of this field (z reconstruction; one warp per item)
-    long long nzseg;  // z segments: nc^2 * ceil(nc / 32)
+    long long zbase;  // first z-line item of this field (z reconstruction; one warp per line)
     int nc;           // cells per edge along x and z (and of the whole field along y)
     int ny;           // planes stored along y: nc, or a slab's interior planes + 6
     int nyw;          // modulus of the y-index wrap: nc, or kNoWrap for a slab (its ghosts are stored)
@@ -84,18 +83,22 @@ struct Batch {
     int nfields;
     long long total;  // end of the last field's item range
     long long wtotal; // end of the last field's window item range
-    long long ztotal; // end of the last field's z-segment item range
+    long long ztotal; // end of the last field's z-line item range
     int *err;         // device error word (bit 0: non-finite / non-positive state after update)
     // work items a launch processes: [lo, hi) of the launched kernel's item
     // space; hi < 0 means all of them (the launchers fill the range in)
     long long lo = 0, hi = -1;
+    // y reconstruction over the interfaces of planes [wy0, wy1) of the one field
+    // (wy1 > 0), in runs of wrun: its items are then nc * nrun * nc
+    int wy0 = 0, wy1 = 0, wrun = 0;
     // the descriptor of a one-field batch (nfields == 1), equal to fields[0]:
     // kernels read it from their launch parameters
     FieldDev one;
 };
 
 // Launch configuration chosen by the tuner per kernel kind and sweep: block
-// size, persistent grid, and the register-cap variant of the kernel.
+// size, persistent grid, and the register-cap variant of the kernel
+// (reconstruction variants v and v + 3 are the same kernel).
 struct LaunchCfg {
     int block;
     int grid;
@@ -111,12 +114,11 @@ constexpr int kReconBlock = 128;
 constexpr int kFluxBlock = 64;
 constexpr int kUpdateBlock = 256;
 
-// Work items of a kernel kind / sweep / variant over the whole batch: window
-// runs (x / y reconstruction variants 0-2), z segments of one warp each (z
-// reconstruction variants 0-2), else cells.
-inline long long batch_items(const Batch &b, int kind, int dir, int variant)
+// Work items of a kernel kind / sweep over the whole batch: window runs (x / y
+// reconstruction), z lines of one warp each (z reconstruction), else cells.
+inline long long batch_items(const Batch &b, int kind, int dir)
 {
-    if (kind == K_RECON && variant < 3) return dir < 2 ? b.wtotal : b.ztotal;
+    if (kind == K_RECON) return dir < 2 ? b.wtotal : b.ztotal;
     return b.total;
 }
 

@@ -544,3 +544,24 @@ def test_mixed_accuracy_to_two_eddy_times(gks):
         a, b = out[gks.MIXED][key], out[gks.FP64][key]
         assert abs(a - b) < 1e-5 * abs(b), (key, a, b)
     assert out[gks.FP64]["tke"] < 0.9 * tke0  # the turbulence decayed
+
+
+@pytest.mark.parametrize("nc", [4, 5, 7, 31, 32, 33, 37, 65])
+def test_line_lengths_match_oracle(gks, oracle, nc):
+    """Edges of the reconstruction's tiles: lines shorter than, equal to and one
+    or a few cells beyond a warp's 32 cells, and window runs of 8 interfaces
+    with remainders; FP64 to 1e-12 per field, mixed to its FP32 WENO's 1e-6."""
+    case = gks_ic.make_dhit(nc, k0=min(4.0, nc / 4), Mt=0.5, seed=nc)
+    W = gks_ic.to_conservative_padded(case)
+    prm = oracle.params(nc, case.gam, case.mu0, case.p0, 1.0, case.Mt, case.t0)
+    for prec, tol in ((gks.FP64, 1e-12), (gks.MIXED, 1e-6)):
+        with gks.Solver(gks.phys_from_case(case), prec) as s:
+            s.upload(W)
+            dt = s.timestep(0.5)
+            s.step(2)
+            s.sync()
+            got = s.download()
+        ref = W.copy()
+        oracle.step(ref, prm, dt, 2)
+        err = np.abs(got - ref).reshape(5, -1).max(1) / np.abs(ref).reshape(5, -1).max(1)
+        assert np.all(err < tol), (prec, err)
