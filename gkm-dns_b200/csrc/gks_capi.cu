@@ -717,11 +717,15 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
         d.ksn = 2.0 * d.inv_dx;
         d.kst = 0.5 * d.inv_dx;
         d.hK2 = (p.K + 2) * 0.5;
-        const int kint[4] = {p.K + 2, p.K + 4, (p.K + 2) * (p.K + 4), -(p.K + 3)};
-        for (int i = 0; i < 4; ++i) {
-            d.kd[i] = (double)kint[i];
-            d.kf[i] = (float)kint[i];
-        }
+        d.igm1 = 1.0 / d.gm1;
+        d.shig = std::sqrt(d.hig);
+        d.rlg = 0.5 / (std::sqrt(pi) * d.shig);
+        d.kA4 = p.pr_factor / (p.K + 3);
+        d.prm1 = p.pr_factor - 1.0;
+        const int kdi[5] = {p.K + 2, 2 * (p.K + 2), p.K + 3, p.K + 4, p.K + 5};
+        for (int i = 0; i < 5; ++i) d.kd[i] = (double)kdi[i];
+        const int kfi[4] = {p.K + 2, p.K + 4, (p.K + 2) * (p.K + 4), -(p.K + 3)};
+        for (int i = 0; i < 4; ++i) d.kf[i] = (float)kfi[i];
         // spline grids of the reference's einspline call (Interpolation.cpp:10-27):
         // a segment's grid starts at its first plane sta, here 0 along x and z
         // and y0 along y

@@ -1,6 +1,7 @@
-// Time-integrated BGK-NS interface flux (weno/src/GKMflux.cpp:11-215) with the
-// moments of every Maxwellian evaluated in the frame that moves with that
-// Maxwellian's transverse velocity.
+// Time-integrated BGK-NS interface flux (weno/src/GKMflux.cpp:11-215), mixed
+// FP32 / FP64 path, with the moments of every Maxwellian evaluated in the frame
+// that moves with that Maxwellian's transverse velocity (the FP64 path, in
+// gks_flux64.cuh, also moves with the normal one).
 //
 // The reference builds 1-D moment tables of all three velocity components for
 // each of its three Maxwellians (left, right, equilibrium; GKMflux.cpp:48-66,
@@ -25,13 +26,13 @@
 // reference's; only the order of evaluation differs, so results agree with it
 // to rounding.
 //
-// Precision: `S` is the type of the slope solves and slope-weighted moment
-// vectors -- the flux assembly -- (double in the FP64 path, float in the
-// mixed path).  The primitive states, collision time and time weights, the
-// moment-table recursions with their erfc / exp seeds, the zeroth-order
-// (slope-free) moments -- the equilibrium state W0, the p0 and p3 terms of the
-// flux and the gm1 / gm3 terms of B_ -- and the flux accumulation stay double
-// in both paths.
+// Precision: the slope solves and slope-weighted moment vectors -- the flux
+// assembly -- are FP32, those of the left and right Maxwellians as the two
+// lanes of paired instructions (f2).  The primitive states, collision time and
+// time weights, the moment-table recursions with their erfc / exp seeds, the
+// zeroth-order (slope-free) moments -- the equilibrium state W0, the p0 and p3
+// terms of the flux and the gm1 / gm3 terms of B_ -- and the flux accumulation
+// are double.
 #pragma once
 
 #include "gks_device.cuh"
@@ -41,24 +42,18 @@ namespace gks {
 constexpr double kHalfRsqrtPi = 0.28209479177387814; // 1 / (2 sqrt(pi))
 
 // Constants of one Maxwellian in its transverse co-moving frame.  The paired
-// type f2 takes no operand negation, so for it the negatives are kept as
-// well, making every use a plain fused multiply-add; in double a negated
-// operand is free, and the negatives are formed at the use.
+// type f2 takes no operand negation, so the negatives are kept as well, making
+// every use a plain fused multiply-add.
 template <typename T> struct CoFrame {
     T U0, U1, U2, hu2;     // normal and transverse velocity, hu2 = (U1^2 + U2^2)/2 (to_lab)
-    T nU0_, nU1_, nU2_, nhu2_; // their negatives (f2 only)
+    T nU0, nU1, nU2, nhu2; // their negatives
     T m2U0, nqn, nqh;      // -2 U0, -qn, -qn/2 with qn = U0^2 + (K+3) s (solve)
     T tl, kal2;            // 2 lambda, kA lambda^2 (solve)
     T s, r2, r4, q4;       // 1/(2 lambda), <rho^2>, <rho^4>, <c1^2 rho^2> (moments)
-    static constexpr bool kDouble = std::is_same<T, double>::value;
-    __device__ __forceinline__ T nU0() const { if constexpr (kDouble) return -U0; else return nU0_; }
-    __device__ __forceinline__ T nU1() const { if constexpr (kDouble) return -U1; else return nU1_; }
-    __device__ __forceinline__ T nU2() const { if constexpr (kDouble) return -U2; else return nU2_; }
-    __device__ __forceinline__ T nhu2() const { if constexpr (kDouble) return -hu2; else return nhu2_; }
 };
 
-template <typename T, typename KT>
-__device__ __forceinline__ CoFrame<T> co_frame(T U0, T U1, T U2, T s, T lam, const KConst<KT> &kc, T kA)
+template <typename T>
+__device__ __forceinline__ CoFrame<T> co_frame(T U0, T U1, T U2, T s, T lam, const KConst &kc, T kA)
 {
     CoFrame<T> f;
     f.U0 = U0;
@@ -66,14 +61,12 @@ __device__ __forceinline__ CoFrame<T> co_frame(T U0, T U1, T U2, T s, T lam, con
     f.U2 = U2;
     f.hu2 = T(0.5f) * fmaT(U1, U1, U2 * U2);
     const T m1 = T(-1.0f);
-    if constexpr (!CoFrame<T>::kDouble) {
-        f.nU0_ = m1 * U0;
-        f.nU1_ = m1 * U1;
-        f.nU2_ = m1 * U2;
-        f.nhu2_ = m1 * f.hu2;
-    }
+    f.nU0 = m1 * U0;
+    f.nU1 = m1 * U1;
+    f.nU2 = m1 * U2;
+    f.nhu2 = m1 * f.hu2;
     f.m2U0 = T(-2.0f) * U0;
-    f.nqn = fmaT(f.nU0(), U0, T(kc.nq) * s);
+    f.nqn = fmaT(f.nU0, U0, T(kc.nq) * s);
     f.nqh = T(0.5f) * f.nqn;
     f.tl = T(2.0f) * lam;
     f.kal2 = (kA * lam) * lam;
@@ -106,7 +99,7 @@ __device__ __forceinline__ void to_prime(T b[5], T nU1, T nU2, T nhu2)
 template <typename T>
 __device__ __forceinline__ void to_prime(T b[5], const CoFrame<T> &f)
 {
-    to_prime<T>(b, f.nU1(), f.nU2(), f.nhu2());
+    to_prime<T>(b, f.nU1, f.nU2, f.nhu2);
 }
 
 // Slope solve (slopesolver, GKMflux.cpp:280-296) in the primed frame: the
@@ -116,13 +109,13 @@ __device__ __forceinline__ void to_prime(T b[5], const CoFrame<T> &f)
 template <typename T>
 __device__ __forceinline__ void solve(const T b[5], const CoFrame<T> &f, T a[5])
 {
-    const T R2 = fmaT(f.nU0(), b[0], b[1]);
+    const T R2 = fmaT(f.nU0, b[0], b[1]);
     const T R5 = fmaT(f.nqn, b[0], T(2.0f) * b[4]);
     a[4] = f.kal2 * fmaT(f.m2U0, R2, R5);
     a[3] = f.tl * b[3];
     a[2] = f.tl * b[2];
-    a[1] = fmaT(f.nU0(), a[4], f.tl * R2);
-    a[0] = fmaT(f.nU0(), a[1], fmaT(f.nqh, a[4], b[0]));
+    a[1] = fmaT(f.nU0, a[4], f.tl * R2);
+    a[0] = fmaT(f.nU0, a[1], fmaT(f.nqh, a[4], b[0]));
 }
 
 // M = <psi' u^k (a.psi')> over the normal table X (primed frame):
@@ -233,13 +226,12 @@ __device__ __forceinline__ Prim side_tables(const Src &src, const FluxConst &c, 
     return g;
 }
 
-// Slope part of the side pass, on the arithmetic type T of the flux assembly:
-// double (one Maxwellian), or f2 (the left and right Maxwellians as the two
-// lanes of paired FP32 instructions).  `io` supplies the state differences,
+// Slope part of the two side passes, the left and right Maxwellians as the two
+// lanes of paired FP32 instructions (T = f2).  `io` supplies the state differences,
 //   io.slope(d, b)        along d = normal, 1st, 2nd transverse, which
 // sc[d] = ks[d] / rho turns into the right-hand sides b = DW / rho,
 // and takes the lab-frame results,
-//   io.emit(slot, den, M) adds den * M to S sum slot `slot` (lanes summed):
+//   io.emit(slot, den, M) sets FP32 sum `slot` to den * M, lanes summed:
 // the transverse right-hand sides by_, bz_ of the equilibrium slopes (slots
 // 0-4, 5-9), B_ (10-14) and the p4 / p5 flux terms (15-19).
 template <typename T, typename IO>
@@ -321,17 +313,6 @@ __device__ __forceinline__ void side_slopes(const IO &io, const CoFrame<T> &f, c
     }
 }
 
-// Slope inputs and results of one side pass in double.
-template <int NEG, typename Src>
-struct SideIO64 {
-    const Src &src;
-    __device__ __forceinline__ void slope(int d, double b[5]) const { src.slope(NEG, d, b); }
-    __device__ __forceinline__ void emit(int slot, double a, double m) const
-    {
-        src.template put_s<NEG == 0>(slot, a, m);
-    }
-};
-
 // Slope inputs and results of the paired side pass (left lane .x, right .y);
 // the lane-summed results stay in the caller's registers (out[20]).
 template <typename Src>
@@ -352,35 +333,13 @@ struct SideIO2 {
     }
 };
 
-// The two side passes of the FP64 path, one after the other; the equilibrium
-// pass reads the parked sums behind a compiler memory barrier, so that the
+// The double parts of the two side passes (their erfc / exp chains overlap),
+// then their FP32 slope parts together as the lanes of paired instructions.
+// The equilibrium pass comes behind a compiler memory barrier, so that the
 // scheduler cannot start its long erfc / exp chains early and keep the side
 // passes' state live at the same time.
 template <typename Src>
-__device__ __forceinline__ void flux_sides(const Src &src, const FluxConst &c, const SideWeights &tw, double, float *)
-{
-    {
-        double Xh[7], Xf[6];
-        const Prim g = side_tables<0>(src, c, tw.p3, Xh, Xf);
-        const CoFrame<double> f = co_frame<double>(g.U0, g.U1, g.U2, g.s, g.lam, c.kd, c.kA);
-        const double sc[3] = {c.ks[0] * g.rinv, c.ks[1] * g.rinv, c.ks[2] * g.rinv};
-        side_slopes<double>(SideIO64<0, Src>{src}, f, Xh, Xf, sc, g.den, tw.w45, -tw.g5, tw.p4, -tw.p5);
-    }
-    {
-        double Xh[7], Xf[6];
-        const Prim g = side_tables<1>(src, c, tw.p3, Xh, Xf);
-        const CoFrame<double> f = co_frame<double>(g.U0, g.U1, g.U2, g.s, g.lam, c.kd, c.kA);
-        const double sc[3] = {c.ks[0] * g.rinv, c.ks[1] * g.rinv, c.ks[2] * g.rinv};
-        side_slopes<double>(SideIO64<1, Src>{src}, f, Xh, Xf, sc, g.den, tw.w45, -tw.g5, tw.p4, -tw.p5);
-    }
-    asm volatile("" ::: "memory");
-}
-
-// The mixed path: the double parts of the two side passes (their erfc / exp
-// chains overlap), then their FP32 slope parts together as the lanes of
-// paired instructions.
-template <typename Src>
-__device__ __forceinline__ void flux_sides(const Src &src, const FluxConst &c, const SideWeights &tw, float, float *sout)
+__device__ __forceinline__ void flux_sides(const Src &src, const FluxConst &c, const SideWeights &tw, float *sout)
 {
     f2 Xh[7], Xf[6];
     f2 U0, U1, U2, s, lam, rinv, den;
@@ -411,11 +370,6 @@ __device__ __forceinline__ void flux_sides(const Src &src, const FluxConst &c, c
     asm volatile("" ::: "memory");
 }
 
-// The field's K constants in the type of the flux assembly.
-template <typename S> __device__ __forceinline__ const KConst<S> &kconst(const FluxConst &c);
-template <> __device__ __forceinline__ const KConst<double> &kconst<double>(const FluxConst &c) { return c.kd; }
-template <> __device__ __forceinline__ const KConst<float> &kconst<float>(const FluxConst &c) { return c.kf; }
-
 // Time-integrated BGK-NS flux through one interface, in the frame of the
 // interface normal.  `src` supplies the inputs when they are needed, so that
 // one side's inputs are not live while the other side is processed, and keeps
@@ -423,13 +377,14 @@ template <> __device__ __forceinline__ const KConst<float> &kconst<float>(const 
 //   src.state(side, W)        reconstructed state Wl (side 0) or Wr (side 1)
 //   src.slope(side, d, DW)    its slopes along d = normal, 1st, 2nd transverse
 //   src.cells(WL, WR)         the cell averages either side of the interface
-//   src.put_d / put_s<FIRST>(slot, v), get_d / get_s(slot)   running sums
-// (the mixed path keeps its type-S sums in registers: the paired side pass
-// produces them all at once).
+//   src.put_d<FIRST>(slot, a, b), get_d(slot)   running double sums
+// (the FP32 sums stay in registers: the paired side pass produces them all at
+// once).
 // mu/p at the left cell = tau_n / tau_d.  Output F[5], the flux integrated over [0, dt].
-template <typename S, typename Src>
+template <typename Src>
 __device__ __forceinline__ void gks_flux(const Src &src, double tau_n, double tau_d, const FluxConst &c, double F[5])
 {
+    using S = float;
     const double dt = c.dt;
     double tau, ex, om, igm0;
     SideWeights tw;
@@ -464,11 +419,8 @@ __device__ __forceinline__ void gks_flux(const Src &src, double tau_n, double ta
         tw.p5 = -tau * Pt;
     }
     float sreg[20];
-    flux_sides(src, c, tw, S(), sreg);
-    auto gets = [&](int k) -> S {
-        if constexpr (sizeof(S) == 4) return sreg[k];
-        else return src.get_s(k);
-    };
+    flux_sides(src, c, tw, sreg);
+    auto gets = [&](int k) -> S { return sreg[k]; };
     const double gm1 = -om * igm0, gm3 = -gm1;
     const double Pt = tau * om, Qt = tau * fma(-dt, ex, Pt);
     const double gm2 = fma(-dt, ex, fma(2.0, Pt, -dt)) * igm0;
@@ -507,7 +459,7 @@ __device__ __forceinline__ void gks_flux(const Src &src, double tau_n, double ta
         for (int q = 0; q < 5; ++q) Bd[q] = (fma(w, M[q], gm3 * We[q]) + double(gets(10 + q))) * e.rinv;
         to_prime<double>(Bd, -e.U1, -e.U2, -0.5 * fma(e.U1, e.U1, e.U2 * e.U2));
     }
-    const CoFrame<S> f = co_frame<S>(S(e.U0), S(e.U1), S(e.U2), S(e.s), S(e.lam), kconst<S>(c), S(c.kA));
+    const CoFrame<S> f = co_frame<S>(S(e.U0), S(e.U1), S(e.U2), S(e.s), S(e.lam), c.kf, S(c.kA));
     S Xfs[6], Xps[7], Xns[7];
 #pragma unroll
     for (int n = 0; n < 6; ++n) Xfs[n] = S(Xf[n]);

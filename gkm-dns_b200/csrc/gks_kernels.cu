@@ -10,6 +10,7 @@
 // in `along` and in the windowed reconstruction's cell map.
 #include "gks_device.cuh"
 #include "gks_flux.cuh"
+#include "gks_flux64.cuh"
 #include "gks_kernels.cuh"
 #include "../../include/gks_b200.h"
 
@@ -518,9 +519,10 @@ __global__ void __launch_bounds__(kReconBlock, MINB) k_recon_win(Batch b)
 // ---------------------------------------------------------------------------
 // Flux at the interface between cell c and its +1 neighbour along DIR
 // (derivsX/Y/Z, update.cpp:201-453, and flux, GKMflux.cpp:11-215).
-// Transverse lines: x sweep N,S = y+-1, F,B = z+-1; y sweep N,S = x-+1 with
-// DWy = -(N-S)/2dx, F,B = z+-1; z sweep N,S = x+-1, F,B = y+-1 (the
-// reference's assignment) or, with GKS_FIX_ZSWEEP, N,S = y+-1, F,B = x+-1.
+// Transverse lines: x sweep N,S = y+-1, F,B = z+-1; y sweep N,S = x+-1 (the
+// reference takes x-+1 with DWy = -(N-S)/2dx), F,B = z+-1; z sweep N,S = x+-1,
+// F,B = y+-1 (the reference's assignment) or, with GKS_FIX_ZSWEEP, N,S = y+-1,
+// F,B = x+-1.
 // Momentum is rotated into slot 1 for y (rho v) and z (rho w).
 // ---------------------------------------------------------------------------
 template <int DIR>
@@ -531,7 +533,7 @@ __device__ __forceinline__ void transverse(const Cell &x, int flags, unsigned &n
         n = along<1>(x, 1); s = along<1>(x, -1);
         fr = along<2>(x, 1); bk = along<2>(x, -1);
     } else if (DIR == 1) {
-        n = along<0>(x, -1); s = along<0>(x, 1);
+        n = along<0>(x, 1); s = along<0>(x, -1);
         fr = along<2>(x, 1); bk = along<2>(x, -1);
     } else {
         if (flags & GKS_FIX_ZSWEEP) {
@@ -544,55 +546,117 @@ __device__ __forceinline__ void transverse(const Cell &x, int flags, unsigned &n
     }
 }
 
-// Inputs and running sums of one interface (see gks_flux).  All global loads
-// are issued at once when the interface starts, so that their latency
-// overlaps; what is not needed until later -- the right state and its slopes,
-// the two cell averages -- is parked in this thread's own shared-memory slots
-// ([slot][thread], no bank conflicts) instead of registers, and so are the
-// sums the two side passes of the flux accumulate for the equilibrium pass.
-// Slot q of the rotated frame holds original component perm(q): rho v (y
-// sweep) or rho w (z sweep) moves into slot 1 (update.cpp:340-350, 429-439).
-template <int DIR, typename S>
+// Inputs and running sums of one interface.  All global loads are issued at
+// once when the interface starts, so that their latency overlaps; the values
+// are parked in this thread's own shared-memory slots ([slot][thread], no bank
+// conflicts) until a pass of the flux needs them, and so are the sums the two
+// side passes accumulate for the equilibrium pass, so that only one pass's
+// state is in registers at a time.  Slot q of the rotated frame holds original
+// component perm(q): rho v (y sweep) or rho w (z sweep) moves into slot 1
+// (update.cpp:340-350, 429-439).  DWxl = 2(Wl - WL)/dx, DWxr = 2(WR - Wr)/dx;
+// transverse central differences of the neighbouring lines' states
+// (update.cpp:253-260, 327-334, 416-423), here the differences in double (they
+// cancel), which the flux scales.
+template <int DIR> __device__ constexpr int perm(int q)
+{
+    return DIR == 0 ? q : (q == 1 ? (DIR == 1 ? 2 : 3) : (q == (DIR == 1 ? 2 : 3) ? 1 : q));
+}
+
+// The ten-value records of the interface and its four transverse neighbours.
+struct Records {
+    double r0[10], rn[10], rs[10], rf[10], rb[10];
+    __device__ __forceinline__ Records(const double *rec, unsigned c, unsigned cn, unsigned cs, unsigned cf, unsigned cb,
+                                       long long n)
+    {
+        get_record(rec, c, r0, n);
+        get_record(rec, cn, rn, n);
+        get_record(rec, cs, rs, n);
+        get_record(rec, cf, rf, n);
+        get_record(rec, cb, rb, n);
+    }
+};
+
+// FP64 path (gks_flux64): 50 slots, 400 B per thread, so that eight blocks fit
+// an SM.  The left side's inputs sit in the slots of sums that its own pass
+// writes after it has read them.
+template <int DIR> struct SweepSrc64 {
+    static constexpr int kWL = 0, kWR = 5, kWr = 10, kDr = 15; // cell averages, right state, its transverse slopes
+    static constexpr int kW0 = 25, kBy = 30, kBz = 35, kB = 40, kF = 45; // sums
+    static constexpr int kWl = kBy, kDl = kB;                            // left state, its transverse slopes
+    static constexpr int kSlots = 50;
+    double (*slots)[kFluxBlock];
+
+    __device__ __forceinline__ double &at(int i) const { return slots[i][threadIdx.x]; }
+
+    __device__ __forceinline__ void load(const FieldDev &f, unsigned c, unsigned c1, unsigned cn, unsigned cs,
+                                         unsigned cf, unsigned cb) const
+    {
+        const Records r(f.rec[DIR], c, cn, cs, cf, cb, f.ncell);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            const int o = perm<DIR>(q);
+            at(kWL + q) = __ldg(f.W[o] + c);
+            at(kWR + q) = __ldg(f.W[o] + c1);
+            at(kWl + q) = r.r0[o];
+            at(kWr + q) = r.r0[5 + o];
+            at(kDl + q) = r.rn[o] - r.rs[o];
+            at(kDl + 5 + q) = r.rf[o] - r.rb[o];
+            at(kDr + q) = r.rn[5 + o] - r.rs[5 + o];
+            at(kDr + 5 + q) = r.rf[5 + o] - r.rb[5 + o];
+        }
+    }
+    template <int SIDE> __device__ __forceinline__ void state(double W[5]) const
+    {
+#pragma unroll
+        for (int q = 0; q < 5; ++q) W[q] = at((SIDE ? kWr : kWl) + q);
+    }
+    // differences of side's state W along d (0 normal, 1 and 2 transverse)
+    template <int SIDE, int D> __device__ __forceinline__ void slope(const double W[5], double b[5]) const
+    {
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            if (D == 0) b[q] = SIDE ? at(kWR + q) - W[q] : W[q] - at(kWL + q);
+            else b[q] = at((SIDE ? kDr : kDl) + 5 * (D - 1) + q);
+        }
+    }
+    __device__ __forceinline__ void cells(double WL[5], double WR[5]) const
+    {
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            WL[q] = at(kWL + q);
+            WR[q] = at(kWR + q);
+        }
+    }
+    template <int SIDE> __device__ __forceinline__ void sum(int i, double v) const { at(i) = SIDE ? at(i) + v : v; }
+    __device__ __forceinline__ double get(int i) const { return at(i); }
+};
+
+// Mixed path (gks_flux): the left state and its slopes stay in registers.
+template <int DIR>
 struct SweepSrc {
     double Wl[5];
-    S DWl[3][5];
-    S (*park_dw)[kFluxBlock];      // [15][block]: right-side slopes
+    float DWl[3][5];
+    float (*park_dw)[kFluxBlock];  // [15][block]: right-side slopes
     double (*park_w)[kFluxBlock];  // [15][block]: WL, WR, Wr
     double (*sum_d)[kFluxBlock];   // [10][block]: double sums of the side passes
-    S (*sum_s)[kFluxBlock];        // [20][block]: S sums of the side passes (FP64 path)
 
-    __device__ static constexpr int perm(int q)
-    {
-        return DIR == 0 ? q : (q == 1 ? (DIR == 1 ? 2 : 3) : (q == (DIR == 1 ? 2 : 3) ? 1 : q));
-    }
-
-    // DWxl = 2(Wl - WL)/dx, DWxr = 2(WR - Wr)/dx; transverse central differences of
-    // the neighbouring lines' states (update.cpp:253-260, 327-334, 416-423), here
-    // the differences, which the flux scales by FluxConst::ks
     __device__ __forceinline__ void load(const FieldDev &f, unsigned c, unsigned c1, unsigned cn, unsigned cs,
                                          unsigned cf, unsigned cb)
     {
-        // differences in double (they cancel); the flux scales them (FluxConst::ks)
         const int t = threadIdx.x;
-        const double *rec = f.rec[DIR];
-        double r0[10], rn[10], rs[10], rf[10], rb[10];
-        get_record(rec, c, r0, f.ncell);
-        get_record(rec, cn, rn, f.ncell);
-        get_record(rec, cs, rs, f.ncell);
-        get_record(rec, cf, rf, f.ncell);
-        get_record(rec, cb, rb, f.ncell);
+        const Records r(f.rec[DIR], c, cn, cs, cf, cb, f.ncell);
 #pragma unroll
         for (int q = 0; q < 5; ++q) {
-            const int o = perm(q);
+            const int o = perm<DIR>(q);
             const double wL = __ldg(f.W[o] + c), wR = __ldg(f.W[o] + c1);
-            const double wr = r0[5 + o];
-            Wl[q] = r0[o];
-            DWl[0][q] = S(Wl[q] - wL);
-            DWl[1][q] = S(rn[o] - rs[o]);
-            DWl[2][q] = S(rf[o] - rb[o]);
-            park_dw[q][t] = S(wR - wr);
-            park_dw[5 + q][t] = S(rn[5 + o] - rs[5 + o]);
-            park_dw[10 + q][t] = S(rf[5 + o] - rb[5 + o]);
+            const double wr = r.r0[5 + o];
+            Wl[q] = r.r0[o];
+            DWl[0][q] = float(Wl[q] - wL);
+            DWl[1][q] = float(r.rn[o] - r.rs[o]);
+            DWl[2][q] = float(r.rf[o] - r.rb[o]);
+            park_dw[q][t] = float(wR - wr);
+            park_dw[5 + q][t] = float(r.rn[5 + o] - r.rs[5 + o]);
+            park_dw[10 + q][t] = float(r.rf[5 + o] - r.rb[5 + o]);
             park_w[q][t] = wL;
             park_w[5 + q][t] = wR;
             park_w[10 + q][t] = wr;
@@ -606,7 +670,7 @@ struct SweepSrc {
     }
 
     // slopes of one side along one direction (0 normal, 1 and 2 transverse)
-    __device__ __forceinline__ void slope(int side, int d, S DW[5]) const
+    __device__ __forceinline__ void slope(int side, int d, float DW[5]) const
     {
 #pragma unroll
         for (int q = 0; q < 5; ++q) DW[q] = side == 0 ? DWl[d][q] : park_dw[5 * d + q][threadIdx.x];
@@ -630,48 +694,54 @@ struct SweepSrc {
         double &x = sum_d[i][threadIdx.x];
         x = FIRST ? __dmul_rn(a, b) : __fma_rn(a, b, x);
     }
-    template <bool FIRST> __device__ __forceinline__ void put_s(int i, S a, S b) const
-    {
-        S &x = sum_s[i][threadIdx.x];
-        if constexpr (sizeof(S) == 8) x = FIRST ? __dmul_rn(a, b) : __fma_rn(a, b, x);
-        else x = FIRST ? __fmul_rn(a, b) : __fmaf_rn(a, b, x);
-    }
     __device__ __forceinline__ double get_d(int i) const { return sum_d[i][threadIdx.x]; }
-    __device__ __forceinline__ S get_s(int i) const { return sum_s[i][threadIdx.x]; }
 };
 
-// The flux of work item `it` of field f.
-template <int DIR, typename S>
-__device__ __forceinline__ void flux_item(const FieldDev &f, long long it, S (*park_dw)[kFluxBlock],
-                                          double (*park_w)[kFluxBlock], double (*sum_d)[kFluxBlock],
-                                          S (*sum_s)[kFluxBlock])
+// The flux of work item `it` of field f; `smem` is the block's parking space.
+template <int PREC> struct FluxPark;
+template <> struct FluxPark<0> {
+    double slots[SweepSrc64<0>::kSlots][kFluxBlock];
+};
+template <> struct FluxPark<1> {
+    double w[15][kFluxBlock], sum[10][kFluxBlock];
+    float dw[15][kFluxBlock];
+};
+
+template <int DIR, int PREC>
+__device__ __forceinline__ void flux_item(const FieldDev &f, long long it, FluxPark<PREC> &park)
 {
     const Cell x = decode(unsigned(it - f.base), f);
     unsigned cn, cs, cf, cb;
     transverse<DIR>(x, f.flags, cn, cs, cf, cb);
-    SweepSrc<DIR, S> src;
-    src.park_dw = park_dw;
-    src.park_w = park_w;
-    src.sum_d = sum_d;
-    src.sum_s = sum_s;
-    src.load(f, x.c, along<DIR>(x, 1), cn, cs, cf, cb);
     // collision time mu / p at the left cell (update.cpp:262-264), stored by
     // this step's x-sweep reconstruction
-    const double tau_n = __ldg(f.tau[0] + x.c), tau_d = __ldg(f.tau[1] + x.c);
-    FluxConst fc;
-    fc.gm1 = f.gm1;
-    fc.hig = f.hig;
-    fc.dt = f.dt;
-    fc.dx = f.dx;
-    fc.ks[0] = f.ksn;
-    fc.ks[1] = DIR == 1 ? -f.kst : f.kst; // y sweep: DWy = -(N - S)/(2 dx)
-    fc.ks[2] = f.kst;
-    fc.kA = f.kA;
-    fc.hK2 = f.hK2;
-    fc.kd = {f.kd[0], f.kd[1], f.kd[2], f.kd[3]};
-    fc.kf = {f.kf[0], f.kf[1], f.kf[2], f.kf[3]};
     double F[5];
-    gks_flux<S>(src, tau_n, tau_d, fc, F);
+    if constexpr (PREC == 0) {
+        SweepSrc64<DIR> src{park.slots};
+        src.load(f, x.c, along<DIR>(x, 1), cn, cs, cf, cb);
+        const double tau_n = __ldg(f.tau[0] + x.c), tau_d = __ldg(f.tau[1] + x.c);
+        const FluxConst64 fc = {f.dt,  f.gm1, f.igm1,  f.shig,  f.rlg,   f.ksn,   f.kst,
+                                f.kA4, f.prm1, f.kd[0], f.kd[1], f.kd[2], f.kd[3], f.kd[4]};
+        gks_flux64(src, tau_n, tau_d, fc, F);
+    } else {
+        SweepSrc<DIR> src;
+        src.park_dw = park.dw;
+        src.park_w = park.w;
+        src.sum_d = park.sum;
+        src.load(f, x.c, along<DIR>(x, 1), cn, cs, cf, cb);
+        const double tau_n = __ldg(f.tau[0] + x.c), tau_d = __ldg(f.tau[1] + x.c);
+        FluxConst fc;
+        fc.gm1 = f.gm1;
+        fc.hig = f.hig;
+        fc.dt = f.dt;
+        fc.dx = f.dx;
+        fc.ks[0] = f.ksn;
+        fc.ks[1] = fc.ks[2] = f.kst;
+        fc.kA = f.kA;
+        fc.hK2 = f.hK2;
+        fc.kf = {f.kf[0], f.kf[1], f.kf[2], f.kf[3]};
+        gks_flux(src, tau_n, tau_d, fc, F);
+    }
     constexpr int ROT = DIR == 0 ? 0 : (DIR == 1 ? 2 : 3);
     if (ROT) {
         const double t = F[1];
@@ -688,22 +758,18 @@ __device__ __forceinline__ void flux_item(const FieldDev &f, long long it, S (*p
 template <int DIR, int PREC, int REGS>
 __global__ void __launch_bounds__(kFluxBlock) __maxnreg__(REGS) k_flux(Batch b)
 {
-    using S = typename std::conditional<PREC == 0, double, float>::type;
-    __shared__ S park_dw[15][kFluxBlock];
-    __shared__ double park_w[15][kFluxBlock];
-    __shared__ double sum_d[10][kFluxBlock];
-    __shared__ S sum_s[20][kFluxBlock];
+    __shared__ FluxPark<PREC> park;
     const long long stride = (long long)gridDim.x * blockDim.x;
     if (b.nfields == 1) {
         const long long end = b.hi < b.one.ncell ? b.hi : b.one.ncell; // alignment padding after the field
         for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < end; it += stride)
-            flux_item<DIR, S>(b.one, it, park_dw, park_w, sum_d, sum_s);
+            flux_item<DIR, PREC>(b.one, it, park);
         return;
     }
     for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < b.hi; it += stride) {
         const FieldDev &f = b.fields[field_of(b.fields, b.nfields, it)];
         if (it - f.base >= f.ncell) continue; // alignment padding after the field
-        flux_item<DIR, S>(f, it, park_dw, park_w, sum_d, sum_s);
+        flux_item<DIR, PREC>(f, it, park);
     }
 }
 
@@ -1180,7 +1246,7 @@ cudaError_t occ(KernelT k, int block, int *n)
 // and caps at 168, as for 6 blocks.  The tuner picks one variant per kernel,
 // precision and sweep.  Every variant gives bit-identical results.
 constexpr int kReconMinb[3] = {3, 4, 5};
-constexpr int kFluxRegs[kFluxVariants] = {200, 168, 128};
+constexpr int kFluxRegs[2][kFluxVariants] = {{168, 144, 128}, {200, 168, 128}};
 
 // The item range of a launch (all items of its kind when b.hi < 0) and the
 // blocks it needs: at most cfg.grid, no more than the range fills.
@@ -1230,9 +1296,9 @@ cudaError_t flux_go(Batch b, LaunchCfg cfg, cudaStream_t st)
     if (b.hi <= b.lo) return cudaSuccess;
     const int g = range_grid(cfg.grid, b.hi - b.lo, cfg.block);
     switch (cfg.variant) {
-    case 1: k_flux<DIR, PREC, kFluxRegs[1]><<<g, cfg.block, 0, st>>>(b); break;
-    case 2: k_flux<DIR, PREC, kFluxRegs[2]><<<g, cfg.block, 0, st>>>(b); break;
-    default: k_flux<DIR, PREC, kFluxRegs[0]><<<g, cfg.block, 0, st>>>(b); break;
+    case 1: k_flux<DIR, PREC, kFluxRegs[PREC][1]><<<g, cfg.block, 0, st>>>(b); break;
+    case 2: k_flux<DIR, PREC, kFluxRegs[PREC][2]><<<g, cfg.block, 0, st>>>(b); break;
+    default: k_flux<DIR, PREC, kFluxRegs[PREC][0]><<<g, cfg.block, 0, st>>>(b); break;
     }
     return cudaGetLastError();
 }
@@ -1251,9 +1317,9 @@ cudaError_t occ_kind(int kind, int variant, int block, int *n)
             return occ(k_recon_zline<PREC, kReconMinb[0]>, block, n);
         }
     }
-    if (variant == 1) return occ(k_flux<DIR, PREC, kFluxRegs[1]>, block, n);
-    if (variant == 2) return occ(k_flux<DIR, PREC, kFluxRegs[2]>, block, n);
-    return occ(k_flux<DIR, PREC, kFluxRegs[0]>, block, n);
+    if (variant == 1) return occ(k_flux<DIR, PREC, kFluxRegs[PREC][1]>, block, n);
+    if (variant == 2) return occ(k_flux<DIR, PREC, kFluxRegs[PREC][2]>, block, n);
+    return occ(k_flux<DIR, PREC, kFluxRegs[PREC][0]>, block, n);
 }
 
 template <int PREC>
