@@ -79,6 +79,7 @@ struct gks_ctx {
     double *d_sums = nullptr;
     unsigned long long *d_bits = nullptr;
     int *d_err = nullptr;
+    unsigned *d_queue = nullptr;
     gks::LaunchCfg cfg[gks::K_KINDS][3];
     std::string err;
 };
@@ -179,8 +180,9 @@ int read_err(gks_ctx *ctx, int *word, bool clear)
     return GKS_OK;
 }
 
-// Persistent grid: `mult` times the resident blocks of the kernel, no more
-// blocks than the work needs.
+// Persistent grid: `mult` times the resident blocks of the kernel, or (mult 0)
+// as many blocks as the work needs, which the hardware hands out as earlier
+// ones end; never more than the work needs.
 gks::LaunchCfg persistent(gks_ctx *ctx, int kind, int dir, int variant, int mult)
 {
     gks::LaunchCfg c;
@@ -194,20 +196,24 @@ gks::LaunchCfg persistent(gks_ctx *ctx, int kind, int dir, int variant, int mult
     // reconstruction), else one per cell
     const long long items = gks::batch_items(ctx->batch, kind, dir) * (kind == gks::K_RECON && dir == 2 ? 32 : 1);
     const long long need = (items + c.block - 1) / c.block;
-    if (g > need) g = need;
+    if (g > need || mult == 0) g = need;
     if (g < 1) g = 1;
     c.grid = (int)g;
     return c;
 }
 
-// Untuned defaults: the flux at the 168-register cap (6 blocks of 64
-// threads per SM), the reconstruction at its natural register count.
+// Untuned defaults: the flux at the 168-register cap (6 blocks of 64 threads
+// per SM), one wave of blocks; the reconstruction with all its blocks launched
+// (a wave of persistent blocks ends unevenly: 256^3 x / y / z, FP64 694 / 627 /
+// 680 -> 670 / 601 / 634 us, mixed 533 / 511 / 501 -> 502 / 465 / 458), at its
+// natural register count but for the FP64 z sweep, which the 96-register cap
+// (20 warps per SM, 40 B spill) serves best (663 at 150 registers).
 void choose_launch(gks_ctx *ctx)
 {
     for (int kind = 0; kind < gks::K_KINDS; ++kind)
         for (int dir = 0; dir < 3; ++dir) {
-            const int variant = kind == gks::K_FLUX ? 1 : 0;
-            ctx->cfg[kind][dir] = persistent(ctx, kind, dir, variant, 1);
+            const int variant = kind == gks::K_FLUX ? 1 : (kind == gks::K_RECON && dir == 2 && ctx->precision == GKS_FP64 ? 2 : 0);
+            ctx->cfg[kind][dir] = persistent(ctx, kind, dir, variant, kind == gks::K_RECON ? 0 : 1);
         }
 }
 
@@ -347,14 +353,20 @@ int ensure_pipe(gks_ctx *ctx, FieldHost &h)
 }
 
 // Run length of the windowed reconstruction over `lines` (count, interfaces
-// per line): the longest that leaves at least kWinItemsPerSm items per SM.
+// per line): the longest that leaves at least kWinItemsPerSm items per SM, or
+// else, from kWinRunFull down, at least kWinItemsMin.  A run of n costs n + 1
+// cells and a prologue of six loads, so long runs are the cheaper ones where
+// the GPU is full anyway (256^3 x sweep, us by run, FP64: 8 708, 16 654, 64 624);
+// a small field is a chain of cells per thread on a part of the SMs, shorter
+// with short runs (32^3 / 48^3, FP64: run 8 18.6 / 19.1, run 2 13.6 / 15.8, run 1
+// 13.4 / 19.7; 64^3: run 8 23.7, run 4 24.5, run 2 26.4).
 int win_run_for(const gks_ctx *ctx, const std::vector<std::pair<long long, long long>> &lines)
 {
-    int run = gks::win_run(ctx->precision == GKS_MIXED ? 1 : 0);
-    for (; run > gks::kWinRunMin; run /= 2) {
+    int run = gks::kWinRunMax;
+    for (; run > 1; run /= 2) {
         long long items = 0;
         for (const auto &l : lines) items += l.first * ((l.second + run - 1) / run);
-        if (items >= (long long)gks::kWinItemsPerSm * ctx->nsm) break;
+        if (items >= (long long)(run > gks::kWinRunFull ? gks::kWinItemsPerSm : gks::kWinItemsMin) * ctx->nsm) break;
     }
     return run;
 }
@@ -378,7 +390,7 @@ int pipe_stage(gks_ctx *ctx, const FieldDev &d, int kind, int dir, long long p0,
         b.wrun = win_run_for(ctx, {{nc * nc, p1 - p0}});
         b.lo = 0;
         b.hi = nc * nc * ((p1 - p0 + b.wrun - 1) / b.wrun);
-        c.grid = (int)std::min<long long>((b.hi + c.block - 1) / c.block, (long long)ctx->nsm * 8);
+        c.grid = (int)((b.hi + c.block - 1) / c.block);
     }
     if (kind == gks::K_RECON) CK(gks::launch_recon(b, dir, ctx->precision, c, ctx->stream));
     else if (kind == gks::K_FLUX) CK(gks::launch_flux(b, dir, ctx->precision, c, ctx->stream));
@@ -747,6 +759,9 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
     if (cudaMalloc(&ctx->d_bits, sizeof(unsigned long long)) != cudaSuccess) return bail(GKS_ENOMEM);
     if (cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess) return bail(GKS_ENOMEM);
     if (cudaMemset(ctx->d_err, 0, sizeof(int)) != cudaSuccess) return bail(GKS_ECUDA);
+    if (cudaMalloc(&ctx->d_queue, 6 * sizeof(unsigned)) != cudaSuccess) return bail(GKS_ENOMEM);
+    if (cudaMemset(ctx->d_queue, 0, 6 * sizeof(unsigned)) != cudaSuccess) return bail(GKS_ECUDA);
+    ctx->batch.queue = ctx->d_queue;
     ctx->batch.fields = ctx->d_fields;
     ctx->batch.nfields = nfields;
     ctx->batch.total = base;
@@ -802,6 +817,7 @@ void gks_destroy(gks_ctx *ctx)
     if (ctx->d_sums) cudaFree(ctx->d_sums);
     if (ctx->d_bits) cudaFree(ctx->d_bits);
     if (ctx->d_err) cudaFree(ctx->d_err);
+    if (ctx->d_queue) cudaFree(ctx->d_queue);
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -1336,7 +1352,6 @@ int gks_autotune(gks_ctx *ctx, int reps)
         if (e == cudaSuccess) e = cudaEventElapsedTime(ms, e0, e1);
         return e;
     };
-    const int mults[2] = {1, 2};
     for (int dir = 0; dir < 3 && rc == GKS_OK; ++dir) {
         for (int kind : {int(gks::K_RECON), int(gks::K_FLUX)}) {
             const int nvar = 3; // reconstruction variants 3-5 repeat 0-2
@@ -1344,7 +1359,7 @@ int gks_autotune(gks_ctx *ctx, int reps)
             // faster one, so that one disturbed measurement does not decide
             std::vector<gks::LaunchCfg> cand;
             for (int v = 0; v < nvar; ++v)
-                for (int m : mults) cand.push_back(persistent(ctx, kind, dir, v, m));
+                for (int m : {kind == gks::K_RECON ? 0 : 1, 2}) cand.push_back(persistent(ctx, kind, dir, v, m));
             std::vector<float> t(cand.size(), 1e30f);
             for (int round = 0; round < 2 && rc == GKS_OK; ++round)
                 for (size_t i = 0; i < cand.size() && rc == GKS_OK; ++i) {

@@ -127,8 +127,7 @@ __device__ __forceinline__ void to_u(double a[5], double U0)
 // bz_ of the equilibrium (:109-117), of B_ (:172-176) and of the flux
 // (:209-212), put into the sums of `src`.
 template <int SIDE, typename Src>
-__device__ __forceinline__ void flux_side(const Src &src, const FluxConst64 &c, double w45, double g5, double p3,
-                                          double p4, double p5)
+__device__ __forceinline__ void flux_side(const Src &src, const FluxConst64 &c)
 {
     double W[5];
     src.template state<SIDE>(W);
@@ -250,8 +249,13 @@ __device__ __forceinline__ void flux_side(const Src &src, const FluxConst64 &c, 
         src.template sum<SIDE>(slot + 3, fma(U2, N0, M3));
         src.template sum<SIDE>(slot + 4, fma(0.5, R, fma(c4, N0, fma(U1, M2, U2 * M3))));
     };
-    collect(Src::kB, std::integral_constant<int, 0>(), m.den * w45, -m.den * g5, 0.0);
-    collect(Src::kF, std::integral_constant<int, 1>(), m.den * p4, -m.den * p5, m.den * p3);
+    // gamma weights (GKMflux.cpp:155-157) and time integrals (GKMflux.cpp:186-190)
+    const double tau = src.get(Src::kTau), ex = src.get(Src::kTau + 1), igm0 = src.get(Src::kTau + 2);
+    const double Pt = tau * (1.0 - ex), tP = tau * Pt;
+    const double g5 = Pt * igm0; // tau gm3
+    collect(Src::kB, std::integral_constant<int, 0>(), m.den * fma(fma(c.dt, ex, -Pt), igm0, g5), -m.den * g5, 0.0);
+    // p3 = P, p4 = -Q - tau P = tau dt ex - 2 tau P, p5 = -tau P
+    collect(Src::kF, std::integral_constant<int, 1>(), m.den * fma(tau, c.dt * ex, -2.0 * tP), m.den * tP, m.den * Pt);
 }
 
 // The flux.  `src` supplies the inputs when they are needed and keeps the sums
@@ -259,13 +263,12 @@ __device__ __forceinline__ void flux_side(const Src &src, const FluxConst64 &c, 
 //   src.state<side>(W)        reconstructed state, left (0) or right (1)
 //   src.slope<side, d>(W, b)  its differences along d = normal, 1st, 2nd transverse
 //   src.cells(WL, WR)         the cell averages either side of the interface
-//   src.sum<side>(slot, v)    side 0 stores, side 1 adds; src.get(slot)
+//   src.sum<side>(slot, v)    side 0 stores, side 1 adds; src.get(slot), src.put(slot, v)
 // mu/p at the left cell = tau_n / tau_d.  Output F[5], integrated over [0, dt].
 template <typename Src>
 __device__ __forceinline__ void gks_flux64(const Src &src, double tau_n, double tau_d, const FluxConst64 &c, double F[5])
 {
     const double dt = c.dt;
-    double tau, ex, om, igm0;
     {
         // collision time with the pressure-jump term (GKMflux.cpp:149-150):
         // rho/lambda = 2p, so w = |p_l - p_r| / (p_l + p_r); with
@@ -280,23 +283,16 @@ __device__ __forceinline__ void gks_flux64(const Src &src, double tau_n, double 
         // tau = N (N r) and 1 / tau = D (D r)
         const double D = tau_d * (a + b);
         const double N = fma(tau_n, a + b, dt * fabs(a - b) * tau_d);
-        const double r = rcp<double>(N * D);
-        tau = N * (N * r);
-        ex = exp(-dt * (D * (D * r)));
-        om = 1.0 - ex;
-        igm0 = rcp_cubic(fma(-tau, om, dt));
+        const double r = rcp_cubic(N * D);
+        const double tau = N * (N * r);
+        const double ex = exp(-dt * (D * (D * r)));
+        src.put(Src::kTau, tau);
+        src.put(Src::kTau + 1, ex);
+        src.put(Src::kTau + 2, rcp_cubic(fma(-tau, 1.0 - ex, dt))); // 1 / gm0
     }
-    // gamma weights (GKMflux.cpp:155-157) and time integrals (GKMflux.cpp:186-190)
-    {
-        const double Pt = tau * om;
-        const double g5 = Pt * igm0; // tau gm3
-        const double w45 = fma(fma(dt, ex, -Pt), igm0, g5);
-        const double Qt = tau * fma(-dt, ex, Pt);
-        const double p4 = fma(-tau, Pt, -Qt), p5 = -tau * Pt;
-        flux_side<0>(src, c, w45, g5, Pt, p4, p5);
-        asm volatile("" ::: "memory"); // one side's state in registers at a time
-        flux_side<1>(src, c, w45, g5, Pt, p4, p5);
-    }
+    flux_side<0>(src, c);
+    asm volatile("" ::: "memory"); // one side's state in registers at a time
+    flux_side<1>(src, c);
     asm volatile("" ::: "memory");
 
     // equilibrium state at the interface (GKMflux.cpp:75-98)
@@ -367,7 +363,8 @@ __device__ __forceinline__ void gks_flux64(const Src &src, double tau_n, double 
         h2[4] = 0.5 * fma(r2, N2, fma(hq, X[2], N4));
     }
     // A_ (phase III, GKMflux.cpp:159-180): its right-hand side in the frame
-    const double Pt = tau * om;
+    const double tau = src.get(Src::kTau), ex = src.get(Src::kTau + 1), igm0 = src.get(Src::kTau + 2);
+    const double Pt = tau * (1.0 - ex);
     double A[5];
     {
         double b[5];

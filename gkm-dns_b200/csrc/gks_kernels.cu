@@ -546,12 +546,12 @@ __device__ __forceinline__ void transverse(const Cell &x, int flags, unsigned &n
     }
 }
 
-// Inputs and running sums of one interface.  All global loads are issued at
-// once when the interface starts, so that their latency overlaps; the values
-// are parked in this thread's own shared-memory slots ([slot][thread], no bank
-// conflicts) until a pass of the flux needs them, and so are the sums the two
-// side passes accumulate for the equilibrium pass, so that only one pass's
-// state is in registers at a time.  Slot q of the rotated frame holds original
+// Inputs and running sums of one interface.  All global loads are issued when
+// the interface starts; the values are parked in this thread's own
+// shared-memory slots ([slot][thread], no bank conflicts) until a pass of the
+// flux needs them, and so are the sums the two side passes accumulate for the
+// equilibrium pass, so that only one pass's state is in registers at a time.
+// Slot q of the rotated frame holds original
 // component perm(q): rho v (y sweep) or rho w (z sweep) moves into slot 1
 // (update.cpp:340-350, 429-439).  DWxl = 2(Wl - WL)/dx, DWxr = 2(WR - Wr)/dx;
 // transverse central differences of the neighbouring lines' states
@@ -576,14 +576,14 @@ struct Records {
     }
 };
 
-// FP64 path (gks_flux64): 50 slots, 400 B per thread, so that eight blocks fit
-// an SM.  The left side's inputs sit in the slots of sums that its own pass
-// writes after it has read them.
+// FP64 path (gks_flux64): 53 slots, 424 B per thread.  The left side's inputs sit
+// in the slots of sums that its own pass writes after it has read them.
 template <int DIR> struct SweepSrc64 {
     static constexpr int kWL = 0, kWR = 5, kWr = 10, kDr = 15; // cell averages, right state, its transverse slopes
     static constexpr int kW0 = 25, kBy = 30, kBz = 35, kB = 40, kF = 45; // sums
     static constexpr int kWl = kBy, kDl = kB;                            // left state, its transverse slopes
-    static constexpr int kSlots = 50;
+    static constexpr int kTau = 50;                                      // tau, exp(-dt/tau), 1/gm0
+    static constexpr int kSlots = 53;
     double (*slots)[kFluxBlock];
 
     __device__ __forceinline__ double &at(int i) const { return slots[i][threadIdx.x]; }
@@ -591,19 +591,30 @@ template <int DIR> struct SweepSrc64 {
     __device__ __forceinline__ void load(const FieldDev &f, unsigned c, unsigned c1, unsigned cn, unsigned cs,
                                          unsigned cf, unsigned cb) const
     {
-        const Records r(f.rec[DIR], c, cn, cs, cf, cb, f.ncell);
+        const double *rec = f.rec[DIR];
 #pragma unroll
         for (int q = 0; q < 5; ++q) {
             const int o = perm<DIR>(q);
-            at(kWL + q) = __ldg(f.W[o] + c);
-            at(kWR + q) = __ldg(f.W[o] + c1);
-            at(kWl + q) = r.r0[o];
-            at(kWr + q) = r.r0[5 + o];
-            at(kDl + q) = r.rn[o] - r.rs[o];
-            at(kDl + 5 + q) = r.rf[o] - r.rb[o];
-            at(kDr + q) = r.rn[5 + o] - r.rs[5 + o];
-            at(kDr + 5 + q) = r.rf[5 + o] - r.rb[5 + o];
+            cp_async8(&at(kWL + q), f.W[o] + c);
+            cp_async8(&at(kWR + q), f.W[o] + c1);
+            cp_async8(&at(kWl + q), rec + 2 * ((o / 2) * f.ncell + c) + o % 2);
+            cp_async8(&at(kWr + q), rec + 2 * (((5 + o) / 2) * f.ncell + c) + (5 + o) % 2);
         }
+        cp_async_commit();
+        double rn[10], rs[10], rf[10], rb[10];
+        get_record(rec, cn, rn, f.ncell);
+        get_record(rec, cs, rs, f.ncell);
+        get_record(rec, cf, rf, f.ncell);
+        get_record(rec, cb, rb, f.ncell);
+#pragma unroll
+        for (int q = 0; q < 5; ++q) {
+            const int o = perm<DIR>(q);
+            at(kDl + q) = rn[o] - rs[o];
+            at(kDl + 5 + q) = rf[o] - rb[o];
+            at(kDr + q) = rn[5 + o] - rs[5 + o];
+            at(kDr + 5 + q) = rf[5 + o] - rb[5 + o];
+        }
+        cp_async_wait<0>();
     }
     template <int SIDE> __device__ __forceinline__ void state(double W[5]) const
     {
@@ -629,6 +640,7 @@ template <int DIR> struct SweepSrc64 {
     }
     template <int SIDE> __device__ __forceinline__ void sum(int i, double v) const { at(i) = SIDE ? at(i) + v : v; }
     __device__ __forceinline__ double get(int i) const { return at(i); }
+    __device__ __forceinline__ void put(int i, double v) const { at(i) = v; }
 };
 
 // Mixed path (gks_flux): the left state and its slopes stay in registers.
@@ -707,41 +719,8 @@ template <> struct FluxPark<1> {
     float dw[15][kFluxBlock];
 };
 
-template <int DIR, int PREC>
-__device__ __forceinline__ void flux_item(const FieldDev &f, long long it, FluxPark<PREC> &park)
+template <int DIR> __device__ __forceinline__ void store_flux(const FieldDev &f, unsigned c, double F[5])
 {
-    const Cell x = decode(unsigned(it - f.base), f);
-    unsigned cn, cs, cf, cb;
-    transverse<DIR>(x, f.flags, cn, cs, cf, cb);
-    // collision time mu / p at the left cell (update.cpp:262-264), stored by
-    // this step's x-sweep reconstruction
-    double F[5];
-    if constexpr (PREC == 0) {
-        SweepSrc64<DIR> src{park.slots};
-        src.load(f, x.c, along<DIR>(x, 1), cn, cs, cf, cb);
-        const double tau_n = __ldg(f.tau[0] + x.c), tau_d = __ldg(f.tau[1] + x.c);
-        const FluxConst64 fc = {f.dt,  f.gm1, f.igm1,  f.shig,  f.rlg,   f.ksn,   f.kst,
-                                f.kA4, f.prm1, f.kd[0], f.kd[1], f.kd[2], f.kd[3], f.kd[4]};
-        gks_flux64(src, tau_n, tau_d, fc, F);
-    } else {
-        SweepSrc<DIR> src;
-        src.park_dw = park.dw;
-        src.park_w = park.w;
-        src.sum_d = park.sum;
-        src.load(f, x.c, along<DIR>(x, 1), cn, cs, cf, cb);
-        const double tau_n = __ldg(f.tau[0] + x.c), tau_d = __ldg(f.tau[1] + x.c);
-        FluxConst fc;
-        fc.gm1 = f.gm1;
-        fc.hig = f.hig;
-        fc.dt = f.dt;
-        fc.dx = f.dx;
-        fc.ks[0] = f.ksn;
-        fc.ks[1] = fc.ks[2] = f.kst;
-        fc.kA = f.kA;
-        fc.hK2 = f.hK2;
-        fc.kf = {f.kf[0], f.kf[1], f.kf[2], f.kf[3]};
-        gks_flux(src, tau_n, tau_d, fc, F);
-    }
     constexpr int ROT = DIR == 0 ? 0 : (DIR == 1 ? 2 : 3);
     if (ROT) {
         const double t = F[1];
@@ -749,27 +728,109 @@ __device__ __forceinline__ void flux_item(const FieldDev &f, long long it, FluxP
         F[ROT] = t;
     }
 #pragma unroll
-    for (int q = 0; q < 5; ++q) f.F[DIR * 5 + q][x.c] = F[q];
+    for (int q = 0; q < 5; ++q) f.F[DIR * 5 + q][c] = F[q];
+}
+
+// FP64: the flux at cell c.
+template <int DIR>
+__device__ __forceinline__ void flux_item64(const FieldDev &f, unsigned c, const SweepSrc64<DIR> &src)
+{
+    const Cell x = decode(c, f);
+    unsigned cn, cs, cf, cb;
+    transverse<DIR>(x, f.flags, cn, cs, cf, cb);
+    src.load(f, c, along<DIR>(x, 1), cn, cs, cf, cb);
+    // collision time mu / p at the left cell (update.cpp:262-264), stored by
+    // this step's x-sweep reconstruction
+    const double tau_n = __ldg(f.tau[0] + c), tau_d = __ldg(f.tau[1] + c);
+    const FluxConst64 fc = {f.dt,  f.gm1,  f.igm1,  f.shig,  f.rlg,   f.ksn,   f.kst,
+                            f.kA4, f.prm1, f.kd[0], f.kd[1], f.kd[2], f.kd[3], f.kd[4]};
+    double F[5];
+    gks_flux64(src, tau_n, tau_d, fc, F);
+    store_flux<DIR>(f, c, F);
+}
+
+// Mixed: all global loads are issued at once when the interface starts, so
+// that their latency overlaps.
+template <int DIR>
+__device__ __forceinline__ void flux_item(const FieldDev &f, unsigned c, FluxPark<1> &park)
+{
+    const Cell x = decode(c, f);
+    unsigned cn, cs, cf, cb;
+    transverse<DIR>(x, f.flags, cn, cs, cf, cb);
+    SweepSrc<DIR> src;
+    src.park_dw = park.dw;
+    src.park_w = park.w;
+    src.sum_d = park.sum;
+    src.load(f, c, along<DIR>(x, 1), cn, cs, cf, cb);
+    const double tau_n = __ldg(f.tau[0] + c), tau_d = __ldg(f.tau[1] + c);
+    FluxConst fc;
+    fc.gm1 = f.gm1;
+    fc.hig = f.hig;
+    fc.dt = f.dt;
+    fc.dx = f.dx;
+    fc.ks[0] = f.ksn;
+    fc.ks[1] = fc.ks[2] = f.kst;
+    fc.kA = f.kA;
+    fc.hK2 = f.hK2;
+    fc.kf = {f.kf[0], f.kf[1], f.kf[2], f.kf[3]};
+    double F[5];
+    gks_flux(src, tau_n, tau_d, fc, F);
+    store_flux<DIR>(f, c, F);
 }
 
 // A batch of one field reads the field's descriptor from the launch
 // parameters (b.one: constant-bank operands, nothing loaded per interface);
 // an ensemble looks each interface's field up in the device array.
+//
+// Mixed: grid-stride loop.  FP64: one wave of resident blocks whose warps draw
+// chunks of 32 interfaces from a queue: the first is the warp's own number,
+// the next ones come from a counter in global memory, asked for one chunk
+// ahead.  (With equal static shares the schedulers run some warps ahead of
+// others and an SM's last fifth passes at falling occupancy: 9.7 of 12 warps
+// active on average, 11.8 with the queue; 1677 -> 1572 us per sweep at 256^3.
+// The mixed kernel gains nothing, 1466 -> 1515 us.)  The warp that is last to find the queue empty sets the counters
+// back to zero for the next launch.
 template <int DIR, int PREC, int REGS>
 __global__ void __launch_bounds__(kFluxBlock) __maxnreg__(REGS) k_flux(Batch b)
 {
     __shared__ FluxPark<PREC> park;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    if (b.nfields == 1) {
-        const long long end = b.hi < b.one.ncell ? b.hi : b.one.ncell; // alignment padding after the field
-        for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < end; it += stride)
-            flux_item<DIR, PREC>(b.one, it, park);
+    const long long end = b.nfields == 1 && b.one.ncell < b.hi ? b.one.ncell : b.hi; // alignment padding after the field
+    if constexpr (PREC == 0) {
+        const int lane = threadIdx.x & 31;
+        const unsigned nwarps = gridDim.x * (kFluxBlock / 32);
+        const unsigned chunks = unsigned((end - b.lo + 31) >> 5);
+        unsigned *queue = b.queue + 2 * DIR;
+        const SweepSrc64<DIR> src{park.slots};
+        unsigned chunk = (blockIdx.x * kFluxBlock + threadIdx.x) >> 5;
+        while (chunk < chunks) {
+            unsigned next = 0;
+            if (lane == 0) next = nwarps + atomicAdd(queue, 1u);
+            const long long it = b.lo + (long long)chunk * 32 + lane;
+            if (b.nfields == 1) {
+                if (it < end) flux_item64<DIR>(b.one, unsigned(it), src);
+            } else {
+                const FieldDev &f = b.fields[field_of(b.fields, b.nfields, it)];
+                if (it - f.base < f.ncell) flux_item64<DIR>(f, unsigned(it - f.base), src); // alignment padding after the field
+            }
+            chunk = __shfl_sync(0xffffffffu, next, 0);
+        }
+        if (lane == 0 && atomicAdd(queue + 1, 1u) == nwarps - 1) {
+            queue[0] = 0;
+            queue[1] = 0;
+        }
         return;
-    }
-    for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < b.hi; it += stride) {
-        const FieldDev &f = b.fields[field_of(b.fields, b.nfields, it)];
-        if (it - f.base >= f.ncell) continue; // alignment padding after the field
-        flux_item<DIR, PREC>(f, it, park);
+    } else {
+        const long long stride = (long long)gridDim.x * blockDim.x;
+        if (b.nfields == 1) {
+            for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < end; it += stride)
+                flux_item<DIR>(b.one, unsigned(it), park);
+            return;
+        }
+        for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < b.hi; it += stride) {
+            const FieldDev &f = b.fields[field_of(b.fields, b.nfields, it)];
+            if (it - f.base >= f.ncell) continue; // alignment padding after the field
+            flux_item<DIR>(f, unsigned(it - f.base), park);
+        }
     }
 }
 
@@ -1246,7 +1307,7 @@ cudaError_t occ(KernelT k, int block, int *n)
 // and caps at 168, as for 6 blocks.  The tuner picks one variant per kernel,
 // precision and sweep.  Every variant gives bit-identical results.
 constexpr int kReconMinb[3] = {3, 4, 5};
-constexpr int kFluxRegs[2][kFluxVariants] = {{168, 144, 128}, {200, 168, 128}};
+constexpr int kFluxRegs[kFluxVariants] = {200, 168, 128};
 
 // The item range of a launch (all items of its kind when b.hi < 0) and the
 // blocks it needs: at most cfg.grid, no more than the range fills.
@@ -1296,9 +1357,9 @@ cudaError_t flux_go(Batch b, LaunchCfg cfg, cudaStream_t st)
     if (b.hi <= b.lo) return cudaSuccess;
     const int g = range_grid(cfg.grid, b.hi - b.lo, cfg.block);
     switch (cfg.variant) {
-    case 1: k_flux<DIR, PREC, kFluxRegs[PREC][1]><<<g, cfg.block, 0, st>>>(b); break;
-    case 2: k_flux<DIR, PREC, kFluxRegs[PREC][2]><<<g, cfg.block, 0, st>>>(b); break;
-    default: k_flux<DIR, PREC, kFluxRegs[PREC][0]><<<g, cfg.block, 0, st>>>(b); break;
+    case 1: k_flux<DIR, PREC, kFluxRegs[1]><<<g, cfg.block, 0, st>>>(b); break;
+    case 2: k_flux<DIR, PREC, kFluxRegs[2]><<<g, cfg.block, 0, st>>>(b); break;
+    default: k_flux<DIR, PREC, kFluxRegs[0]><<<g, cfg.block, 0, st>>>(b); break;
     }
     return cudaGetLastError();
 }
@@ -1317,9 +1378,9 @@ cudaError_t occ_kind(int kind, int variant, int block, int *n)
             return occ(k_recon_zline<PREC, kReconMinb[0]>, block, n);
         }
     }
-    if (variant == 1) return occ(k_flux<DIR, PREC, kFluxRegs[PREC][1]>, block, n);
-    if (variant == 2) return occ(k_flux<DIR, PREC, kFluxRegs[PREC][2]>, block, n);
-    return occ(k_flux<DIR, PREC, kFluxRegs[PREC][0]>, block, n);
+    if (variant == 1) return occ(k_flux<DIR, PREC, kFluxRegs[1]>, block, n);
+    if (variant == 2) return occ(k_flux<DIR, PREC, kFluxRegs[2]>, block, n);
+    return occ(k_flux<DIR, PREC, kFluxRegs[0]>, block, n);
 }
 
 template <int PREC>

@@ -71,13 +71,11 @@ constexpr int kNoWrap = 1 << 30;
 // kItemAlign consecutive items never spans two fields.
 constexpr int kItemAlign = 256;
 
-// Longest run of interfaces per work item of the windowed x / y
-// reconstruction, for either precision (0 FP64, 1 mixed; 64 measured fastest
-// on B200 at 256^3 for both).  A batch halves it, down to kWinRunMin, while it has fewer than
-// kWinItemsPerSm items per SM, so that small fields still fill the GPU.
-__host__ __device__ constexpr int win_run(int) { return 64; }
-constexpr int kWinRunMin = 8;
-constexpr int kWinItemsPerSm = 768;
+// Run lengths of the windowed x / y reconstruction (interfaces per work item):
+// at most kWinRunMax; above kWinRunFull a batch must keep kWinItemsPerSm items
+// per SM, below it kWinItemsMin (seven warps).
+constexpr int kWinRunMax = 64, kWinRunFull = 8;
+constexpr int kWinItemsPerSm = 768, kWinItemsMin = 220;
 
 struct Batch {
     FieldDev *fields; // device array
@@ -89,6 +87,10 @@ struct Batch {
     // work items a launch processes: [lo, hi) of the launched kernel's item
     // space; hi < 0 means all of them (the launchers fill the range in)
     long long lo = 0, hi = -1;
+    // flux work queues, one pair of counters per sweep (k_flux): next chunk beyond
+    // the first of every warp, warps that found the queue empty; both zero
+    // between launches
+    unsigned *queue = nullptr;
     // y reconstruction over the interfaces of planes [wy0, wy1) of the one field
     // (wy1 > 0), in runs of wrun: its items are then nc * nrun * nc
     int wy0 = 0, wy1 = 0, wrun = 0;
