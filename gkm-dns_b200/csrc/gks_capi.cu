@@ -67,6 +67,7 @@ struct gks_ctx {
     cudaStream_t stream = nullptr;
     bool own_stream = false;
     cudaGraphExec_t graph = nullptr;
+    int direct = 0; // steps launched one by one since the last change of the step (kDirectSteps)
     double *d_stage = nullptr;
     size_t stage_elems = 0;
     // gks_evolve: the padded staging of the downloaded state, the copy streams
@@ -81,6 +82,11 @@ struct gks_ctx {
     int *d_err = nullptr;
     unsigned *d_queue = nullptr;
     gks::LaunchCfg cfg[gks::K_KINDS][3];
+    // concurrent sweeps (kSweepCells): the y and z sweeps' streams in a captured
+    // step and the events that fork and join them
+    bool concurrent = false;
+    cudaStream_t side[2] = {nullptr, nullptr};
+    cudaEvent_t fork[2] = {nullptr, nullptr}, join[2] = {nullptr, nullptr};
     std::string err;
 };
 
@@ -109,6 +115,7 @@ void drop_graph(gks_ctx *ctx)
         cudaGraphExecDestroy(ctx->graph);
         ctx->graph = nullptr;
     }
+    ctx->direct = 0;
 }
 
 int check_field(gks_ctx *ctx, int f)
@@ -217,6 +224,15 @@ void choose_launch(gks_ctx *ctx)
         }
 }
 
+// A batch of up to this many cells keeps a reconstruction buffer per sweep
+// (20 more doubles per cell, at most 168 MB) and runs its three sweeps side by
+// side in the captured step: three dependent levels instead of seven, and the
+// sweeps' last waves overlap.  us per step, one after the other / side by
+// side, FP64: 16^3 35.0 / 23.7, 32^3 45.4 / 36.0, 64^3 152 / 137, 100^3 499 / 477,
+// 128^3 939 / 915; mixed: 37.3 / 30.0 at 32^3, 428 / 415 at 100^3, 826 / 837 at
+// 128^3.
+constexpr long long kSweepCells = 1LL << 20;
+
 // Tuned configurations of this process, per device / precision / flags / sizes.
 std::mutex g_tune_mu;
 std::map<std::string, std::array<gks::LaunchCfg, gks::K_KINDS * 3>> g_tune_cache;
@@ -237,6 +253,27 @@ int record_slab_step(gks_ctx *ctx);
 int record_step(gks_ctx *ctx)
 {
     if (ctx->fh[0].slab) return record_slab_step(ctx);
+    if (ctx->concurrent) {
+        // the three sweeps side by side; every flux reads the mu/p that the x
+        // reconstruction stores
+        cudaStream_t st[3] = {ctx->stream, ctx->side[0], ctx->side[1]};
+        CK(cudaEventRecord(ctx->fork[0], st[0]));
+        for (int dir = 0; dir < 3; ++dir) {
+            if (dir) CK(cudaStreamWaitEvent(st[dir], ctx->fork[0], 0));
+            CK(gks::launch_recon(ctx->batch, dir, ctx->precision, ctx->cfg[gks::K_RECON][dir], st[dir]));
+            if (dir == 0) CK(cudaEventRecord(ctx->fork[1], st[0]));
+        }
+        for (int dir = 0; dir < 3; ++dir) {
+            if (dir) CK(cudaStreamWaitEvent(st[dir], ctx->fork[1], 0));
+            CK(gks::launch_flux(ctx->batch, dir, ctx->precision, ctx->cfg[gks::K_FLUX][dir], st[dir]));
+            if (dir) {
+                CK(cudaEventRecord(ctx->join[dir - 1], st[dir]));
+                CK(cudaStreamWaitEvent(st[0], ctx->join[dir - 1], 0));
+            }
+        }
+        CK(gks::launch_update(ctx->batch, ctx->cfg[gks::K_UPDATE][0], st[0]));
+        return GKS_OK;
+    }
     for (int dir = 0; dir < 3; ++dir) {
         CK(gks::launch_recon(ctx->batch, dir, ctx->precision, ctx->cfg[gks::K_RECON][dir], ctx->stream));
         CK(gks::launch_flux(ctx->batch, dir, ctx->precision, ctx->cfg[gks::K_FLUX][dir], ctx->stream));
@@ -244,6 +281,11 @@ int record_step(gks_ctx *ctx)
     CK(gks::launch_update(ctx->batch, ctx->cfg[gks::K_UPDATE][0], ctx->stream));
     return GKS_OK;
 }
+
+// Steps launched kernel by kernel before a step is captured: capturing and
+// instantiating it costs the host as much as about ten such steps, and a new
+// dt (a caller that takes one every step) asks for it again.
+constexpr int kDirectSteps = 16;
 
 int build_graph(gks_ctx *ctx)
 {
@@ -272,9 +314,10 @@ int build_graph(gks_ctx *ctx)
 //
 // Planes are counted in an unwrapped y coordinate u in [-3, nc - 3) (plane
 // u mod nc), uploaded in increasing u: first the three planes below 0 (nc-3
-// .. nc-1), then thin slabs (4, 4, 8 planes), so that the first updated
-// planes start down early, slabs of about nc / kPipeSlabs planes, and thin
-// slabs again (8, 4, 4), so that little work is left after the last upload.
+// .. nc-1), then, in a large field, thin slabs (4, 4, 8 planes), so that the
+// first updated planes start down early, slabs of about nc / kPipeSlabs planes,
+// and thin slabs again (8, 4, 4), so that little work is left after the last
+// upload; a smaller field goes in fewer, thicker slabs (kPipeSlabCells).
 // The y ghost planes go down with the planes they copy: the top ones
 // (images of planes 0-2) early, the bottom ones (nc-3 .. nc-1) last.  With F the uploaded
 // frontier, the stages advance as far as the planes they read allow (each
@@ -290,15 +333,24 @@ int build_graph(gks_ctx *ctx)
 // is still read by later slabs' stencils); afterwards the two swap.  The
 // sweeps keep separate reconstruction buffers, as their slabs interleave.
 // ---------------------------------------------------------------------------
+// A slab costs about a dozen launches and copies to enqueue whatever its size,
+// so it has at least kPipeSlabCells padded cells (0.35 ms of one PCIe
+// direction) up to kPipeMaxPlanes planes, and a field below kPipeMinNc goes up,
+// through a step and down in one piece.  us per call by planes per
+// slab, pinned: 64^3 1: 1351, 8: 1034, 32: 672, one piece 708; 128^3 4: 3759, 12:
+// 3027, 24: 2864, 48: 3221, one piece 4592; 200^3 8: 8935, 16: 8935, 32: 9480; 48^3
+// 8: 591, 32: 418, one piece 370; 24^3 4: 467, one piece 133.
 constexpr int kPipeSlabs = 24;
-constexpr int kPipeMinNc = 16;
+constexpr long long kPipeSlabCells = 430000, kPipeMaxPlanes = 32;
+constexpr int kPipeMinNc = 56;
 constexpr int kPipeEvents = kPipeSlabs + 16; // events per direction: at least the slabs + 1
 
 // The upload slabs of a field of nc planes, in unwrapped planes (see above).
 std::vector<std::pair<long long, long long>> pipe_slabs(long long nc)
 {
     std::vector<std::pair<long long, long long>> s{{-3, 0}};
-    const long long n = nc - 3, S = (n + kPipeSlabs - 1) / kPipeSlabs;
+    const long long n = nc - 3, P = (nc + 6) * (nc + 6);
+    const long long S = std::max((n + kPipeSlabs - 1) / kPipeSlabs, std::min(kPipeMaxPlanes, (kPipeSlabCells + P - 1) / P));
     const long long head[3] = {4, 4, 8}, tail[3] = {8, 4, 4};
     long long a = 0;
     if (n >= 32 + 2 * S) {
@@ -322,7 +374,8 @@ int ensure_pipe(gks_ctx *ctx, FieldHost &h)
 {
     const size_t n = (size_t)h.phys.nc * h.phys.nc * h.phys.nc;
     if (!h.pipe) {
-        if (cudaMalloc(&h.pipe, (25 * n + 2) * sizeof(double)) != cudaSuccess) {
+        const size_t elems = ctx->concurrent ? 5 * n : 25 * n + 2; // a field with a buffer per sweep needs no others
+        if (cudaMalloc(&h.pipe, elems * sizeof(double)) != cudaSuccess) {
             h.pipe = nullptr;
             return fail(ctx, GKS_ENOMEM, "pipelined-step buffers allocation failed");
         }
@@ -458,9 +511,11 @@ int evolve_slabs(gks_ctx *ctx, double *const W[5])
     FieldDev d = h.dev;
     const size_t n = (size_t)nc * nc * nc;
     for (int q = 0; q < 5; ++q) d.Wout[q] = h.spare[q];
-    const size_t r0 = (5 * n + 1) & ~(size_t)1; // 16-byte aligned pair arrays
-    d.rec[1] = h.pipe + r0;
-    d.rec[2] = h.pipe + r0 + 10 * n;
+    if (!ctx->concurrent) {
+        const size_t r0 = (5 * n + 1) & ~(size_t)1; // 16-byte aligned pair arrays
+        d.rec[1] = h.pipe + r0;
+        d.rec[2] = h.pipe + r0 + 10 * n;
+    }
     CK(cudaMemcpyAsync(ctx->d_fields, &d, sizeof(FieldDev), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream)); // the h2d stream writes the stage the last call may still read
 
@@ -643,6 +698,14 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
     for (int f = 0; f < nfields; ++f)
         lines.push_back({(long long)(slab ? slab + 6 : phys[f].nc) * phys[f].nc, phys[f].nc});
     const int run = win_run_for(ctx, lines);
+    long long cells = 0;
+    for (int f = 0; f < nfields; ++f) cells += (long long)phys[f].nc * phys[f].nc * phys[f].nc;
+    ctx->concurrent = !slab && cells <= kSweepCells;
+    for (int i = 0; i < 2 && ctx->concurrent; ++i)
+        if (cudaStreamCreateWithFlags(&ctx->side[i], cudaStreamNonBlocking) != cudaSuccess ||
+            cudaEventCreateWithFlags(&ctx->fork[i], cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&ctx->join[i], cudaEventDisableTiming) != cudaSuccess)
+            return bail(GKS_ECUDA);
     long long base = 0, wbase = 0, zbase = 0;
     const double pi = std::atan(1.0) * 4.0; // param.h:14
     for (int f = 0; f < nfields; ++f) {
@@ -653,17 +716,17 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
         const int ny = slab ? slab + 6 : p.nc; // stored planes
         const long long n = (long long)ny * p.nc * p.nc;
         // state 5 n, reconstruction pairs 10 n (from an even offset: 16-byte
-        // aligned), fluxes 15 n, mu/p 2 n
-        const long long r0 = (5 * n + 1) & ~1LL;
-        const size_t elems = (size_t)(r0 + 27 * n);
+        // aligned) for all sweeps or for each, fluxes 15 n, mu/p 2 n
+        const long long r0 = (5 * n + 1) & ~1LL, nrec = ctx->concurrent ? 30 : 10;
+        const size_t elems = (size_t)(r0 + (nrec + 17) * n);
         if (cudaMalloc(&h.mem, elems * sizeof(double)) != cudaSuccess) return bail(GKS_ENOMEM);
         if (cudaMemset(h.mem, 0, elems * sizeof(double)) != cudaSuccess) return bail(GKS_ECUDA);
         FieldDev &d = h.dev;
         memset(&d, 0, sizeof(d));
         for (int q = 0; q < 5; ++q) d.W[q] = d.Wout[q] = h.mem + q * n;
-        for (int sw = 0; sw < 3; ++sw) d.rec[sw] = h.mem + r0;
-        for (int q = 0; q < 15; ++q) d.F[q] = h.mem + r0 + (10 + q) * n;
-        for (int q = 0; q < 2; ++q) d.tau[q] = h.mem + r0 + (25 + q) * n;
+        for (int sw = 0; sw < 3; ++sw) d.rec[sw] = h.mem + r0 + (ctx->concurrent ? 10 * sw * n : 0);
+        for (int q = 0; q < 15; ++q) d.F[q] = h.mem + r0 + (nrec + q) * n;
+        for (int q = 0; q < 2; ++q) d.tau[q] = h.mem + r0 + (nrec + 15 + q) * n;
         // spline coefficients: x / z lines of nt nodes, y lines of nty (a
         // slab's own when it is a slab)
         const int nt = p.nc + 6, nty = slab ? ny : nt;
@@ -775,6 +838,46 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
     return GKS_OK;
 }
 
+// Copy field f's five padded arrays between W and the staging buffer on the
+// context's stream: in one copy when they lie one after another, else (or when
+// such a block is page-locked in several pieces, which one copy refuses) in five.
+int copy_padded(gks_ctx *ctx, int f, double *const W[5], cudaMemcpyKind kind)
+{
+    const size_t Nt = host_elems(ctx, f) / 5;
+    const bool up = kind == cudaMemcpyHostToDevice;
+    bool contiguous = true;
+    for (int q = 1; q < 5; ++q) contiguous = contiguous && W[q] == W[0] + q * Nt;
+    if (contiguous) {
+        if (cudaMemcpyAsync(up ? ctx->d_stage : W[0], up ? W[0] : ctx->d_stage, 5 * Nt * sizeof(double), kind, ctx->stream) ==
+            cudaSuccess)
+            return GKS_OK;
+        cudaGetLastError();
+    }
+    for (int q = 0; q < 5; ++q) {
+        double *stage = ctx->d_stage + q * Nt;
+        CK(cudaMemcpyAsync(up ? stage : W[q], up ? W[q] : stage, Nt * sizeof(double), kind, ctx->stream));
+    }
+    return GKS_OK;
+}
+
+// Upload / download of field f, enqueued on the context's stream.
+int enqueue_upload(gks_ctx *ctx, int f, double *const W[5])
+{
+    int rc = ensure_stage(ctx, f);
+    if (!rc) rc = copy_padded(ctx, f, W, cudaMemcpyHostToDevice);
+    if (rc) return rc;
+    CK(gks::launch_gather(ctx->fh[f].dev, ctx->d_stage, ctx->nsm, ctx->stream));
+    return GKS_OK;
+}
+
+int enqueue_download(gks_ctx *ctx, int f, double *const W[5])
+{
+    const int rc = ensure_stage(ctx, f);
+    if (rc) return rc;
+    CK(gks::launch_scatter(ctx->fh[f].dev, ctx->d_stage, ctx->nsm, ctx->stream));
+    return copy_padded(ctx, f, W, cudaMemcpyDeviceToHost);
+}
+
 } // namespace
 
 extern "C" {
@@ -818,6 +921,11 @@ void gks_destroy(gks_ctx *ctx)
     if (ctx->d_bits) cudaFree(ctx->d_bits);
     if (ctx->d_err) cudaFree(ctx->d_err);
     if (ctx->d_queue) cudaFree(ctx->d_queue);
+    for (int i = 0; i < 2; ++i) {
+        if (ctx->side[i]) cudaStreamDestroy(ctx->side[i]);
+        if (ctx->fork[i]) cudaEventDestroy(ctx->fork[i]);
+        if (ctx->join[i]) cudaEventDestroy(ctx->join[i]);
+    }
     if (ctx->own_stream && ctx->stream) cudaStreamDestroy(ctx->stream);
     delete ctx;
 }
@@ -830,11 +938,7 @@ int gks_upload(gks_ctx *ctx, int f, double *const W[5])
     for (int q = 0; q < 5; ++q)
         if (!W[q]) return fail(ctx, GKS_EINVAL, "null component pointer");
     CK(cudaSetDevice(ctx->device));
-    if ((rc = ensure_stage(ctx, f))) return rc;
-    const size_t Nt = host_elems(ctx, f) / 5;
-    for (int q = 0; q < 5; ++q)
-        CK(cudaMemcpyAsync(ctx->d_stage + q * Nt, W[q], Nt * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
-    CK(gks::launch_gather(ctx->fh[f].dev, ctx->d_stage, ctx->nsm, ctx->stream));
+    if ((rc = enqueue_upload(ctx, f, W))) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->fh[f].uploaded = true;
     return GKS_OK;
@@ -848,11 +952,7 @@ int gks_download(gks_ctx *ctx, int f, double *const W[5])
     for (int q = 0; q < 5; ++q)
         if (!W[q]) return fail(ctx, GKS_EINVAL, "null component pointer");
     CK(cudaSetDevice(ctx->device));
-    if ((rc = ensure_stage(ctx, f))) return rc;
-    const size_t Nt = host_elems(ctx, f) / 5;
-    CK(gks::launch_scatter(ctx->fh[f].dev, ctx->d_stage, ctx->nsm, ctx->stream));
-    for (int q = 0; q < 5; ++q)
-        CK(cudaMemcpyAsync(W[q], ctx->d_stage + q * Nt, Nt * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+    if ((rc = enqueue_download(ctx, f, W))) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     return GKS_OK;
 }
@@ -871,12 +971,15 @@ int gks_evolve(gks_ctx *ctx, int f, double *const W[5], int nsteps)
     CK(cudaSetDevice(ctx->device));
     if (ctx->nfields == 1 && nsteps == 1 && ctx->fh[f].phys.nc >= kPipeMinNc && !ctx->fh[f].slab)
         return evolve_pipelined(ctx, W);
-    // several fields or steps: upload, the captured steps, download
-    if ((rc = gks_upload(ctx, f, W))) return rc;
+    // several fields or steps: upload, the captured steps, download, in stream order
+    if ((rc = enqueue_upload(ctx, f, W))) return rc;
+    ctx->fh[f].uploaded = true;
     for (int g = 0; g < ctx->nfields; ++g)
         if (!ctx->fh[g].uploaded) return fail(ctx, GKS_ESTATE, "evolve with field " + std::to_string(g) + " not uploaded");
     if ((rc = gks_step(ctx, nsteps))) return rc;
-    return gks_download(ctx, f, W);
+    if ((rc = enqueue_download(ctx, f, W))) return rc;
+    CK(cudaStreamSynchronize(ctx->stream));
+    return GKS_OK;
 }
 
 int gks_host_register(void *p, size_t bytes, int *registered)
@@ -946,11 +1049,18 @@ int gks_step(gks_ctx *ctx, int nsteps)
         if (!ctx->fh[f].have_dt) return fail(ctx, GKS_ESTATE, "step before dt of field " + std::to_string(f));
     }
     CK(cudaSetDevice(ctx->device));
-    if (!ctx->graph) {
-        int rc = build_graph(ctx);
-        if (rc) return rc;
+    for (int s = 0; s < nsteps; ++s) {
+        if (!ctx->graph) {
+            const bool direct = ctx->direct < kDirectSteps;
+            const int rc = direct ? record_step(ctx) : build_graph(ctx);
+            if (rc) return rc;
+            if (direct) {
+                ++ctx->direct;
+                continue;
+            }
+        }
+        CK(cudaGraphLaunch(ctx->graph, ctx->stream));
     }
-    for (int s = 0; s < nsteps; ++s) CK(cudaGraphLaunch(ctx->graph, ctx->stream));
     return GKS_OK;
 }
 

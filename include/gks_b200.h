@@ -122,7 +122,7 @@ int gks_download(gks_ctx *ctx, int f, double *const W[5]);
  * moves in one pitched copy per direction instead of five; page-lock such a
  * block as one range (gks_host_register) to keep that.  The first such call
  * allocates 25 nc^3 + 5 (nc+6)^3 doubles of pipeline buffers for the context
- * (4.1 GB at 256^3).  Otherwise (an ensemble, nsteps > 1, nc < 16) it is
+ * (4.1 GB at 256^3; 20 nc^3 fewer up to 101^3).  Otherwise (an ensemble, nsteps > 1, nc < 56) it is
  * gks_upload + gks_step + gks_download.  Results are bit-identical either way.
  * After a failure the field's device state is undefined: upload it again. */
 int gks_evolve(gks_ctx *ctx, int f, double *const W[5], int nsteps);
@@ -143,8 +143,9 @@ int gks_set_dt(gks_ctx *ctx, int f, double dt);
 
 /* Advance every field of the context by nsteps single-stage steps
  * (evolveEulerian, update.cpp:194-199): three fused reconstruction + flux
- * sweeps and the conservative update per step, captured once as a CUDA
- * graph.  Asynchronous on the context's stream. */
+ * sweeps and the conservative update per step; the first few are launched
+ * kernel by kernel, then a step is captured as a CUDA graph.  Asynchronous on
+ * the context's stream. */
 int gks_step(gks_ctx *ctx, int nsteps);
 
 /* Diagnostics of field f on the current state (synchronises). */
