@@ -110,20 +110,23 @@ __device__ __forceinline__ void store_tau(const FieldDev &f, unsigned c, const d
     f.tau[1][c] = d;
 }
 
-__device__ __forceinline__ double temperature(const double W[5], double cT)
+// FP64: 1/rho from rcp_cubic.  Mixed: correctly rounded (its FP32 steps round
+// differences of these values, so that path's double arithmetic is kept as it
+// is: a last-place change flips an FP32 rounding now and then).
+template <int PREC> __device__ __forceinline__ double temperature(const double W[5], double cT)
 {
     // (gam-1)(E/rho - |m|^2/(2 rho^2))/R, update.cpp:560
-    const double ri = rcp_cubic(W[0]);
+    const double ri = PREC == 0 ? rcp_cubic(W[0]) : __drcp_rn(W[0]);
     const double ke = fma(W[1], W[1], fma(W[2], W[2], W[3] * W[3]));
     return cT * fma(-0.5 * ke, ri * ri, W[4] * ri);
 }
 
 // rho E from the reconstructed density, momentum and temperature
-// (update.cpp:618-619): rho T R/(gam-1) + |m|^2 / (2 rho).
-__device__ __forceinline__ double energy(const double w[4], double T, double icT)
+// (update.cpp:618-619): rho T R/(gam-1) + |m|^2 / (2 rho), ri = 1/rho.
+__device__ __forceinline__ double energy(const double w[4], double T, double ri, double icT)
 {
     const double ke = fma(w[1], w[1], fma(w[2], w[2], w[3] * w[3]));
-    return fma(w[0] * T, icT, (0.5 * ke) * rcp_cubic(w[0]));
+    return fma(w[0] * T, icT, (0.5 * ke) * ri);
 }
 
 // The reconstruction record of cell c: Wl[0..4] then Wr[0..4] as five
@@ -170,8 +173,8 @@ __device__ __forceinline__ void cell_states(const double (&d)[5][6], const doubl
         wr[q] = g[q] + dr;
     }
     if (direct) return;
-    wl[4] = energy(wl, wl[4], icT);
-    wr[4] = energy(wr, wr[4], icT);
+    wl[4] = energy(wl, wl[4], rcp_cubic(wl[0]), icT);
+    wr[4] = energy(wr, wr[4], rcp_cubic(wr[0]), icT);
 }
 
 // Mixed: both states of one interface from its stencil's quantities s(a, q),
@@ -202,8 +205,9 @@ __device__ __forceinline__ void interface_states(const SG &s, bool direct, doubl
     wl[4] = c0 + double(dl);
     wr[4] = c0 + double(dr);
     if (direct) return;
-    wl[4] = energy(wl, wl[4], icT);
-    wr[4] = energy(wr, wr[4], icT);
+    const double r = __drcp_rn(wl[0] * wr[0]); // one reciprocal for both densities
+    wl[4] = energy(wl, wl[4], wr[0] * r, icT);
+    wr[4] = energy(wr, wr[4], wl[0] * r, icT);
 }
 
 // Asynchronous 8-byte copy global -> shared (cp.async), its groups and waits.
@@ -269,7 +273,7 @@ __global__ void __launch_bounds__(kReconBlock, MINB) k_recon_zline(Batch b)
         auto put = [&](int col) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) tile[q][col] = w[q];
-            tile[4][col] = direct ? w[4] : temperature(w, cT);
+            tile[4][col] = direct ? w[4] : temperature<PREC>(w, cT);
         };
         if (lane < 6) { // cells -3 .. 2
             load(lane - 3);
@@ -421,7 +425,7 @@ __global__ void __launch_bounds__(kReconBlock, MINB) k_recon_win(Batch b)
             for (int q = 0; q < 5; ++q) w[q] = ring[pc & (NR - 1)][q][tid];
 #pragma unroll
             for (int q = 0; q < 4; ++q) g[q] = w[q];
-            g[4] = direct ? w[4] : temperature(w, cT);
+            g[4] = direct ? w[4] : temperature<PREC>(w, cT);
         };
         if constexpr (PREC == 0) {
             double d[5][6];
