@@ -8,12 +8,12 @@
 // value and gradient at each particle (getParticleProp,
 // ParticleTrack.cpp:90-97).  Here the same interpolant is built on the device
 // from the resident state:
-//   * k_node_prims: the five primitives (den, u, v, w, p) at the (nc+6)^3
-//     nodes of the padded block -- the ghost nodes as the periodic image --
-//     written into the interior of one coefficient array of (nc+8)^3 nodes
+//   * k_prims_zlines: the five primitives (den, u, v, w, p) at the (nc+6)^3
+//     nodes of the padded block -- the ghost nodes as the periodic image -- go
+//     straight into the z lines of one coefficient array of (nc+8)^3 nodes
 //     with the five fields interleaved per node (node-major, so that the 4 x 4
 //     x 4 block a particle reads is 16 runs of 20 contiguous doubles);
-//   * k_bspline_zlines, k_bspline_lines<AXIS>: the natural cubic B-spline
+//   * k_prims_zlines, k_bspline_lines<AXIS>: the natural cubic B-spline
 //     coefficients, one tridiagonal (1, 4, 1) solve per grid line, along z,
 //     then x, then y (the tensor product).  With c_1 = f_0 and c_N = f_{N-1} fixed by the natural
 //     end conditions, c_2 .. c_{N-1} come from forward elimination with the
@@ -48,81 +48,89 @@ constexpr int kNF = 5;   // fields interleaved per node: den, u, v, w, p
 
 __device__ __forceinline__ int wrap_nc(int x, int n) { return x < 0 ? x + n : (x >= n ? x - n : x); }
 
-// generateSplines' primitives at every node of the padded block
-// (update.cpp:1201-1208): den, u, v, w, p, into the coefficient array at
-// node offset (1, 1, 1).
-__global__ void __launch_bounds__(kLineBlock) k_node_prims(FieldDev f, double *coef)
+// generateSplines' primitives (update.cpp:1201-1208) of one cell.
+__device__ __forceinline__ void cell_prims(const FieldDev &f, double gm1, long long cell, double o[5])
 {
-    const int nc = f.nc;
-    const long long nt = nc + 6, M = nt + 2, N3 = nt * nt * nt;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    const double gm1 = f.gam - 1;
-    for (long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x; c < N3; c += stride) {
-        const int k = int(c % nt);
-        const long long r = c / nt;
-        const int i = int(r % nt), j = int(r / nt);
-        const long long cell = ((long long)wrap_nc(j - 3, nc) * nc + wrap_nc(i - 3, nc)) * nc + wrap_nc(k - 3, nc);
-        const double den = f.W[0][cell];
-        const double u = f.W[1][cell] / den, v = f.W[2][cell] / den, w = f.W[3][cell] / den;
-        const double Vsqr = u * u + v * v + w * w;
-        const double p = (den * gm1) * (f.W[4][cell] / den - 0.5 * Vsqr);
-        double *o = coef + kNF * (((long long)(j + 1) * M + (i + 1)) * M + (k + 1));
-        o[0] = den;
-        o[1] = u;
-        o[2] = v;
-        o[3] = w;
-        o[4] = p;
-    }
+    const double den = f.W[0][cell];
+    const double u = f.W[1][cell] / den, v = f.W[2][cell] / den, w = f.W[3][cell] / den;
+    const double Vsqr = u * u + v * v + w * w;
+    o[0] = den;
+    o[1] = u;
+    o[2] = v;
+    o[3] = w;
+    o[4] = (den * gm1) * (f.W[4][cell] / den - 0.5 * Vsqr);
 }
 
 // Natural cubic B-spline coefficients of one grid line in place:
 // c[m * s], m = 1 .. N, hold the data f_{m-1} on entry (N >= 4).
 // Both recurrences move through the line in groups of kLineGroup positions,
-// every load of a group issued before its first use, so that a thread keeps
-// kLineGroup loads in flight instead of one (the recurrences themselves are
-// sequential).
-constexpr int kLineGroup = 8;
+// the loads of a group issued before the group ahead of it is computed, so
+// that a thread keeps kLineGroup loads in flight over its (sequential)
+// arithmetic.  Bound: HBM -- the array is read and written twice, 2.1 GB of DRAM
+// traffic a pass at 256^3 (part of the second reading comes from L2), 415 us
+// (530 x / 457 y with groups of 8 and no loads ahead).  Measured alternatives:
+// whole lines in shared memory, one reading and one writing, 422 / 436 us (an
+// SM holds 100 such lines, too few for the recurrences); fewer lines at a time,
+// so that the second reading hits L2, 1.75 GB but 459 - 500 us.
+constexpr int kLineGroup = 16;
 
-__device__ __forceinline__ void bspline_line(long long N, double *c, long long s, const double *__restrict__ w)
+__device__ __forceinline__ void bspline_line(int N, double *c, long long s, const double *__restrict__ w)
 {
     const double f0 = c[s], fl = c[N * s];
-    double d = (6.0 * c[2 * s] - f0) * __ldg(w + 2);
-    c[2 * s] = d;
-    // forward elimination over m = 3 .. N-2, then the last row m = N-1
-    long long m = 3;
-    for (; m + kLineGroup <= N - 1; m += kLineGroup) {
-        double v[kLineGroup];
+    double v[kLineGroup], nx[kLineGroup], wm[kLineGroup];
+    // forward elimination over m = 2 .. N-2 (c_1 = f_0 starts it), then the last
+    // row m = N-1; groups of positions m = 2 + kLineGroup i
+    auto fetch = [&](int m) {
 #pragma unroll
-        for (int g = 0; g < kLineGroup; ++g) v[g] = c[(m + g) * s];
+        for (int g = 0; g < kLineGroup; ++g)
+            if (m + g <= N - 1) nx[g] = c[(m + g) * s];
+    };
+    double d = f0;
+    fetch(2);
+    for (int m = 2; m <= N - 1; m += kLineGroup) {
 #pragma unroll
         for (int g = 0; g < kLineGroup; ++g) {
-            d = (6.0 * v[g] - d) * __ldg(w + m + g);
-            c[(m + g) * s] = d;
+            v[g] = nx[g];
+            wm[g] = __ldg(w + min(m + g, N));
+        }
+        fetch(m + kLineGroup);
+        if (m + kLineGroup <= N - 1) {
+#pragma unroll
+            for (int g = 0; g < kLineGroup; ++g) {
+                d = (6.0 * v[g] - d) * wm[g];
+                c[(m + g) * s] = d;
+            }
+        } else {
+#pragma unroll
+            for (int g = 0; g < kLineGroup; ++g)
+                if (m + g <= N - 1) {
+                    d = (m + g == N - 1 ? (6.0 * v[g] - fl) - d : 6.0 * v[g] - d) * wm[g];
+                    c[(m + g) * s] = d;
+                }
         }
     }
-    for (; m < N - 1; ++m) {
-        d = (6.0 * c[m * s] - d) * __ldg(w + m);
-        c[m * s] = d;
-    }
-    d = ((6.0 * c[(N - 1) * s] - fl) - d) * __ldg(w + N - 1);
-    c[(N - 1) * s] = d;
     const double cl = d; // c_{N-1}
     double cn = d;
     // back substitution over m = N-2 .. 2
-    m = N - 2;
-    for (; m - kLineGroup + 1 >= 2; m -= kLineGroup) {
-        double v[kLineGroup];
+    auto back = [&](int m) {
 #pragma unroll
-        for (int g = 0; g < kLineGroup; ++g) v[g] = c[(m - g) * s];
+        for (int g = 0; g < kLineGroup; ++g)
+            if (m - g >= 2) nx[g] = c[(m - g) * s];
+    };
+    back(N - 2);
+    for (int m = N - 2; m >= 2; m -= kLineGroup) {
 #pragma unroll
         for (int g = 0; g < kLineGroup; ++g) {
-            cn = v[g] - __ldg(w + m - g) * cn;
-            c[(m - g) * s] = cn;
+            v[g] = nx[g];
+            wm[g] = __ldg(w + max(m - g, 0));
         }
-    }
-    for (; m >= 2; --m) {
-        cn = c[m * s] - __ldg(w + m) * cn;
-        c[m * s] = cn;
+        back(m - kLineGroup);
+#pragma unroll
+        for (int g = 0; g < kLineGroup; ++g)
+            if (m - g >= 2) {
+                cn = v[g] - wm[g] * cn;
+                c[(m - g) * s] = cn;
+            }
     }
     c[0] = 2.0 * f0 - cn;
     c[(N + 1) * s] = 2.0 * fl - cl;
@@ -144,17 +152,17 @@ __global__ void __launch_bounds__(kLineBlock) k_bspline_lines(double *coef, long
         if (AXIS == 1) {
             // t = ((j - 1) M + k) kNF + q: element m of the line at ((j M + m) M + k) kNF + q
             const long long l = t / kNF, q = t - l * kNF, j = 1 + l / M, k = l % M;
-            bspline_line(N, coef + (j * M * M + k) * kNF + q, M * kNF, w);
+            bspline_line(int(N), coef + (j * M * M + k) * kNF + q, M * kNF, w);
         } else {
             // t = (i M + k) kNF + q: element m at ((m M + i) M + k) kNF + q
-            bspline_line(N, coef + t, M * M * kNF, w);
+            bspline_line(int(N), coef + t, M * M * kNF, w);
         }
     }
 }
 
-// The z pass, whose lines are contiguous: a block takes kZRows grid rows
-// (j, i) with their kNF interleaved fields and moves them through shared
-// memory in tiles of kZChunk positions -- a row's chunk is one contiguous run
+// The primitives and the z pass, whose lines are contiguous: a block takes
+// kZRows grid rows (j, i) with their kNF interleaved fields and moves them
+// through shared memory in tiles of kZChunk positions -- a row's chunk is one contiguous run
 // of kNF kZChunk doubles -- each thread running the recurrences of one row
 // and field: the arithmetic of bspline_line, chunk by chunk, forward
 // elimination over increasing positions, back substitution and the two end
@@ -168,25 +176,32 @@ constexpr int kZRun = kNF * kZChunk;     // doubles of one row's chunk
 constexpr int kZPitch = kZRun + 5;       // 165 = 5 mod 16
 constexpr int kZBatch = 16;              // reads of a thread in flight at once
 
-__global__ void __launch_bounds__(kZThreads) k_bspline_zlines(double *coef, long long N, const double *__restrict__ w)
+__global__ void __launch_bounds__(kZThreads) k_prims_zlines(FieldDev f, double *coef, long long N,
+                                                            const double *__restrict__ w)
 {
     __shared__ double tile[kZRows][kZPitch];
     __shared__ double *rbase[kZRows];
+    __shared__ long long cbase[kZRows]; // the row's first cell
     const long long M = N + 2, R = N * N;
+    const int nc = f.nc, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const double gm1 = f.gam - 1;
     const int t = threadIdx.x, r = t / kNF, q = t - r * kNF;
     const long long nchunk = (M + kZChunk - 1) / kZChunk;
     for (long long r0 = (long long)blockIdx.x * kZRows; r0 < R; r0 += (long long)gridDim.x * kZRows) {
         if (t < kZRows) {
             const long long rr = r0 + t; // row (1 + rr / N, 1 + rr % N)
             rbase[t] = rr < R ? coef + ((1 + rr / N) * M + (1 + rr % N)) * M * kNF : nullptr;
+            cbase[t] = ((long long)wrap_nc(int(rr / N) - 3, nc) * nc + wrap_nc(int(rr % N) - 3, nc)) * nc;
         }
         __syncthreads();
         const bool mine = rbase[r] != nullptr;
-        const double *line = mine ? rbase[r] + q : nullptr; // element m at line[m * kNF]
         double f0 = 0.0, fl = 0.0, d = 0.0;
-        if (mine) {
-            f0 = line[kNF];
-            fl = line[N * kNF];
+        if (mine) { // the first and last node: the images of cells nc - 3 and 2
+            double o[5];
+            cell_prims(f, gm1, cbase[r] + nc - 3, o);
+            f0 = q == 0 ? o[0] : q == 1 ? o[1] : q == 2 ? o[2] : q == 3 ? o[3] : o[4];
+            cell_prims(f, gm1, cbase[r] + 2, o);
+            fl = q == 0 ? o[0] : q == 1 ? o[1] : q == 2 ? o[2] : q == 3 ? o[3] : o[4];
         }
         // tile <-> global: each row's chunk [p0, p0 + kZChunk) x fields is one run
         auto move = [&](long long p0, bool load) {
@@ -218,7 +233,18 @@ __global__ void __launch_bounds__(kZThreads) k_bspline_zlines(double *coef, long
         };
         for (long long c = 0; c < nchunk; ++c) {
             const long long p0 = c * kZChunk;
-            move(p0, true);
+            // the primitives of the chunk's nodes, position m holding node m - 1 = cell m - 4
+            {
+                const int m = int(p0) + lane, k = wrap_nc(m - 4, nc);
+                const bool node = m >= 1 && m <= N;
+#pragma unroll 4
+                for (int rw = wid; rw < kZRows; rw += kZThreads / 32) {
+                    double o[5] = {0.0, 0.0, 0.0, 0.0, 0.0};
+                    if (node && rbase[rw]) cell_prims(f, gm1, cbase[rw] + k, o);
+#pragma unroll
+                    for (int a = 0; a < kNF; ++a) tile[rw][lane * kNF + a] = o[a];
+                }
+            }
             __syncthreads();
             if (mine) {
 #pragma unroll
@@ -267,87 +293,95 @@ __global__ void __launch_bounds__(kZThreads) k_bspline_zlines(double *coef, long
 
 // Cell and cubic B-spline weights of position x along one axis of num nodes;
 // the cell is clamped to the last interval (as the oracle's).
-__device__ __forceinline__ int bspline_weights(double x, double start, double hinv, int num, double b[4],
-                                               double db[4])
+__device__ __forceinline__ int bspline_cell(double x, double start, double hinv, int num, double *t)
 {
     const double u = (x - start) * hinv;
     double fl = floor(u);
     fl = fmin(fmax(fl, 0.0), double(num - 2)); // NaN -> 0: stays inside the arrays
-    const int i = int(fl);
-    const double t = u - fl;
+    *t = u - fl;
+    return int(fl);
+}
+
+__device__ __forceinline__ void bspline_weights(double t, double b[8])
+{
     const double s = 1.0 - t, t2 = t * t, t3 = t2 * t;
     b[0] = (s * s * s) / 6.0;
     b[1] = (3.0 * t3 - 6.0 * t2 + 4.0) / 6.0;
     b[2] = (-3.0 * t3 + 3.0 * t2 + 3.0 * t + 1.0) / 6.0;
     b[3] = t3 / 6.0;
-    db[0] = -0.5 * (s * s);
-    db[1] = 1.5 * t2 - 2.0 * t;
-    db[2] = (-1.5 * t2 + t) + 0.5;
-    db[3] = 0.5 * t2;
-    return i;
+    b[4] = -0.5 * (s * s);
+    b[5] = 1.5 * t2 - 2.0 * t;
+    b[6] = (-1.5 * t2 + t) + 0.5;
+    b[7] = 0.5 * t2;
 }
 
 // getParticleProp (ParticleTrack.cpp:90-97) of every particle: value and
-// gradient of the five splines at its position.  A row of the 4 x 4 x 4
-// coefficient block -- four nodes along z with their five fields -- is one
-// contiguous run of 20 doubles, read once for all fields; each field's sums
+// gradient of the five splines at its position.  A warp takes six particles,
+// lane l the field l % 5 of particle l / 5: the five lanes of a particle read
+// its 4 x 4 x 4 block as 16 contiguous runs of 20 doubles, and a thread holds
+// seven sums instead of the 35 of a particle.  Lanes 0-2 of a particle form the
+// weights of one axis each and hand them over through shared memory.  The sums
 // keep the order of a field-by-field evaluation (rows along y, then x, nodes
-// along z innermost).  Measured alternatives: the five fields in separate
-// arrays read 8.4 GB of DRAM per 2^20 particles at 256^3 (1.43 ms) against
-// 4.1 GB here (1.65 ms, latency-bound at 8 warps per SM: the 35 sums and the
-// row take 254 registers; capped at 168 they spill and take 1.74 ms); field
-// by field over the interleaved rows, each field's pass fetching the rows
-// again, 17 GB and 5.7 ms (L2 does not hold a resident wave's rows between
-// passes).
-__global__ void __launch_bounds__(kPrtBlock) k_particle_props(const double *__restrict__ coef, int nt, double start,
-                                                              double hinv, double *rec, long long n)
+// along z innermost).  Bound: latency of random reads, 16 rows of 160 B a
+// particle (4.3 GB of DRAM traffic for 2^20 particles at 256^3).  Measured there:
+// a thread per particle (254 registers, 8 warps per SM) 1.65 ms, this form
+// 0.69 ms; visiting the particles tile by tile of the grid 0.88 ms and a sort
+// (their records are then scattered).
+constexpr int kPropWarps = 4, kPropParticles = 6;
+
+__global__ void __launch_bounds__(32 * kPropWarps) k_particle_props(const double *__restrict__ coef, int nt, double start,
+                                                                    double hinv, double *rec, long long n)
 {
+    __shared__ double weights[kPropWarps][kPropParticles][3][8];
+    __shared__ int cells[kPropWarps][kPropParticles][3];
     const long long M = nt + 2;
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long a = (long long)blockIdx.x * blockDim.x + threadIdx.x; a < n; a += stride) {
-        double by[4], dby[4], bx[4], dbx[4], bz[4], dbz[4];
-        const int iy = bspline_weights(rec[a], start, hinv, nt, by, dby);
-        const int ix = bspline_weights(rec[n + a], start, hinv, nt, bx, dbx);
-        const int iz = bspline_weights(rec[2 * n + a], start, hinv, nt, bz, dbz);
-        double v[kNF], gy[kNF], gx[kNF], gz[kNF];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int p = lane / kNF, q = lane - p * kNF;
+    const long long groups = (n + kPropParticles - 1) / kPropParticles;
+    for (long long g = (long long)blockIdx.x * kPropWarps + wid; g < groups; g += (long long)gridDim.x * kPropWarps) {
+        const long long idx = g * kPropParticles + p;
+        const bool mine = lane < kNF * kPropParticles && idx < n;
+        const long long a = mine ? idx : 0;
+        if (mine && q < 3) {
+            double t;
+            cells[wid][p][q] = bspline_cell(rec[q * n + a], start, hinv, nt, &t);
+            bspline_weights(t, weights[wid][p][q]);
+        }
+        __syncwarp();
+        if (mine) {
+            const double (*b)[8] = weights[wid][p];
+            const int *ic = cells[wid][p];
+            const double *c0 = coef + (((long long)ic[0] * M + ic[1]) * M + ic[2]) * kNF + q;
+            double bz[8];
 #pragma unroll
-        for (int q = 0; q < kNF; ++q) v[q] = gy[q] = gx[q] = gz[q] = 0.0;
+            for (int c = 0; c < 8; ++c) bz[c] = b[2][c];
+            double v = 0.0, gy = 0.0, gx = 0.0, gz = 0.0;
 #pragma unroll
-        for (int ia = 0; ia < 4; ++ia) {
-            double va[kNF], gxa[kNF], gza[kNF];
+            for (int ia = 0; ia < 4; ++ia) {
+                double va = 0.0, gxa = 0.0, gza = 0.0;
 #pragma unroll
-            for (int q = 0; q < kNF; ++q) va[q] = gxa[q] = gza[q] = 0.0;
-#pragma unroll
-            for (int ib = 0; ib < 4; ++ib) {
-                const double *r = coef + (((long long)(iy + ia) * M + (ix + ib)) * M + iz) * kNF;
-                double x[4 * kNF];
-#pragma unroll
-                for (int c = 0; c < 4 * kNF; ++c) x[c] = __ldg(r + c);
-#pragma unroll
-                for (int q = 0; q < kNF; ++q) {
-                    const double r0 = x[q], r1 = x[kNF + q], r2 = x[2 * kNF + q], r3 = x[3 * kNF + q];
+                for (int ib = 0; ib < 4; ++ib) {
+                    const double *r = c0 + (ia * M + ib) * M * kNF;
+                    const double r0 = __ldg(r), r1 = __ldg(r + kNF), r2 = __ldg(r + 2 * kNF), r3 = __ldg(r + 3 * kNF);
                     const double sv = ((bz[0] * r0 + bz[1] * r1) + bz[2] * r2) + bz[3] * r3;
-                    const double sd = ((dbz[0] * r0 + dbz[1] * r1) + dbz[2] * r2) + dbz[3] * r3;
-                    va[q] += bx[ib] * sv;
-                    gxa[q] += dbx[ib] * sv;
-                    gza[q] += bx[ib] * sd;
+                    const double sd = ((bz[4] * r0 + bz[5] * r1) + bz[6] * r2) + bz[7] * r3;
+                    const double bx = b[1][ib], dbx = b[1][4 + ib];
+                    va += bx * sv;
+                    gxa += dbx * sv;
+                    gza += bx * sd;
                 }
+                const double by = b[0][ia], dby = b[0][4 + ia];
+                v += by * va;
+                gy += dby * va;
+                gx += by * gxa;
+                gz += by * gza;
             }
-#pragma unroll
-            for (int q = 0; q < kNF; ++q) {
-                v[q] += by[ia] * va[q];
-                gy[q] += dby[ia] * va[q];
-                gx[q] += by[ia] * gxa[q];
-                gz[q] += by[ia] * gza[q];
-            }
+            rec[(3 + q) * n + a] = v;
+            rec[(8 + 3 * q) * n + a] = gy * hinv;
+            rec[(9 + 3 * q) * n + a] = gx * hinv;
+            rec[(10 + 3 * q) * n + a] = gz * hinv;
         }
-#pragma unroll
-        for (int q = 0; q < kNF; ++q) {
-            rec[(3 + q) * n + a] = v[q];
-            rec[(8 + 3 * q) * n + a] = gy[q] * hinv;
-            rec[(9 + 3 * q) * n + a] = gx[q] * hinv;
-            rec[(10 + 3 * q) * n + a] = gz[q] * hinv;
-        }
+        __syncwarp();
     }
 }
 
@@ -436,8 +470,9 @@ int particle_partial_elems(int nsm) { return nsm * 4 * kNSum; }
 cudaError_t launch_particle_splines(const FieldDev &f, double *coef, const double *w, int nsm, cudaStream_t st)
 {
     const long long nt = f.nc + 6, M = nt + 2;
-    k_node_prims<<<grid_for(nt * nt * nt, kLineBlock, nsm, 16), kLineBlock, 0, st>>>(f, coef);
-    k_bspline_zlines<<<grid_for(kNF * nt * nt, kZThreads, nsm, 4), kZThreads, 0, st>>>(coef, nt, w);
+    // 5 blocks of the z pass fit an SM's shared memory; at 256^3 its rows then make
+    // three even rounds (980 us; 4 blocks: 1140)
+    k_prims_zlines<<<grid_for(kNF * nt * nt, kZThreads, nsm, 5), kZThreads, 0, st>>>(f, coef, nt, w);
     k_bspline_lines<1><<<grid_for(kNF * nt * M, kLineBlock, nsm, 16), kLineBlock, 0, st>>>(coef, nt, w);
     k_bspline_lines<0><<<grid_for(kNF * M * M, kLineBlock, nsm, 16), kLineBlock, 0, st>>>(coef, nt, w);
     return cudaGetLastError();
@@ -446,7 +481,9 @@ cudaError_t launch_particle_splines(const FieldDev &f, double *coef, const doubl
 cudaError_t launch_particle_props(const FieldDev &f, const double *coef, double start, double hinv, double *rec,
                                   long long n, int nsm, cudaStream_t st)
 {
-    k_particle_props<<<grid_for(n, kPrtBlock, nsm, 16), kPrtBlock, 0, st>>>(coef, f.nc + 6, start, hinv, rec, n);
+    const long long groups = (n + kPropParticles - 1) / kPropParticles;
+    k_particle_props<<<grid_for(32 * groups, 32 * kPropWarps, nsm, 16), 32 * kPropWarps, 0, st>>>(coef, f.nc + 6, start, hinv,
+                                                                                             rec, n);
     return cudaGetLastError();
 }
 

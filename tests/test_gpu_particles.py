@@ -232,3 +232,17 @@ def test_driver_tracks_particles_like_the_oracle(tmp_path, oracle):
         if s < steps:
             oracle.particle_track(rec, dt)
             oracle.step(W, prm, dt, 1)
+
+
+@pytest.mark.parametrize("nc,n", [(4, 1), (5, 5), (9, 6), (10, 7), (25, 12), (26, 13), (27, 193), (59, 1000)])
+def test_particles_at_group_edges(gks, oracle, nc, n):
+    """Lines whose nodes are a few more or fewer than the groups of positions the
+    recurrences move in and than the z tiles' chunks, and particle numbers around
+    the six a warp takes: records bit for bit."""
+    case, W, x0, y0, z0 = setup(nc, 3 + nc, n)
+    prm, want = oracle_records(oracle, case, W, x0, y0, z0)
+    with gks.Solver(gks.phys_from_case(case)) as s:
+        s.upload(W)
+        s.particles_locate(x0, y0, z0)
+        s.particles_props()
+        assert np.array_equal(s.particles_get(), want)
