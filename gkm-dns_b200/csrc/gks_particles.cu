@@ -8,17 +8,19 @@
 // value and gradient at each particle (getParticleProp,
 // ParticleTrack.cpp:90-97).  Here the same interpolant is built on the device
 // from the resident state:
-//   * k_prims_zlines: the five primitives (den, u, v, w, p) at the (nc+6)^3
-//     nodes of the padded block -- the ghost nodes as the periodic image -- go
-//     straight into the z lines of one coefficient array of (nc+8)^3 nodes
-//     with the five fields interleaved per node (node-major, so that the 4 x 4
-//     x 4 block a particle reads is 16 runs of 20 contiguous doubles);
-//   * k_prims_zlines, k_bspline_lines<AXIS>: the natural cubic B-spline
-//     coefficients, one tridiagonal (1, 4, 1) solve per grid line, along z,
-//     then x, then y (the tensor product).  With c_1 = f_0 and c_N = f_{N-1} fixed by the natural
-//     end conditions, c_2 .. c_{N-1} come from forward elimination with the
-//     host-computed pivots w_2 = 1/4, w_m = 1/(4 - w_{m-1}) and back
-//     substitution, then c_0 = 2 c_1 - c_2 and c_{N+1} = 2 c_N - c_{N-1};
+//   * the five primitives (den, u, v, w, p) at the (nc+6)^3 nodes of the padded
+//     block -- the ghost nodes as the periodic image -- go straight into the z
+//     lines of one coefficient array of (nc+8)^3 nodes with the five fields
+//     interleaved per node (node-major, so that the 4 x 4 x 4 block a particle
+//     reads is 16 runs of 20 contiguous doubles);
+//   * the natural cubic B-spline coefficients, one tridiagonal (1, 4, 1) solve
+//     per grid line, along z, then x, then y (the tensor product).  With c_1 =
+//     f_0 and c_N = f_{N-1} fixed by the natural end conditions, c_2 .. c_{N-1}
+//     come from forward elimination with the host-computed pivots w_2 = 1/4,
+//     w_m = 1/(4 - w_{m-1}) and back substitution, then c_0 = 2 c_1 - c_2 and
+//     c_{N+1} = 2 c_N - c_{N-1}: k_prims_rows (primitives and z lines) and
+//     k_line_cols<AXIS> (x, y lines) up to kLineShort nodes, k_prims_zlines and
+//     k_bspline_lines<AXIS> beyond;
 //   * k_particle_props: per particle the cell and cubic B-spline weights
 //     along each axis, then value and gradient of the five splines from
 //     their 4 x 4 x 4 coefficient blocks.
@@ -291,6 +293,166 @@ __global__ void __launch_bounds__(kZThreads) k_prims_zlines(FieldDev f, double *
     }
 }
 
+// Asynchronous 8-byte copy global -> shared, its groups and waits.
+__device__ __forceinline__ void cp_async8(double *smem, const double *gmem)
+{
+    const unsigned a = unsigned(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\
+" ::"r"(a), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\
+" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;\
+" ::"n"(N) : "memory");
+}
+
+// ---------------------------------------------------------------------------
+// Short lines stay in shared memory between their two recurrences, so that a
+// pass reads and writes the array once, and an SM holds enough of them (100 of
+// 262 nodes, 400 of 64) for the serial recurrences not to be the bound.
+// gks_particles_props with few particles, us, this form / the two-pass kernels:
+// 16^3 30 / 42, 32^3 35 / 61, 64^3 45 / 86, 96^3 102 / 131, 128^3 254 / 277, 160^3
+// 479 / 571, 200^3 1069 / 893.
+// ---------------------------------------------------------------------------
+constexpr int kLineShort = 176; // nodes
+
+// x (AXIS 1) and y (AXIS 0) lines: a block is one warp, a thread one line and
+// field, consecutive threads on consecutive (k, field), so that a row of the
+// warp is 256 contiguous bytes.  The forward elimination follows the rows as
+// they arrive, kColAhead groups of kColRows rows in flight; the back
+// substitution writes its results straight to global memory.
+constexpr int kColRows = 16, kColAhead = 5;
+
+template <int AXIS>
+__global__ void __launch_bounds__(32) k_line_cols(double *coef, int N, const double *__restrict__ w)
+{
+    extern __shared__ double tile[]; // row m at 32 (m - 1), m = 1 .. N
+    const int lane = threadIdx.x;
+    const long long M = N + 2, P = kNF * M;
+    const long long L = (AXIS == 1 ? N : M) * P;
+    const long long l0 = (long long)blockIdx.x * 32 + lane;
+    const bool mine = l0 < L;
+    const long long l = mine ? l0 : L - 1;
+    // x: line (j, k, field), its elements P apart; y: line (i, k, field), M P apart
+    double *c = AXIS == 1 ? coef + (1 + l / P) * (M * P) + l % P : coef + l;
+    const long long s = AXIS == 1 ? P : M * P;
+    double *col = tile + lane - 32; // element m at col[32 m]
+    auto fetch = [&](int g) {
+        const int m0 = 1 + g * kColRows;
+#pragma unroll
+        for (int r = 0; r < kColRows; ++r)
+            if (m0 + r <= N) cp_async8(col + 32 * (m0 + r), c + (m0 + r) * s);
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int g = 0; g < kColAhead; ++g) fetch(g);
+    const double f0 = c[s], fl = c[N * s];
+    double d = f0; // d_2 = (6 f_1 - f_0) w_2 is the general step with d_1 = f_0
+    const int ng = (N + kColRows - 1) / kColRows;
+    for (int g = 0; g < ng; ++g) {
+        fetch(g + kColAhead);
+        cp_async_wait<kColAhead>();
+        const int m0 = 1 + g * kColRows;
+        if (g > 0 && m0 + kColRows <= N - 1) {
+#pragma unroll
+            for (int r = 0; r < kColRows; ++r) {
+                d = (6.0 * col[32 * (m0 + r)] - d) * __ldg(w + m0 + r);
+                col[32 * (m0 + r)] = d;
+            }
+        } else {
+            for (int m = max(m0, 2); m < min(m0 + kColRows, N); ++m) {
+                d = m < N - 1 ? (6.0 * col[32 * m] - d) * __ldg(w + m) : ((6.0 * col[32 * m] - fl) - d) * __ldg(w + m);
+                col[32 * m] = d;
+            }
+        }
+    }
+    if (!mine) return;
+    const double cl = d; // c_{N-1}
+    double cn = d;
+    c[(N - 1) * s] = cl;
+    c[(N + 1) * s] = 2.0 * fl - cl;
+    int m = N - 2;
+    for (; m - kColRows + 1 >= 2; m -= kColRows) {
+#pragma unroll
+        for (int r = 0; r < kColRows; ++r) {
+            cn = col[32 * (m - r)] - __ldg(w + m - r) * cn;
+            c[(m - r) * s] = cn;
+        }
+    }
+    for (; m >= 2; --m) {
+        cn = col[32 * m] - __ldg(w + m) * cn;
+        c[m * s] = cn;
+    }
+    c[0] = 2.0 * f0 - cn;
+}
+
+// The recurrences of bspline_line on a line in shared memory.
+__device__ __forceinline__ void bspline_smem(int N, double *c, const double *__restrict__ w)
+{
+    const double f0 = c[kNF], fl = c[N * kNF];
+    double d = f0;
+#pragma unroll 8
+    for (int m = 2; m < N - 1; ++m) {
+        d = (6.0 * c[m * kNF] - d) * __ldg(w + m);
+        c[m * kNF] = d;
+    }
+    d = ((6.0 * c[(N - 1) * kNF] - fl) - d) * __ldg(w + N - 1);
+    c[(N - 1) * kNF] = d;
+    double cn = d;
+#pragma unroll 8
+    for (int m = N - 2; m >= 2; --m) {
+        cn = c[m * kNF] - __ldg(w + m) * cn;
+        c[m * kNF] = cn;
+    }
+    c[0] = 2.0 * f0 - cn;
+    c[(N + 1) * kNF] = 2.0 * fl - d;
+}
+
+// The primitives and the z lines: a block takes kRowRows grid rows (j, i).
+// Its warps read the rows' cells and write the nodes' primitives to the rows'
+// tiles (five fields interleaved per node, row pitch 5 mod 16 doubles, so that
+// thread t at row t / 5 and field t % 5 reads without bank conflicts), 30
+// threads run the recurrences, and the rows leave as contiguous runs.
+constexpr int kRowRows = 6, kRowThreads = 128;
+__host__ __device__ inline int row_pitch(int M) { return (kNF * M - kNF + 15) / 16 * 16 + kNF; }
+
+__global__ void __launch_bounds__(kRowThreads) k_prims_rows(FieldDev f, double *coef, const double *__restrict__ w)
+{
+    extern __shared__ double rows[];
+    const int nc = f.nc, N = nc + 6, M = N + 2, pitch = row_pitch(M);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const long long r0 = (long long)blockIdx.x * kRowRows, R = (long long)N * N;
+    const double gm1 = f.gam - 1;
+    for (int r = wid; r < kRowRows && r0 + r < R; r += kRowThreads / 32) {
+        const int j = int((r0 + r) / N), i = int((r0 + r) % N);
+        const long long base = ((long long)wrap_nc(j - 3, nc) * nc + wrap_nc(i - 3, nc)) * nc;
+        double *row = rows + r * pitch;
+#pragma unroll 2
+        for (int k = lane; k < nc; k += 32) {
+            double o[5];
+            cell_prims(f, gm1, base + k, o);
+#pragma unroll
+            for (int q = 0; q < kNF; ++q) row[kNF * (k + 4) + q] = o[q]; // node of cell k: m = k + 4
+        }
+        __syncwarp();
+        // ghost nodes m = 1 .. 3 (cells nc-3 .. nc-1) and nc + 4 .. nc + 6 (cells 0 .. 2)
+        if (lane < 3 * kNF) {
+            row[kNF + lane] = row[kNF * (nc + 1) + lane];
+            row[kNF * (nc + 4) + lane] = row[kNF * 4 + lane];
+        }
+    }
+    __syncthreads();
+    if (threadIdx.x < kNF * kRowRows && r0 + threadIdx.x / kNF < R)
+        bspline_smem(N, rows + (threadIdx.x / kNF) * pitch + threadIdx.x % kNF, w);
+    __syncthreads();
+    for (int r = 0; r < kRowRows && r0 + r < R; ++r) {
+        double *o = coef + ((1 + (r0 + r) / N) * M + (1 + (r0 + r) % N)) * (long long)(kNF * M);
+        for (int e = threadIdx.x; e < kNF * M; e += kRowThreads) o[e] = rows[r * pitch + e];
+    }
+}
+
 // Cell and cubic B-spline weights of position x along one axis of num nodes;
 // the cell is clamped to the last interval (as the oracle's).
 __device__ __forceinline__ int bspline_cell(double x, double start, double hinv, int num, double *t)
@@ -470,6 +632,17 @@ int particle_partial_elems(int nsm) { return nsm * 4 * kNSum; }
 cudaError_t launch_particle_splines(const FieldDev &f, double *coef, const double *w, int nsm, cudaStream_t st)
 {
     const long long nt = f.nc + 6, M = nt + 2;
+    if (nt <= kLineShort) {
+        const size_t rows = (size_t)kRowRows * row_pitch((int)M) * sizeof(double), cols = (size_t)nt * 32 * sizeof(double);
+        cudaError_t e = cudaFuncSetAttribute(k_prims_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line_cols<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols);
+        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line_cols<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols);
+        if (e != cudaSuccess) return e;
+        k_prims_rows<<<(unsigned)((nt * nt + kRowRows - 1) / kRowRows), kRowThreads, rows, st>>>(f, coef, w);
+        k_line_cols<1><<<(unsigned)((kNF * nt * M + 31) / 32), 32, cols, st>>>(coef, (int)nt, w);
+        k_line_cols<0><<<(unsigned)((kNF * M * M + 31) / 32), 32, cols, st>>>(coef, (int)nt, w);
+        return cudaGetLastError();
+    }
     // 5 blocks of the z pass fit an SM's shared memory; at 256^3 its rows then make
     // three even rounds (980 us; 4 blocks: 1140)
     k_prims_zlines<<<grid_for(kNF * nt * nt, kZThreads, nsm, 5), kZThreads, 0, st>>>(f, coef, nt, w);

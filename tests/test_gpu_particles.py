@@ -234,11 +234,12 @@ def test_driver_tracks_particles_like_the_oracle(tmp_path, oracle):
             oracle.step(W, prm, dt, 1)
 
 
-@pytest.mark.parametrize("nc,n", [(4, 1), (5, 5), (9, 6), (10, 7), (25, 12), (26, 13), (27, 193), (59, 1000)])
+@pytest.mark.parametrize("nc,n", [(4, 1), (5, 5), (9, 6), (10, 7), (25, 12), (26, 13), (27, 193), (59, 1000), (170, 50), (171, 50)])
 def test_particles_at_group_edges(gks, oracle, nc, n):
     """Lines whose nodes are a few more or fewer than the groups of positions the
     recurrences move in and than the z tiles' chunks, and particle numbers around
-    the six a warp takes: records bit for bit."""
+    the six a warp takes, and the last and first field of the short and the long
+    lines' kernels (176 nodes): records bit for bit."""
     case, W, x0, y0, z0 = setup(nc, 3 + nc, n)
     prm, want = oracle_records(oracle, case, W, x0, y0, z0)
     with gks.Solver(gks.phys_from_case(case)) as s:
