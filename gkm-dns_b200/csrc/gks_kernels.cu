@@ -16,6 +16,7 @@
 
 #include <cuda_runtime.h>
 #include <algorithm>
+#include <climits>
 #include <type_traits>
 
 namespace gks {
@@ -942,8 +943,8 @@ __global__ void k_maxwave(FieldDev f, unsigned long long *out)
 // node slopes of the natural cubic spline through each padded grid line
 // (nt = nc + 6 points, periodic ghosts), the interpolant the reference builds
 // with einspline (Interpolation.cpp:3-31); at nodes a tensor-product natural
-// spline reduces to these 1-D slopes.  Scratch layout: [3 + 3*comp + axis]
-// d(comp)/d(axis), axis 0 = y, 1 = x, 2 = z (slots 0-2 unused).
+// spline reduces to these 1-D slopes.  Scratch layout: [3*comp + axis]
+// d(comp)/d(axis), axis 0 = y, 1 = x (those along z are not stored).
 // ---------------------------------------------------------------------------
 
 // Slopes of the natural cubic spline through the nt = nc + 6 nodes of a
@@ -952,224 +953,77 @@ __global__ void k_maxwave(FieldDev f, unsigned long long *out)
 //   2 m0 + m1 = s (f1 - f0);  m_{p-1} + 4 m_p + m_{p+1} = s (f_{p+1} - f_{p-1});
 //   m_{n-2} + 2 m_{n-1} = s (f_{n-1} - f_{n-2}),  s = 3/h,
 // solved by the Thomas recurrences with precomputed pivots,
-//   forward  d_p = (r_p - d_{p-1}) inv_p,   backward  m_p = d_p - cp_p m_{p+1},
-// each step an affine map of the previous value.  One warp solves one line:
-// lane L owns the B consecutive nodes [L B, L B + B) (B odd, 32 B >= nt),
-// composes the affine maps of its nodes, an inclusive warp scan of the
-// composed maps (five shuffle steps) hands every lane the value entering its
-// nodes, and the lane runs its nodes again from there -- forward, then the
-// same backward.  The associativity of the scan changes only the rounding.
-//
-// A block takes LW lines: it copies rho, rho u, rho v, rho w of all their
-// nodes into shared memory with asynchronous copies (all in flight at once,
-// no registers), turns the momenta into velocities in place, each warp solves
-// its line for the components (NCI of them interleaved, for latency), and the
-// slopes leave through the same tiles:
+//   forward  d_p = (r_p - d_{p-1}) inv_p,   backward  m_p = d_p - cp_p m_{p+1}.
+// A block takes LW lines at a time: its threads load rho and the momenta of
+// their nodes and stage the velocities in shared memory, one thread per line
+// and component runs the recurrences in place (24 cycles of dependent FP64 a
+// node), and the slopes leave through the same tiles:
 //   y, x lines: LW consecutive k of one (i) / (j): tiles [node][line], every
 //               group of LW threads one contiguous run of LW doubles;
-//   z lines:    LW consecutive (j, i) lines:      tiles [line][node], each
-//               line one contiguous run of nc doubles.
-// Odd B keeps the solve's shared-memory accesses free of bank conflicts.
-template <int AXIS, int B, int LW> struct SplineTiles {
-    static constexpr int NCI = B <= 9 ? 3 : 1; // components solved together
-    __host__ __device__ static int tile(int nt) { return AXIS == 2 ? LW * nt : nt * (LW + 1); }
-    __host__ __device__ static size_t bytes(int nt) { return (4 * (size_t)tile(nt) + 2 * (size_t)nt) * sizeof(double); }
+//   z lines:    LW consecutive (j, i) lines:      tiles [line][node], the
+//               pitch odd so that the lines' threads use distinct banks.
+// Two blocks fit an SM at 256^3, so that one's lines are solved while the
+// other's are moved.
+template <int AXIS, int LW> struct SplineTiles {
+    __host__ __device__ static int tile(int nt) { return AXIS == 2 ? LW * (nt | 1) : nt * LW; }
+    __host__ __device__ static size_t bytes(int nt) { return (3 * (size_t)tile(nt) + 2 * (size_t)nt) * sizeof(double); }
 };
+constexpr int kSplineBlock = 256, kStage = 4; // threads; nodes a thread loads at a time
 
-template <int AXIS, int B, int LW>
-__global__ void __launch_bounds__(32 * LW, B <= 9 ? 2 : 1) k_spline_scan(FieldDev f, double *scr)
+// The line f_p at c[p S], p = 0 .. nt-1, replaced by its slopes.  Nodes move in
+// groups whose data and pivots are loaded before the group's stores, which the
+// compiler could not move loads across.
+constexpr int kSplineGroup = 8;
+template <int S> __device__ __forceinline__ void spline_slopes(double *c, int nt, double s, const double *inv, const double *cp)
 {
-    using ST = SplineTiles<AXIS, B, LW>;
-    constexpr int NCI = ST::NCI;
-    extern __shared__ double smem[];
-    // nodes of a line: nc + 6 along x / z; along y ny + 2 yhost (the same for a
-    // periodic field; a slab's ny stored planes, its ghosts included)
-    const int nc = f.nc, nt = AXIS == 0 ? f.ny + 2 * f.yhost : nc + 6;
-    const long long n = f.ncell;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const int tsz = ST::tile(nt);
-    double *cpv = smem + 4 * tsz, *invv = cpv + nt;
-    // tile a (0 rho, 1-3 the velocity components), node, line
-    auto T = [&](int a, int node, int line) -> double & {
-        return AXIS == 2 ? smem[a * tsz + line * nt + node] : smem[a * tsz + node * (LW + 1) + line];
-    };
-    for (int p = threadIdx.x; p < nt; p += blockDim.x) {
-        cpv[p] = AXIS == 0 ? f.spl_cpy[p] : f.spl_cp[p];
-        invv[p] = AXIS == 0 ? f.spl_invy[p] : f.spl_inv[p];
+    constexpr int G = kSplineGroup;
+    double prev = c[0], cur = c[S];
+    double d = (s * (cur - prev)) * inv[0];
+    c[0] = d;
+    int p = 1;
+    for (; p + G <= nt - 1; p += G) {
+        double f[G], iv[G];
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            f[g] = c[(p + 1 + g) * S];
+            iv[g] = inv[p + g];
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+            const double next = f[g];
+            f[g] = d = fma(s, next - prev, -d) * iv[g];
+            prev = cur;
+            cur = next;
+        }
+#pragma unroll
+        for (int g = 0; g < G; ++g) c[(p + g) * S] = f[g];
     }
-    // the block's lines: y / x lines are (outer, k) with k in [k0, k0 + LW),
-    // outer = i (y lines) or j (x lines, interior planes); z lines are l in
-    // [l0, l0 + LW), l = j nc + i (interior planes)
-    const int nkb = (nc + LW - 1) / LW;
-    const long long set = blockIdx.x;
-    const int outer = AXIS == 2 ? 0 : (AXIS == 1 ? f.ylo : 0) + int(set / nkb);
-    const int k0 = AXIS == 2 ? 0 : int(set - (long long)(outer - (AXIS == 1 ? f.ylo : 0)) * nkb) * LW;
-    const long long l0 = AXIS == 2 ? (long long)f.ylo * nc + set * LW : 0;
-    // cell of line `line` at position q (0 .. nc-1) along the axis
-    auto cell = [&](int line, int q) -> long long {
-        if (AXIS == 0) return ((long long)q * nc + outer) * nc + k0 + line;
-        if (AXIS == 1) return ((long long)outer * nc + q) * nc + k0 + line;
-        return (l0 + line) * nc + q;
-    };
-    auto active = [&](int line) -> bool {
-        return AXIS == 2 ? l0 + line < (long long)f.yhi * nc : k0 + line < nc;
-    };
-    // visit every (node, line) of the set: y / x, LW consecutive threads on
-    // the LW lines of one node; z, warp w along the nodes of line w
-    auto each = [&](auto fn) {
-        if (AXIS == 2) {
-            if (active(w))
-                for (int p = lane; p < nt; p += 32) fn(p, w);
-        } else {
-            for (int e = threadIdx.x; e < nt * LW; e += 32 * LW) {
-                const int line = e % LW;
-                if (active(line)) fn(e / LW, line);
-            }
-        }
-    };
-    // stage rho and the momenta (node p holds cell wrap(p - 3); along y plane
-    // wrap(p - yhost, nyw), a slab's plane p), then velocities
-    each([&](int p, int line) {
-        const long long c = cell(line, AXIS == 0 ? wrap(p - f.yhost, f.nyw) : wrap(p - 3, nc));
-#pragma unroll
-        for (int a = 0; a < 4; ++a) cp_async8(&T(a, p, line), f.W[a] + c);
-    });
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-    each([&](int p, int line) {
-        const double ri = __drcp_rn(T(0, p, line));
-#pragma unroll
-        for (int a = 1; a < 4; ++a) T(a, p, line) *= ri;
-    });
-    __syncthreads();
-    if (active(w)) {
-        const double s = AXIS == 0 ? f.spl_sy : f.spl_s;
-        const int p0 = lane * B;
-#pragma unroll 1
-        for (int c0 = 0; c0 < 3; c0 += NCI) {
-            // right-hand sides and the composed forward maps d -> A d + C of the lane's nodes
-            double r[NCI][B], A[NCI], C[NCI];
-#pragma unroll
-            for (int q = 0; q < NCI; ++q) {
-                A[q] = 1.0;
-                C[q] = 0.0;
-            }
-#pragma unroll
-            for (int j = 0; j < B; ++j) {
-                const int p = p0 + j;
-                if (p < nt) {
-                    const double iv = invv[p];
-                    // rows 0 and nt-1 are the one-sided natural-end rows
-                    const int pa = p == 0 ? 0 : p - 1, pb = p == nt - 1 ? p : p + 1;
-#pragma unroll
-                    for (int q = 0; q < NCI; ++q) {
-                        r[q][j] = s * (T(1 + c0 + q, pb, w) - T(1 + c0 + q, pa, w));
-                        A[q] = -iv * A[q];
-                        C[q] = (r[q][j] - C[q]) * iv;
-                    }
-                }
-            }
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-#pragma unroll
-                for (int q = 0; q < NCI; ++q) {
-                    const double Ap = __shfl_up_sync(0xffffffffu, A[q], off);
-                    const double Cp = __shfl_up_sync(0xffffffffu, C[q], off);
-                    if (lane >= off) {
-                        C[q] = A[q] * Cp + C[q];
-                        A[q] = A[q] * Ap;
-                    }
-                }
-            }
-            double d[NCI];
-#pragma unroll
-            for (int q = 0; q < NCI; ++q) {
-                d[q] = __shfl_up_sync(0xffffffffu, C[q], 1);
-                if (lane == 0) d[q] = 0.0;
-            }
-#pragma unroll
-            for (int j = 0; j < B; ++j) {
-                const int p = p0 + j;
-                if (p < nt) {
-                    const double iv = invv[p];
-#pragma unroll
-                    for (int q = 0; q < NCI; ++q) {
-                        d[q] = (r[q][j] - d[q]) * iv;
-                        r[q][j] = d[q];
-                    }
-                }
-            }
-            // backward: the composed maps m_next -> G m_next + H of the lane's nodes
-            double G[NCI], H[NCI];
-#pragma unroll
-            for (int q = 0; q < NCI; ++q) {
-                G[q] = 1.0;
-                H[q] = 0.0;
-            }
-#pragma unroll
-            for (int j = B - 1; j >= 0; --j) {
-                const int p = p0 + j;
-                if (p < nt) {
-                    const double cc = cpv[p];
-#pragma unroll
-                    for (int q = 0; q < NCI; ++q) {
-                        H[q] = r[q][j] - cc * H[q];
-                        G[q] = -cc * G[q];
-                    }
-                }
-            }
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-#pragma unroll
-                for (int q = 0; q < NCI; ++q) {
-                    const double Gn = __shfl_down_sync(0xffffffffu, G[q], off);
-                    const double Hn = __shfl_down_sync(0xffffffffu, H[q], off);
-                    if (lane + off < 32) {
-                        H[q] = G[q] * Hn + H[q];
-                        G[q] = G[q] * Gn;
-                    }
-                }
-            }
-            double m[NCI];
-#pragma unroll
-            for (int q = 0; q < NCI; ++q) {
-                m[q] = __shfl_down_sync(0xffffffffu, H[q], 1);
-                if (lane == 31) m[q] = 0.0;
-            }
-#pragma unroll
-            for (int j = B - 1; j >= 0; --j) {
-                const int p = p0 + j;
-                if (p < nt) {
-                    const double cc = cpv[p];
-#pragma unroll
-                    for (int q = 0; q < NCI; ++q) {
-                        m[q] = r[q][j] - cc * m[q];
-                        r[q][j] = m[q];
-                    }
-                }
-            }
-            __syncwarp(); // every lane has read its neighbours' velocities
-#pragma unroll
-            for (int j = 0; j < B; ++j) {
-                const int p = p0 + j;
-                if (p < nt) {
-#pragma unroll
-                    for (int q = 0; q < NCI; ++q) T(1 + c0 + q, p, w) = r[q][j];
-                }
-            }
-            __syncwarp();
-        }
+    for (; p < nt - 1; ++p) {
+        const double next = c[(p + 1) * S];
+        d = fma(s, next - prev, -d) * inv[p];
+        c[p * S] = d;
+        prev = cur;
+        cur = next;
     }
-    __syncthreads();
-    // slopes of nodes 3 .. nt-4 (the interior cells)
-    each([&](int p, int line) {
-        if (p >= 3 && p <= nt - 4) {
-            const long long c = cell(line, AXIS == 0 ? p - f.yhost : p - 3);
+    double m = fma(s, cur - prev, -d) * inv[nt - 1];
+    c[(nt - 1) * S] = m;
+    p = nt - 2;
+    for (; p - G + 1 >= 0; p -= G) {
+        double f[G], cc[G];
 #pragma unroll
-            for (int a = 1; a < 4; ++a) scr[(3 + 3 * (a - 1) + AXIS) * n + c] = T(a, p, line);
+        for (int g = 0; g < G; ++g) {
+            f[g] = c[(p - g) * S];
+            cc[g] = cp[p - g];
         }
-    });
+#pragma unroll
+        for (int g = 0; g < G; ++g) f[g] = m = fma(-cc[g], m, f[g]);
+#pragma unroll
+        for (int g = 0; g < G; ++g) c[(p - g) * S] = f[g];
+    }
+    for (; p >= 0; --p) {
+        m = fma(-cp[p], m, c[p * S]);
+        c[p * S] = m;
+    }
 }
 
 constexpr int NSUM1 = kStatsSums;
@@ -1214,61 +1068,159 @@ __device__ __forceinline__ void cell_prim(const FieldDev &f, long long c, double
     T = P * ri * f.iR;
 }
 
-// One pass over the interior cells: the means PrintStats forms
-// (update.cpp:659-712) and, for the rms of p, T and 1/rho (update.cpp:751-762),
-// the first two moments of x - K with K the value at the first interior cell
-// (shifted one-pass variance, well conditioned because K lies inside the
-// field's range); K goes to kout[0..2].
-__global__ void __launch_bounds__(256, 2) k_sums1(FieldDev f, const double *scr, double *partial, double *kout)
+// A cell's terms of the means PrintStats forms (update.cpp:659-712) and, for
+// the rms of p, T and 1/rho (update.cpp:751-762), of the first two moments of x
+// - K with K the value at the first interior cell (shifted one-pass variance,
+// well conditioned because K lies inside the field's range).  g: d(u, v, w)/dy,
+// then /dx, then /dz.
+__device__ __forceinline__ void add_sums(const FieldDev &f, long long c, const double (&g)[9], double Kp, double Kt, double Kv,
+                                         double (&acc)[NSUM1])
 {
+    double den, ri, u, v, w, P, T;
+    cell_prim(f, c, den, ri, u, v, w, P, T);
+    const double dudy = g[0], dvdy = g[1], dwdy = g[2], dudx = g[3], dvdx = g[4], dwdx = g[5];
+    const double dudz = g[6], dvdz = g[7], dwdz = g[8];
+    const double mu = viscosity(f, T);
+    acc[0] += den * (u * u + v * v + w * w);
+    acc[1] += mu * (dudx * dudx + dudy * dudy + dudz * dudz + dvdx * dvdx + dvdy * dvdy + dvdz * dvdz + dwdx * dwdx +
+                    dwdy * dwdy + dwdz * dwdz);
+    acc[2] += dudx * dudx + 0.5 * (dudy + dvdx) * (dudy + dvdx) + 0.5 * (dudz + dwdx) * (dudz + dwdx) +
+              0.5 * (dwdy + dvdz) * (dwdy + dvdz) + dvdy * dvdy + dwdz * dwdz;
+    const double a2 = dudx * dudx, b2 = dvdy * dvdy, c2 = dwdz * dwdz;
+    acc[3] += a2; acc[4] += a2 * dudx; acc[5] += a2 * a2;
+    acc[6] += b2; acc[7] += b2 * dvdy; acc[8] += b2 * b2;
+    acc[9] += c2; acc[10] += c2 * dwdz; acc[11] += c2 * c2;
+    acc[12] += P;
+    acc[13] += T;
+    acc[14] += ri;
+    acc[15] += u * u + v * v + w * w;
+    acc[16] += sqrt(f.gam * P * ri);
+    acc[17] += den;
+    const double dP = P - Kp, dT = T - Kt, dV = ri - Kv;
+    acc[18] += dP;
+    acc[19] += dP * dP;
+    acc[20] += dT;
+    acc[21] += dT * dT;
+    acc[22] += dV;
+    acc[23] += dV * dV;
+}
+
+// The slopes along one axis.  The y and x passes write theirs to scr; the z
+// pass, last, adds every cell's terms straight from its tiles and the six
+// slopes before (partial: NSUM1 sums per block; kout: the shifts K), one wave
+// of blocks over all sets of lines.  HBM: 56 B a cell and pass for y and x, 88 B
+// for z and the sums (3.4 GB at 256^3, 0.51 ms); measured 275 + 272 + 532 us, a
+// block's load, solve and store phases only partly covered by the other's.
+// Before: a warp per line (affine-map scans, 40 instructions a node) and sums of
+// their own, 327 + 317 + 267 + 362 us.  Measured alternatives: 8 lines and 128
+// threads at four blocks per SM 329 + 315 + 800, 512 threads 285 + 283 (y, x).
+template <int AXIS, int LW>
+__global__ void __launch_bounds__(kSplineBlock, 2) k_spline(FieldDev f, double *scr, int nsets, double *partial, double *kout)
+{
+    using ST = SplineTiles<AXIS, LW>;
+    constexpr bool SUMS = AXIS == 2;
+    constexpr int NG = kSplineBlock / LW;    // y / x: threads on one line
+    constexpr int NW = kSplineBlock / 32;    // z: warps
+    extern __shared__ double smem[];
+    // nodes of a line: nc + 6 along x / z; along y ny + 2 yhost (the same for a
+    // periodic field; a slab's ny stored planes, its ghosts included)
+    const int nc = f.nc, nt = AXIS == 0 ? f.ny + 2 * f.yhost : nc + 6;
     const long long n = f.ncell;
-    const long long plane = (long long)f.nc * f.nc, c0 = f.ylo * plane, c1 = f.yhi * plane;
-    double acc[NSUM1];
+    const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    const int tsz = ST::tile(nt), pitch = nt | 1;
+    double *cpv = smem + 3 * tsz, *invv = cpv + nt;
+    // tile of velocity component a, node, line
+    auto T = [&](int a, int node, int line) -> double & {
+        return AXIS == 2 ? smem[a * tsz + line * pitch + node] : smem[a * tsz + node * LW + line];
+    };
+    for (int p = tid; p < nt; p += kSplineBlock) {
+        cpv[p] = AXIS == 0 ? f.spl_cpy[p] : f.spl_cp[p];
+        invv[p] = AXIS == 0 ? f.spl_invy[p] : f.spl_inv[p];
+    }
+    double acc[SUMS ? NSUM1 : 1];
+    double Kp = 0.0, Kt = 0.0, Kv = 0.0;
+    if constexpr (SUMS) {
 #pragma unroll
-    for (int i = 0; i < NSUM1; ++i) acc[i] = 0.0;
-    double Kp, Kt, Kv;
-    {
-        double den, u, v, w;
-        cell_prim(f, c0, den, Kv, u, v, w, Kp, Kt);
+        for (int i = 0; i < NSUM1; ++i) acc[i] = 0.0;
+        double den, u, v, x;
+        cell_prim(f, (long long)f.ylo * nc * nc, den, Kv, u, v, x, Kp, Kt);
+        if (blockIdx.x == 0 && tid == 0) {
+            kout[0] = Kp;
+            kout[1] = Kt;
+            kout[2] = Kv;
+        }
     }
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        kout[0] = Kp;
-        kout[1] = Kt;
-        kout[2] = Kv;
+    const int nkb = (nc + LW - 1) / LW;
+    const unsigned step = AXIS == 0 ? unsigned(nc) * nc : (AXIS == 1 ? nc : 1); // cells between positions of a line
+    for (int set = blockIdx.x; set < nsets; set += gridDim.x) {
+        // the block's lines: y / x lines are (outer, k) with k in [k0, k0 + LW),
+        // outer = i (y lines) or j (x lines, interior planes); z lines are l in
+        // [l0, l0 + LW), l = j nc + i (interior planes)
+        const int outer = AXIS == 2 ? 0 : (AXIS == 1 ? f.ylo : 0) + set / nkb;
+        const int k0 = AXIS == 2 ? 0 : (set % nkb) * LW;
+        const int l0 = AXIS == 2 ? f.ylo * nc + set * LW : 0;
+        const int live = AXIS == 2 ? min(LW, f.yhi * nc - l0) : min(LW, nc - k0); // lines of this set
+        auto base = [&](int line) -> unsigned {
+            if (AXIS == 0) return unsigned(outer) * nc + k0 + line;
+            if (AXIS == 1) return (unsigned(outer) * nc) * nc + k0 + line;
+            return unsigned(l0 + line) * nc;
+        };
+        // this thread's nodes, DP apart: y / x, LW consecutive threads on the LW lines
+        // of one node; z, a warp along the nodes of a line, NW lines apart
+        constexpr int DP = AXIS == 2 ? 32 : NG;
+        for (int line = AXIS == 2 ? w : tid % LW; line < live; line += AXIS == 2 ? NW : LW) {
+            const unsigned cb = base(line);
+            // velocities at the nodes (node p holds cell wrap(p - 3); along y plane
+            // wrap(p - yhost, nyw), a slab's plane p)
+            for (int p = AXIS == 2 ? lane : tid / LW; p < nt; p += DP * kStage) {
+                double v[kStage][4];
+#pragma unroll
+                for (int h = 0; h < kStage; ++h) {
+                    const int q = p + DP * h;
+                    const unsigned c = cb + step * unsigned(AXIS == 0 ? wrap(q - f.yhost, f.nyw) : wrap(q - 3, nc));
+#pragma unroll
+                    for (int a = 0; a < 4; ++a) v[h][a] = q < nt ? __ldg(f.W[a] + c) : 1.0;
+                }
+#pragma unroll
+                for (int h = 0; h < kStage; ++h) {
+                    const int q = p + DP * h;
+                    const double ri = __drcp_rn(v[h][0]);
+                    if (q < nt)
+#pragma unroll
+                        for (int a = 0; a < 3; ++a) T(a, q, line) = v[h][a + 1] * ri;
+                }
+            }
+        }
+        __syncthreads();
+        if (tid < 3 * LW && tid % LW < live)
+            spline_slopes<AXIS == 2 ? 1 : LW>(&T(tid / LW, 0, tid % LW), nt, AXIS == 0 ? f.spl_sy : f.spl_s, invv, cpv);
+        __syncthreads();
+        // slopes of nodes 3 .. nt-4 (the interior cells)
+        if constexpr (SUMS) {
+            for (int e = tid; e < live * nc; e += kSplineBlock) {
+                const int line = e / nc, k = e - line * nc;
+                const long long c = (long long)l0 * nc + e;
+                double g[9];
+#pragma unroll
+                for (int a = 0; a < 3; ++a) {
+                    g[a] = __ldg(scr + (3 * a) * n + c);
+                    g[3 + a] = __ldg(scr + (3 * a + 1) * n + c);
+                    g[6 + a] = T(a, k + 3, line);
+                }
+                add_sums(f, c, g, Kp, Kt, Kv, acc);
+            }
+        } else {
+            const int line = tid % LW;
+            if (line < live)
+                for (int p = 3 + tid / LW; p < nt - 3; p += NG) {
+                    const unsigned c = base(line) + step * unsigned(AXIS == 0 ? p - f.yhost : p - 3);
+#pragma unroll
+                    for (int a = 0; a < 3; ++a) scr[(3 * a + AXIS) * n + c] = T(a, p, line);
+                }
+        }
+        __syncthreads();
     }
-    const long long stride = (long long)gridDim.x * blockDim.x;
-    for (long long c = c0 + (long long)blockIdx.x * blockDim.x + threadIdx.x; c < c1; c += stride) {
-        double den, ri, u, v, w, P, T;
-        cell_prim(f, c, den, ri, u, v, w, P, T);
-        const double *g = scr + 3 * n;
-        const double dudy = g[c], dudx = g[n + c], dudz = g[2 * n + c];
-        const double dvdy = g[3 * n + c], dvdx = g[4 * n + c], dvdz = g[5 * n + c];
-        const double dwdy = g[6 * n + c], dwdx = g[7 * n + c], dwdz = g[8 * n + c];
-        const double mu = viscosity(f, T);
-        acc[0] += den * (u * u + v * v + w * w);
-        acc[1] += mu * (dudx * dudx + dudy * dudy + dudz * dudz + dvdx * dvdx + dvdy * dvdy + dvdz * dvdz +
-                        dwdx * dwdx + dwdy * dwdy + dwdz * dwdz);
-        acc[2] += dudx * dudx + 0.5 * (dudy + dvdx) * (dudy + dvdx) + 0.5 * (dudz + dwdx) * (dudz + dwdx) +
-                  0.5 * (dwdy + dvdz) * (dwdy + dvdz) + dvdy * dvdy + dwdz * dwdz;
-        const double a2 = dudx * dudx, b2 = dvdy * dvdy, c2 = dwdz * dwdz;
-        acc[3] += a2; acc[4] += a2 * dudx; acc[5] += a2 * a2;
-        acc[6] += b2; acc[7] += b2 * dvdy; acc[8] += b2 * b2;
-        acc[9] += c2; acc[10] += c2 * dwdz; acc[11] += c2 * c2;
-        acc[12] += P;
-        acc[13] += T;
-        acc[14] += ri;
-        acc[15] += u * u + v * v + w * w;
-        acc[16] += sqrt(f.gam * P * ri);
-        acc[17] += den;
-        const double dP = P - Kp, dT = T - Kt, dV = ri - Kv;
-        acc[18] += dP;
-        acc[19] += dP * dP;
-        acc[20] += dT;
-        acc[21] += dT * dT;
-        acc[22] += dV;
-        acc[23] += dV * dV;
-    }
-    block_sums<NSUM1>(acc, partial + (long long)blockIdx.x * NSUM1);
+    if constexpr (SUMS) block_sums<NSUM1>(acc, partial + (long long)blockIdx.x * NSUM1);
 }
 
 // Sum the per-block partials, one warp per quantity, in a fixed order (so the
@@ -1445,43 +1397,39 @@ cudaError_t launch_maxwave(const FieldDev &f, unsigned long long *out_bits, int 
     return cudaGetLastError();
 }
 
-template <int AXIS, int B, int LW>
-cudaError_t spline_go(const FieldDev &f, double *scratch, cudaStream_t st)
+template <int AXIS, int LW>
+cudaError_t spline_go(const FieldDev &f, double *scratch, double *partial, double *kout, int max_grid, int *grid, cudaStream_t st)
 {
-    const size_t bytes = SplineTiles<AXIS, B, LW>::bytes(f.nc + 6);
-    cudaError_t e = cudaFuncSetAttribute(k_spline_scan<AXIS, B, LW>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)bytes);
+    const size_t bytes = SplineTiles<AXIS, LW>::bytes(f.nc + 6);
+    cudaError_t e = cudaFuncSetAttribute(k_spline<AXIS, LW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     if (e != cudaSuccess) return e;
     // lines: y lines (i, k) of the whole slab, x and z lines of the interior planes
-    const long long ny = f.yhi - f.ylo;
-    const long long sets = AXIS == 2 ? (ny * f.nc + LW - 1) / LW
-                                     : (AXIS == 0 ? f.nc : ny) * ((f.nc + LW - 1) / LW);
-    k_spline_scan<AXIS, B, LW><<<(unsigned)sets, 32 * LW, bytes, st>>>(f, scratch);
+    const int ny = f.yhi - f.ylo;
+    const int sets = AXIS == 2 ? (ny * f.nc + LW - 1) / LW : (AXIS == 0 ? f.nc : ny) * ((f.nc + LW - 1) / LW);
+    *grid = std::min(sets, max_grid);
+    k_spline<AXIS, LW><<<*grid, kSplineBlock, bytes, st>>>(f, scratch, sets, partial, kout);
     return cudaGetLastError();
 }
 
-// Nodes per lane B (odd, 32 B >= nt) and lines per block LW: 8 lines (64
-// contiguous bytes per row of a y / x tile) up to nt = 288, 4 beyond, so that
-// the four tiles stay within 170 KB of shared memory.
+// Lines per block: 16 (128 contiguous bytes per row of a y / x tile) up to nt =
+// 288, 8 beyond, so that two blocks fit an SM's shared memory up to nt = 576.
 template <int AXIS>
-cudaError_t spline_axis(const FieldDev &f, double *scratch, cudaStream_t st)
+cudaError_t spline_axis(const FieldDev &f, double *scratch, double *partial, double *kout, int max_grid, int *grid,
+                        cudaStream_t st)
 {
-    const int nt = f.nc + 6;
-    if (nt <= 160) return spline_go<AXIS, 5, 8>(f, scratch, st);
-    if (nt <= 288) return spline_go<AXIS, 9, 8>(f, scratch, st);
-    if (nt <= 544) return spline_go<AXIS, 17, 4>(f, scratch, st);
-    return spline_go<AXIS, 33, 4>(f, scratch, st);
+    if (f.nc + 6 <= 288) return spline_go<AXIS, 16>(f, scratch, partial, kout, max_grid, grid, st);
+    return spline_go<AXIS, 8>(f, scratch, partial, kout, max_grid, grid, st);
 }
 
 cudaError_t launch_stats(const FieldDev &f, double *scratch, double *partial, double *sums, int nsm, cudaStream_t st)
 {
-    const int block = 256;
-    const int grid = stats_grid(f.ncell, block, nsm); // partial holds stats_partial_elems(nsm) >= kStatsSums * grid
-    cudaError_t e = spline_axis<0>(f, scratch, st);
-    if (e == cudaSuccess) e = spline_axis<1>(f, scratch, st);
-    if (e == cudaSuccess) e = spline_axis<2>(f, scratch, st);
+    int grid = 0;
+    cudaError_t e = spline_axis<0>(f, scratch, nullptr, nullptr, INT_MAX, &grid, st);
+    if (e == cudaSuccess) e = spline_axis<1>(f, scratch, nullptr, nullptr, INT_MAX, &grid, st);
+    // partial holds stats_partial_elems(nsm) >= kStatsSums * stats_grid
+    const int wave = std::min(2 * nsm, stats_grid(f.ncell, kSplineBlock, nsm));
+    if (e == cudaSuccess) e = spline_axis<2>(f, scratch, partial, sums + NSUM1, wave, &grid, st);
     if (e != cudaSuccess) return e;
-    k_sums1<<<grid, block, 0, st>>>(f, scratch, partial, sums + NSUM1);
     const double cells = double(f.yhi - f.ylo) * f.nc * f.nc;
     k_finalize<<<1, 32 * NSUM1, 0, st>>>(partial, grid, NSUM1, 1.0 / cells, sums);
     return cudaGetLastError();

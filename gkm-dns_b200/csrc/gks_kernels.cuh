@@ -149,8 +149,8 @@ cudaError_t launch_scatter(const FieldDev &f, double *stage, int nsm, cudaStream
 // *out_bits must be zero on entry).
 cudaError_t launch_maxwave(const FieldDev &f, unsigned long long *out_bits, int nsm, cudaStream_t st);
 
-// Statistics of one field over its interior planes.  scratch: 12 * ncell doubles
-// (the first 3 unused); partial: stats_partial_elems(nsm) doubles.
+// Statistics of one field over its interior planes.  scratch: 9 * ncell doubles;
+// partial: stats_partial_elems(nsm) doubles.
 // Writes 24 means into sums[0..23]: the 18 PrintStats means and, for p, T and
 // 1/rho, the means of x - K and (x - K)^2, and K itself into sums[24..26]
 // (K = the values at the first interior cell).

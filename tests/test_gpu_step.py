@@ -565,3 +565,16 @@ def test_line_lengths_match_oracle(gks, oracle, nc):
         oracle.step(ref, prm, dt, 2)
         err = np.abs(got - ref).reshape(5, -1).max(1) / np.abs(ref).reshape(5, -1).max(1)
         assert np.all(err < tol), (prec, err)
+
+
+@pytest.mark.parametrize("nc", [4, 5, 9, 10, 11, 15, 17, 33, 282])
+def test_stats_at_tile_edges_match_oracle(gks, oracle, nc):
+    """Lines a few nodes more or fewer than the groups of eight the spline
+    recurrences move in, fewer lines than a block takes, one line beyond a
+    block's sixteen, and the longest line of the sixteen-line form."""
+    case, W = analytic_case(nc, seed=nc)
+    prm = oracle.params(nc, case.gam, case.mu0, case.p0, 1.0, case.Mt, case.t0)
+    with gks.Solver(gks.phys_from_case(case)) as s:
+        s.upload(W)
+        got = s.stats_array()
+    np.testing.assert_allclose(got, oracle.stats(W, prm), rtol=STATS_RTOL, atol=1e-300)
