@@ -3,7 +3,7 @@
 // A context owns, per field, one device allocation of 32 * nc^3 doubles
 // (state 5, reconstruction records 10, fluxes 15, mu/p 2; the statistics reuse
 // the flux arrays as scratch), the field's descriptor in a device array, and one
-// CUDA graph holding a whole step for all fields (seven persistent launches).
+// CUDA graph holding a whole step for all fields (seven launches, or six).
 // The reference instead allocates 50 padded arrays per rank and copies the
 // whole field host<->device every step (GPUAlloc.cu:3-17, GPUupdate.cu:74-190).
 #include "../../include/gks_b200.h"
@@ -250,6 +250,23 @@ std::string tune_key(const gks_ctx *ctx)
 
 int record_slab_step(gks_ctx *ctx);
 
+// Whether the z flux applies the update itself (k_flux_update): one field whose
+// sweeps run one after the other (with concurrent sweeps the x and y fluxes
+// still read the state) and whose z lines fill the warps' 32 lanes (at 250^3,
+// where 2.4 % of them idle, nothing is left of the gain).  us per step,
+// separate / with the flux, runs in turn: FP64 128^3 989 / 971, 256^3 7596 / 7469;
+// mixed 128^3 858 / 845, 256^3 6741 / 6605, 320^3 13265 / 12947, 512^3 55859 / 54205.
+bool update_with_flux(const gks_ctx *ctx)
+{
+    return ctx->nfields == 1 && ctx->fh[0].phys.nc % 32 == 0;
+}
+
+int launch_flux_update(gks_ctx *ctx)
+{
+    CK(gks::launch_flux_update(ctx->batch, ctx->precision, ctx->nsm, ctx->stream));
+    return GKS_OK;
+}
+
 int record_step(gks_ctx *ctx)
 {
     if (ctx->fh[0].slab) return record_slab_step(ctx);
@@ -276,6 +293,7 @@ int record_step(gks_ctx *ctx)
     }
     for (int dir = 0; dir < 3; ++dir) {
         CK(gks::launch_recon(ctx->batch, dir, ctx->precision, ctx->cfg[gks::K_RECON][dir], ctx->stream));
+        if (dir == 2 && update_with_flux(ctx)) return launch_flux_update(ctx);
         CK(gks::launch_flux(ctx->batch, dir, ctx->precision, ctx->cfg[gks::K_FLUX][dir], ctx->stream));
     }
     CK(gks::launch_update(ctx->batch, ctx->cfg[gks::K_UPDATE][0], ctx->stream));

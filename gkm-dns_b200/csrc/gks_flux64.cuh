@@ -265,8 +265,10 @@ __device__ __forceinline__ void flux_side(const Src &src, const FluxConst64 &c)
 //   src.cells(WL, WR)         the cell averages either side of the interface
 //   src.sum<side>(slot, v)    side 0 stores, side 1 adds; src.get(slot), src.put(slot, v)
 // mu/p at the left cell = tau_n / tau_d.  Output F[5], integrated over [0, dt].
-template <typename Src>
-__device__ __forceinline__ void gks_flux64(const Src &src, double tau_n, double tau_d, const FluxConst64 &c, double F[5])
+// ahead() is called when the inputs have been read (their slots are free).
+template <typename Src, typename Ahead>
+__device__ __forceinline__ void gks_flux64(const Src &src, double tau_n, double tau_d, const FluxConst64 &c,
+                                           const Ahead &ahead, double F[5])
 {
     const double dt = c.dt;
     {
@@ -327,6 +329,7 @@ __device__ __forceinline__ void gks_flux64(const Src &src, double tau_n, double 
         to_frame(b, m, hU);
         solve(b, m.k3, 1.0, m.tl, m.kh, z);
     }
+    ahead();
     const double vx = fma(m.k5, x[4], x[0]), vy = fma(m.k5, y[4], y[0]), vz = fma(m.k5, z[4], z[0]);
     const double D = x[1] + (y[2] + z[3]);
     // full-space second-order part of the flux, <psi'' u (c . slopes)>, in units of s

@@ -657,6 +657,8 @@ struct SweepSrc {
     double (*park_w)[kFluxBlock];  // [15][block]: WL, WR, Wr
     double (*sum_d)[kFluxBlock];   // [10][block]: double sums of the side passes
 
+    // RO: the state is not written by this kernel
+    template <bool RO>
     __device__ __forceinline__ void load(const FieldDev &f, unsigned c, unsigned c1, unsigned cn, unsigned cs,
                                          unsigned cf, unsigned cb)
     {
@@ -665,7 +667,7 @@ struct SweepSrc {
 #pragma unroll
         for (int q = 0; q < 5; ++q) {
             const int o = perm<DIR>(q);
-            const double wL = __ldg(f.W[o] + c), wR = __ldg(f.W[o] + c1);
+            const double wL = RO ? __ldg(f.W[o] + c) : f.W[o][c], wR = RO ? __ldg(f.W[o] + c1) : f.W[o][c1];
             const double wr = r.r0[5 + o];
             Wl[q] = r.r0[o];
             DWl[0][q] = float(Wl[q] - wL);
@@ -724,7 +726,8 @@ template <> struct FluxPark<1> {
     float dw[15][kFluxBlock];
 };
 
-template <int DIR> __device__ __forceinline__ void store_flux(const FieldDev &f, unsigned c, double F[5])
+// The flux at cell c, components in the state's order.
+template <int DIR> __device__ __forceinline__ void unrotate(double F[5])
 {
     constexpr int ROT = DIR == 0 ? 0 : (DIR == 1 ? 2 : 3);
     if (ROT) {
@@ -732,13 +735,22 @@ template <int DIR> __device__ __forceinline__ void store_flux(const FieldDev &f,
         F[1] = F[ROT];
         F[ROT] = t;
     }
+}
+
+template <int DIR> __device__ __forceinline__ void store_flux(const FieldDev &f, unsigned c, const double F[5])
+{
 #pragma unroll
     for (int q = 0; q < 5; ++q) f.F[DIR * 5 + q][c] = F[q];
 }
 
-// FP64: the flux at cell c.
-template <int DIR>
-__device__ __forceinline__ void flux_item64(const FieldDev &f, unsigned c, const SweepSrc64<DIR> &src)
+struct Nothing {
+    __device__ __forceinline__ void operator()() const {}
+};
+
+// FP64.
+template <int DIR, typename Ahead>
+__device__ __forceinline__ void flux_item64(const FieldDev &f, unsigned c, const SweepSrc64<DIR> &src, const Ahead &ahead,
+                                            double F[5])
 {
     const Cell x = decode(c, f);
     unsigned cn, cs, cf, cb;
@@ -749,15 +761,13 @@ __device__ __forceinline__ void flux_item64(const FieldDev &f, unsigned c, const
     const double tau_n = __ldg(f.tau[0] + c), tau_d = __ldg(f.tau[1] + c);
     const FluxConst64 fc = {f.dt,  f.gm1,  f.igm1,  f.shig,  f.rlg,   f.ksn,   f.kst,
                             f.kA4, f.prm1, f.kd[0], f.kd[1], f.kd[2], f.kd[3], f.kd[4]};
-    double F[5];
-    gks_flux64(src, tau_n, tau_d, fc, F);
-    store_flux<DIR>(f, c, F);
+    gks_flux64(src, tau_n, tau_d, fc, ahead, F);
+    unrotate<DIR>(F);
 }
 
-// Mixed: all global loads are issued at once when the interface starts, so
-// that their latency overlaps.
-template <int DIR>
-__device__ __forceinline__ void flux_item(const FieldDev &f, unsigned c, FluxPark<1> &park)
+// Mixed.
+template <int DIR, bool RO>
+__device__ __forceinline__ void flux_item(const FieldDev &f, unsigned c, FluxPark<1> &park, double F[5])
 {
     const Cell x = decode(c, f);
     unsigned cn, cs, cf, cb;
@@ -766,7 +776,7 @@ __device__ __forceinline__ void flux_item(const FieldDev &f, unsigned c, FluxPar
     src.park_dw = park.dw;
     src.park_w = park.w;
     src.sum_d = park.sum;
-    src.load(f, c, along<DIR>(x, 1), cn, cs, cf, cb);
+    src.template load<RO>(f, c, along<DIR>(x, 1), cn, cs, cf, cb);
     const double tau_n = __ldg(f.tau[0] + c), tau_d = __ldg(f.tau[1] + c);
     FluxConst fc;
     fc.gm1 = f.gm1;
@@ -778,9 +788,8 @@ __device__ __forceinline__ void flux_item(const FieldDev &f, unsigned c, FluxPar
     fc.kA = f.kA;
     fc.hK2 = f.hK2;
     fc.kf = {f.kf[0], f.kf[1], f.kf[2], f.kf[3]};
-    double F[5];
     gks_flux(src, tau_n, tau_d, fc, F);
-    store_flux<DIR>(f, c, F);
+    unrotate<DIR>(F);
 }
 
 // A batch of one field reads the field's descriptor from the launch
@@ -811,11 +820,18 @@ __global__ void __launch_bounds__(kFluxBlock) __maxnreg__(REGS) k_flux(Batch b)
             unsigned next = 0;
             if (lane == 0) next = nwarps + atomicAdd(queue, 1u);
             const long long it = b.lo + (long long)chunk * 32 + lane;
+            double F[5];
             if (b.nfields == 1) {
-                if (it < end) flux_item64<DIR>(b.one, unsigned(it), src);
+                if (it < end) {
+                    flux_item64<DIR>(b.one, unsigned(it), src, Nothing(), F);
+                    store_flux<DIR>(b.one, unsigned(it), F);
+                }
             } else {
                 const FieldDev &f = b.fields[field_of(b.fields, b.nfields, it)];
-                if (it - f.base < f.ncell) flux_item64<DIR>(f, unsigned(it - f.base), src); // alignment padding after the field
+                if (it - f.base < f.ncell) { // else alignment padding after the field
+                    flux_item64<DIR>(f, unsigned(it - f.base), src, Nothing(), F);
+                    store_flux<DIR>(f, unsigned(it - f.base), F);
+                }
             }
             chunk = __shfl_sync(0xffffffffu, next, 0);
         }
@@ -826,17 +842,31 @@ __global__ void __launch_bounds__(kFluxBlock) __maxnreg__(REGS) k_flux(Batch b)
         return;
     } else {
         const long long stride = (long long)gridDim.x * blockDim.x;
+        double F[5];
         if (b.nfields == 1) {
-            for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < end; it += stride)
-                flux_item<DIR>(b.one, unsigned(it), park);
+            for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < end; it += stride) {
+                flux_item<DIR, true>(b.one, unsigned(it), park, F);
+                store_flux<DIR>(b.one, unsigned(it), F);
+            }
             return;
         }
         for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < b.hi; it += stride) {
             const FieldDev &f = b.fields[field_of(b.fields, b.nfields, it)];
             if (it - f.base >= f.ncell) continue; // alignment padding after the field
-            flux_item<DIR>(f, unsigned(it - f.base), park);
+            flux_item<DIR, true>(f, unsigned(it - f.base), park, F);
+            store_flux<DIR>(f, unsigned(it - f.base), F);
         }
     }
+}
+
+// Finite, with positive density and pressure.  The division is left out where
+// rho^2 p / (gamma - 1) = rho2p(w) is well above its rounding.
+__device__ __forceinline__ bool physical(const double w[5], double gm1)
+{
+    const double e = w[0] * w[4];
+    if (w[0] > 0.0 && rho2p(w) > 1e-8 * e && e > 0.0 && isfinite(w[0] + w[1] + w[2] + w[3] + w[4])) return true;
+    const double p = gm1 * (w[4] - 0.5 * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]) / w[0]);
+    return w[0] > 0.0 && p > 0.0 && isfinite(w[0] + w[1] + w[2] + w[3] + w[4]);
 }
 
 // ---------------------------------------------------------------------------
@@ -865,9 +895,116 @@ __global__ void __launch_bounds__(kUpdateBlock) k_update(Batch b)
             w[q] = __dsub_rn(f.W[q][c], __dmul_rn(f.inv_dx, d));
             f.Wout[q][c] = w[q];
         }
-        const double p = f.gm1 * (w[4] - 0.5 * (w[1] * w[1] + w[2] * w[2] + w[3] * w[3]) / w[0]);
-        if (!(w[0] > 0.0) || !(p > 0.0) || !isfinite(w[0] + w[1] + w[2] + w[3] + w[4]))
-            atomicOr(b.err, 1);
+        if (!physical(w, f.gm1)) atomicOr(b.err, 1);
+    }
+}
+
+// ---------------------------------------------------------------------------
+// z flux and update of one field in one kernel, in place.  A warp walks whole z
+// lines (drawn from the queue of k_flux), 32 interfaces at a time: a lane's
+// lower z flux comes from the lane below by a shuffle, lane 0's from the chunk
+// before (park), and the x and y fluxes of its cell arrive by asynchronous
+// copies while the equilibrium pass is computed.  The state of a cell is read
+// by its own warp only (as left or right cell average), before it is written;
+// cell 0, which the line's last interface reads and whose lower flux is that
+// interface's, is written last.  The update alone is bound by HBM (200 B a
+// cell, 0.50 ms at 256^3); here its traffic, 120 B without the z fluxes, passes
+// under the flux's arithmetic.  The arithmetic is that of k_flux and k_update.
+// ---------------------------------------------------------------------------
+template <int PREC> struct LinePark;
+template <> struct LinePark<0> {
+    FluxPark<0> flux;
+    double line[kFluxBlock / 32][10]; // per warp: z flux below the next chunk; cell 0's sum of flux differences
+};
+template <> struct LinePark<1> {
+    FluxPark<1> flux;
+    double xy[20][kFluxBlock];
+    double line[kFluxBlock / 32][10];
+};
+
+template <int PREC, int REGS>
+__global__ void __launch_bounds__(kFluxBlock) __maxnreg__(REGS) k_flux_update(Batch b)
+{
+    __shared__ LinePark<PREC> park;
+    const FieldDev &f = b.one;
+    const int t = threadIdx.x, lane = t & 31;
+    const int nc = f.nc;
+    const unsigned nwarps = gridDim.x * (kFluxBlock / 32), lines = unsigned(f.ncell / nc);
+    unsigned *queue = b.queue + 4;
+    double *below = park.line[t >> 5], *first = below + 5;
+    // slots of the cell's Fx, Fx below, Fy, Fy below: FP64 in those of the inputs
+    // behind the left cell average, free once the equilibrium pass has read them
+    double (*xy)[kFluxBlock];
+    if constexpr (PREC == 0) xy = park.flux.slots + SweepSrc64<2>::kWR;
+    else xy = park.xy;
+    static_assert(SweepSrc64<2>::kWR == 5 && SweepSrc64<2>::kW0 == 25, "twenty input slots between WL and the sums");
+    for (unsigned line = (blockIdx.x * kFluxBlock + t) >> 5; line < lines;) {
+        unsigned next = 0;
+        if (lane == 0) next = nwarps + atomicAdd(queue, 1u);
+        const unsigned lbase = line * unsigned(nc);
+        for (int k0 = 0; k0 < nc; k0 += 32) {
+            const int k = k0 + lane;
+            const unsigned c = lbase + unsigned(min(k, nc - 1)); // lanes past the line repeat its last cell
+            auto fetch = [&]() {
+                const Cell x = decode(c, f);
+                const unsigned cx = along<0>(x, -1), cy = along<1>(x, -1);
+#pragma unroll
+                for (int q = 0; q < 5; ++q) {
+                    cp_async8(&xy[q][t], f.F[q] + c);
+                    cp_async8(&xy[5 + q][t], f.F[q] + cx);
+                    cp_async8(&xy[10 + q][t], f.F[5 + q] + c);
+                    cp_async8(&xy[15 + q][t], f.F[5 + q] + cy);
+                }
+                cp_async_commit();
+            };
+            double F[5], w[5];
+            if constexpr (PREC == 0) {
+                const SweepSrc64<2> src{park.flux.slots};
+                flux_item64<2>(f, c, src, fetch, F);
+#pragma unroll
+                for (int q = 0; q < 5; ++q) w[q] = src.at(SweepSrc64<2>::kWL + perm<2>(q));
+            } else {
+                fetch();
+                flux_item<2, false>(f, c, park.flux, F);
+#pragma unroll
+                for (int q = 0; q < 5; ++q) w[q] = park.flux.w[perm<2>(q)][t];
+            }
+            cp_async_wait<0>();
+            const int last = min(31, nc - 1 - k0); // the lane whose z flux the next chunk (or cell 0) takes
+            bool bad = false;
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                double d = __dsub_rn(xy[q][t], xy[5 + q][t]);
+                d = __dadd_rn(d, xy[10 + q][t]);
+                d = __dsub_rn(d, xy[15 + q][t]);
+                d = __dadd_rn(d, F[q]);
+                const double up = __shfl_sync(0xffffffffu, F[q], lane ? lane - 1 : last);
+                const double lo = lane ? up : below[q];
+                if (lane == 0) below[q] = up;
+                if (k == 0) {
+                    first[q] = d;
+                } else if (k < nc) {
+                    w[q] = __dsub_rn(w[q], __dmul_rn(f.inv_dx, __dsub_rn(d, lo)));
+                    f.W[q][c] = w[q];
+                }
+            }
+            if (k > 0 && k < nc) bad = !physical(w, f.gm1);
+            if (bad) atomicOr(b.err, 1);
+        }
+        if (lane == 0) {
+            double w[5];
+#pragma unroll
+            for (int q = 0; q < 5; ++q) {
+                w[q] = __dsub_rn(f.W[q][lbase], __dmul_rn(f.inv_dx, __dsub_rn(first[q], below[q])));
+                f.W[q][lbase] = w[q];
+            }
+            if (!physical(w, f.gm1)) atomicOr(b.err, 1);
+        }
+        line = __shfl_sync(0xffffffffu, next, 0);
+    }
+    if (lane == 0 && atomicAdd(queue + 1, 1u) == nwarps - 1) {
+        queue[0] = 0;
+        queue[1] = 0;
     }
 }
 
@@ -1365,6 +1502,18 @@ cudaError_t launch_update(const Batch &batch, LaunchCfg cfg, cudaStream_t st)
     const Batch b = resolve_range(batch, K_UPDATE, 0);
     if (b.hi <= b.lo) return cudaSuccess;
     k_update<<<range_grid(cfg.grid, b.hi - b.lo, cfg.block), cfg.block, 0, st>>>(b);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_flux_update(const Batch &b, int prec, int nsm, cudaStream_t st)
+{
+    int per_sm = 1;
+    cudaError_t e = prec == 0 ? occ(k_flux_update<0, kFluxRegs[1]>, kFluxBlock, &per_sm) : occ(k_flux_update<1, kFluxRegs[1]>, kFluxBlock, &per_sm);
+    if (e != cudaSuccess) return e;
+    const long long lines = b.one.ncell / b.one.nc;
+    const int g = range_grid(nsm * std::max(per_sm, 1), lines, kFluxBlock / 32);
+    if (prec == 0) k_flux_update<0, kFluxRegs[1]><<<g, kFluxBlock, 0, st>>>(b);
+    else k_flux_update<1, kFluxRegs[1]><<<g, kFluxBlock, 0, st>>>(b);
     return cudaGetLastError();
 }
 

@@ -131,6 +131,8 @@ inline long long batch_items(const Batch &b, int kind, int dir)
 cudaError_t launch_recon(const Batch &b, int dir, int prec, LaunchCfg cfg, cudaStream_t st);
 cudaError_t launch_flux(const Batch &b, int dir, int prec, LaunchCfg cfg, cudaStream_t st);
 cudaError_t launch_update(const Batch &b, LaunchCfg cfg, cudaStream_t st);
+// The z flux and the update of a one-field batch together, in place (Wout == W).
+cudaError_t launch_flux_update(const Batch &b, int prec, int nsm, cudaStream_t st);
 
 // Resident blocks per SM of a kernel kind / variant (for persistent grids).
 cudaError_t max_resident_blocks(int kind, int dir, int prec, int variant, int block, int *blocks_per_sm);

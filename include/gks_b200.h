@@ -225,7 +225,9 @@ int gks_select_device(int device);
 
 /* Advance reps steps launching the seven stages one by one with CUDA events
  * between them; ms[0..6] receives the mean time of recon x, flux x, recon y,
- * flux y, recon z, flux z, update.  For profiling: the state advances. */
+ * flux y, recon z, flux z, update.  For profiling: the state advances.
+ * (gks_step applies the update inside the z flux for a large field whose nc is
+ * a multiple of 32, with the same result.) */
 int gks_time_stages(gks_ctx *ctx, int reps, double *ms);
 
 /* Tune the launch configuration of the reconstruction and flux kernels of

@@ -578,3 +578,31 @@ def test_stats_at_tile_edges_match_oracle(gks, oracle, nc):
         s.upload(W)
         got = s.stats_array()
     np.testing.assert_allclose(got, oracle.stats(W, prm), rtol=STATS_RTOL, atol=1e-300)
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_update_inside_the_z_flux_is_the_separate_update(gks, prec):
+    """A large field whose z lines fill whole warps takes the update inside the z
+    flux kernel: bit for bit the state of the stages launched one by one, and
+    the same report of a step that breaks the state."""
+    nc = 128
+    case = gks_ic.make_dhit(nc, k0=4.0, Mt=0.5, seed=4)
+    W = gks_ic.to_conservative_padded(case)
+    out = []
+    with gks.Solver(gks.phys_from_case(case), gks.FP64 if prec == "fp64" else gks.MIXED) as s:
+        for staged in (False, True):
+            s.upload(W)
+            s.timestep(0.5)
+            if staged:
+                s.time_stages(3)
+            else:
+                s.step(3)
+            s.sync()
+            out.append(s.download())
+        assert np.array_equal(out[0], out[1])
+        s.upload(near_vacuum_double_rarefaction(case))
+        s.timestep(0.5)
+        s.step(1)
+        with pytest.raises(gks.GksError) as ei:
+            s.sync()
+        assert ei.value.code == -5
