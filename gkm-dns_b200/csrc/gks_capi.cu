@@ -2,7 +2,8 @@
 //
 // A context owns, per field, one device allocation of 32 * nc^3 doubles
 // (state 5, reconstruction records 10, fluxes 15, mu/p 2; the statistics reuse
-// the flux arrays as scratch), the field's descriptor in a device array, and one
+// the flux arrays as scratch; 52 * nc^3 up to kSweepCells cells, with
+// reconstruction records per sweep), the field's descriptor in a device array, and one
 // CUDA graph holding a whole step for all fields (seven launches, or six).
 // The reference instead allocates 50 padded arrays per rank and copies the
 // whole field host<->device every step (GPUAlloc.cu:3-17, GPUupdate.cu:74-190).

@@ -34,7 +34,7 @@
 // The algebra is the reference's; only the order of evaluation differs, so
 // results agree with it to rounding.
 //
-// Bound: the FP64 pipe.  About 1010 FP64 instructions per interface (1471 with
+// Bound: the FP64 pipe.  1111 FP64 instructions per interface (1471 with
 // tables of the full space as well and a moment vector per slope).
 #pragma once
 

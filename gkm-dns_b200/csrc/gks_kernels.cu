@@ -3,9 +3,9 @@
 // A step is seven launches over every field of the batch: for each sweep
 // direction a reconstruction launch (WENO once per cell line and interface)
 // and a flux launch (transverse slopes from the neighbouring lines' WENO
-// states, BGK-NS flux), then the conservative update.  All launches are
-// persistent grid-stride loops over the cells of all fields, so one launch
-// covers an ensemble of fields of different sizes.  The periodic halo of the
+// states, BGK-NS flux), then the conservative update; or six, where the z flux
+// applies the update itself.  Every launch loops over the cells of all
+// fields, so one launch covers an ensemble of fields of different sizes.  The periodic halo of the
 // reference (HaloTransfer on one rank, update.cpp:894-1054) is the index wrap
 // in `along` and in the windowed reconstruction's cell map.
 #include "gks_device.cuh"

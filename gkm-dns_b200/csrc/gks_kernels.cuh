@@ -25,7 +25,7 @@ struct FieldDev {
     double *W[5];     // state, interior layout
     double *Wout[5];  // where the update writes the new state: W itself, except in the slab-pipelined host step
     double *rec[3];   // per sweep x, y, z: five arrays of nc^3 16-byte pairs, Wl[0..4] then Wr[0..4]
-                      // (one shared buffer except in the pipelined step)
+                      // (one shared buffer except in small batches and the pipelined step)
     double *F[15];    // Fx[0..4], Fy[0..4], Fz[0..4]
     double *tau[2];   // mu/p of each cell as numerator / denominator, set by the x-sweep reconstruction
     const double *spl_cp;   // natural-spline Thomas coefficients of the x / z lines, nc + 6 entries

@@ -146,7 +146,7 @@ __device__ __forceinline__ void bspline_line(int N, double *c, long long s, cons
 template <int AXIS>
 __global__ void __launch_bounds__(kLineBlock) k_bspline_lines(double *coef, long long N, const double *w)
 {
-    static_assert(AXIS == 0 || AXIS == 1, "the z pass is k_bspline_zlines");
+    static_assert(AXIS == 0 || AXIS == 1, "the z pass is k_prims_zlines");
     const long long M = N + 2;
     const long long L = kNF * (AXIS == 1 ? N * M : M * M);
     const long long stride = (long long)gridDim.x * blockDim.x;
