@@ -34,6 +34,34 @@ __device__ __forceinline__ int field_of(const FieldDev *f, int n, long long it)
     return lo;
 }
 
+// The field of a warp's items in a flux kernel.  A warp's items ascend, so the
+// field is searched for once and then walked forward, its end kept in a
+// register: a search per interface is up to seven dependent loads, about 50
+// cycles each, that three warps per scheduler do not cover.  FP64 us per sweep
+// (x / y / z), 96 fields of 32^3, 48^3 and 64^3: 1397 / 1398 / 1495 -> 1287 / 1284 / 1322.
+struct FieldWalk {
+    const FieldDev *f;
+    long long end; // first item of the next field
+    int left;      // fields after this one
+    __device__ __forceinline__ FieldWalk(const Batch &b, long long it, bool ensemble = true)
+    {
+        if (!ensemble) return;
+        const int i = field_of(b.fields, b.nfields, it);
+        f = b.fields + i;
+        left = b.nfields - 1 - i;
+        end = left ? f[1].base : LLONG_MAX;
+    }
+    __device__ __forceinline__ const FieldDev &at(long long it)
+    {
+        while (it >= end) {
+            ++f;
+            --left;
+            end = left ? f[1].base : LLONG_MAX;
+        }
+        return *f;
+    }
+};
+
 struct Cell {
     int j, i, k, nc;
     int nyw;    // y-wrap modulus (FieldDev::nyw)
@@ -224,14 +252,20 @@ __device__ __forceinline__ void cp_async_wait()
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
-// Field of z line `it` (the last field whose line range starts at or before it).
-__device__ __forceinline__ int field_of_zline(const FieldDev *f, int n, long long it)
+// The last field whose range (FieldDev::*BASE) starts at or before item `it`, the
+// same item range for all 32 lanes: each round splits the fields left into 32
+// parts, a lane looking at the start of one, so up to 32 fields take one load's
+// latency and up to 1024 two (a binary search of 96 fields: seven).
+// FP64 us per sweep, 96 fields of 32^3: 148 / 131 / 174 -> 145 / 127 / 166.
+template <long long FieldDev::*BASE>
+__device__ __forceinline__ int field_of_warp(const FieldDev *f, int n, long long it)
 {
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (f[mid].zbase <= it) lo = mid;
-        else hi = mid - 1;
+    int lo = 0, hi = n;
+    while (hi - lo > 1) {
+        const int part = (hi - lo + 31) / 32, i = lo + int(threadIdx.x & 31) * part;
+        const unsigned below = __ballot_sync(0xffffffffu, i < hi && f[i < hi ? i : lo].*BASE <= it);
+        lo += (31 - __clz(below)) * part;
+        hi = min(lo + part, hi);
     }
     return lo;
 }
@@ -260,7 +294,7 @@ __global__ void __launch_bounds__(kReconBlock, MINB) k_recon_zline(Batch b)
     double (*tile)[kZLineCells] = tiles[wid];
     const long long stride = (long long)gridDim.x * kZLineWarps;
     for (long long it = b.lo + (long long)blockIdx.x * kZLineWarps + wid; it < b.hi; it += stride) {
-        const FieldDev &f = b.fields[field_of_zline(b.fields, b.nfields, it)];
+        const FieldDev &f = b.fields[field_of_warp<&FieldDev::zbase>(b.fields, b.nfields, it)];
         const int nc = f.nc;
         const unsigned lbase = unsigned(it - f.zbase) * unsigned(nc); // cell (j, i, 0)
         const bool direct = (f.flags & GKS_DIRECT_ENERGY) != 0;
@@ -340,18 +374,6 @@ __global__ void __launch_bounds__(kReconBlock, MINB) k_recon_zline(Batch b)
     }
 }
 
-// Field of window item `it` (the last field whose window range starts at or before it).
-__device__ __forceinline__ int field_of_win(const FieldDev *f, int n, long long it)
-{
-    int lo = 0, hi = n - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (f[mid].wbase <= it) lo = mid;
-        else hi = mid - 1;
-    }
-    return lo;
-}
-
 // ---------------------------------------------------------------------------
 // Reconstruction for the x (DIR 0) and y (DIR 1) sweeps with a sliding
 // window: a work item is a run of consecutive interfaces along the sweep at
@@ -384,7 +406,7 @@ __global__ void __launch_bounds__(kReconBlock, MINB) k_recon_win(Batch b)
     static_assert(DIR == 0 || DIR == 1, "windowed reconstruction is for the x and y sweeps");
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < b.hi; it += stride) {
-        const FieldDev &f = b.fields[field_of_win(b.fields, b.nfields, it)];
+        const FieldDev &f = b.fields[field_of_warp<&FieldDev::wbase>(b.fields, b.nfields, it)];
         const bool ranged = DIR == 1 && b.wy1 > 0;
         const long long loc = ranged ? it : it - f.wbase;
         if (!ranged && loc >= f.nwin) continue; // alignment padding after the field
@@ -794,52 +816,60 @@ __device__ __forceinline__ void flux_item(const FieldDev &f, unsigned c, FluxPar
 
 // A batch of one field reads the field's descriptor from the launch
 // parameters (b.one: constant-bank operands, nothing loaded per interface);
-// an ensemble looks each interface's field up in the device array.
+// an ensemble walks the device array (FieldWalk).
 //
 // Mixed: grid-stride loop.  FP64: one wave of resident blocks whose warps draw
 // chunks of 32 interfaces from a queue: the first is the warp's own number,
 // the next ones come from a counter in global memory, asked for one chunk
 // ahead.  (With equal static shares the schedulers run some warps ahead of
 // others and an SM's last fifth passes at falling occupancy: 9.7 of 12 warps
-// active on average, 11.8 with the queue; 1677 -> 1572 us per sweep at 256^3.
-// The mixed kernel gains nothing, 1466 -> 1515 us.)  The warp that is last to find the queue empty sets the counters
-// back to zero for the next launch.
+// active on average, 11.8 with the queue; 1677 -> 1572 us per sweep at 256^3,
+// 1548 with a loop of its own for one field and for an ensemble.  The mixed
+// kernel gains nothing, 1466 -> 1515 us.)  The warp that is last to find the
+// queue empty sets the counters back to zero for the next launch.
+template <int DIR, bool ENSEMBLE>
+__device__ __forceinline__ void flux_queue(const Batch &b, long long end, const SweepSrc64<DIR> &src)
+{
+    const int lane = threadIdx.x & 31;
+    const unsigned nwarps = gridDim.x * (kFluxBlock / 32);
+    const unsigned chunks = unsigned((end - b.lo + 31) >> 5);
+    unsigned *queue = b.queue + 2 * DIR;
+    unsigned chunk = (blockIdx.x * kFluxBlock + threadIdx.x) >> 5;
+    FieldWalk walk(b, b.lo + (long long)chunk * 32, ENSEMBLE);
+    while (chunk < chunks) {
+        unsigned next = 0;
+        if (lane == 0) next = nwarps + atomicAdd(queue, 1u);
+        const long long it = b.lo + (long long)chunk * 32 + lane;
+        double F[5];
+        if (!ENSEMBLE) {
+            if (it < end) {
+                flux_item64<DIR>(b.one, unsigned(it), src, Nothing(), F);
+                store_flux<DIR>(b.one, unsigned(it), F);
+            }
+        } else {
+            const FieldDev &f = walk.at(it);
+            if (it - f.base < f.ncell) { // else alignment padding after the field
+                flux_item64<DIR>(f, unsigned(it - f.base), src, Nothing(), F);
+                store_flux<DIR>(f, unsigned(it - f.base), F);
+            }
+        }
+        chunk = __shfl_sync(0xffffffffu, next, 0);
+    }
+    if (lane == 0 && atomicAdd(queue + 1, 1u) == nwarps - 1) {
+        queue[0] = 0;
+        queue[1] = 0;
+    }
+}
+
 template <int DIR, int PREC, int REGS>
 __global__ void __launch_bounds__(kFluxBlock) __maxnreg__(REGS) k_flux(Batch b)
 {
     __shared__ FluxPark<PREC> park;
     const long long end = b.nfields == 1 && b.one.ncell < b.hi ? b.one.ncell : b.hi; // alignment padding after the field
     if constexpr (PREC == 0) {
-        const int lane = threadIdx.x & 31;
-        const unsigned nwarps = gridDim.x * (kFluxBlock / 32);
-        const unsigned chunks = unsigned((end - b.lo + 31) >> 5);
-        unsigned *queue = b.queue + 2 * DIR;
         const SweepSrc64<DIR> src{park.slots};
-        unsigned chunk = (blockIdx.x * kFluxBlock + threadIdx.x) >> 5;
-        while (chunk < chunks) {
-            unsigned next = 0;
-            if (lane == 0) next = nwarps + atomicAdd(queue, 1u);
-            const long long it = b.lo + (long long)chunk * 32 + lane;
-            double F[5];
-            if (b.nfields == 1) {
-                if (it < end) {
-                    flux_item64<DIR>(b.one, unsigned(it), src, Nothing(), F);
-                    store_flux<DIR>(b.one, unsigned(it), F);
-                }
-            } else {
-                const FieldDev &f = b.fields[field_of(b.fields, b.nfields, it)];
-                if (it - f.base < f.ncell) { // else alignment padding after the field
-                    flux_item64<DIR>(f, unsigned(it - f.base), src, Nothing(), F);
-                    store_flux<DIR>(f, unsigned(it - f.base), F);
-                }
-            }
-            chunk = __shfl_sync(0xffffffffu, next, 0);
-        }
-        if (lane == 0 && atomicAdd(queue + 1, 1u) == nwarps - 1) {
-            queue[0] = 0;
-            queue[1] = 0;
-        }
-        return;
+        if (b.nfields == 1) flux_queue<DIR, false>(b, end, src);
+        else flux_queue<DIR, true>(b, end, src);
     } else {
         const long long stride = (long long)gridDim.x * blockDim.x;
         double F[5];
@@ -850,8 +880,9 @@ __global__ void __launch_bounds__(kFluxBlock) __maxnreg__(REGS) k_flux(Batch b)
             }
             return;
         }
-        for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < b.hi; it += stride) {
-            const FieldDev &f = b.fields[field_of(b.fields, b.nfields, it)];
+        long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x;
+        for (FieldWalk walk(b, it); it < b.hi; it += stride) {
+            const FieldDev &f = walk.at(it);
             if (it - f.base >= f.ncell) continue; // alignment padding after the field
             flux_item<DIR, true>(f, unsigned(it - f.base), park, F);
             store_flux<DIR>(f, unsigned(it - f.base), F);

@@ -606,3 +606,29 @@ def test_update_inside_the_z_flux_is_the_separate_update(gks, prec):
         with pytest.raises(gks.GksError) as ei:
             s.sync()
         assert ei.value.code == -5
+
+
+@pytest.mark.parametrize("nfields", [2, 32, 33, 100])
+def test_many_small_fields_equal_individual_runs(gks, nfields):
+    """Ensembles whose launches walk over several fields between two chunks of a
+    warp, and whose field searches take one round and two (above 32 fields)."""
+    cases = [gks_ic.make_dhit(n, k0=4.0, Mt=0.3, seed=n) for n in (10, 12, 13)]
+    Ws = [gks_ic.to_conservative_padded(c) for c in cases]
+    for prec in (gks.FP64, gks.MIXED):
+        alone = []
+        for c, W in zip(cases, Ws):
+            with gks.Solver(gks.phys_from_case(c), prec) as s:
+                s.upload(W)
+                s.set_dt(0.02)
+                s.step(2)
+                s.sync()
+                alone.append(s.download())
+        which = [f * f % 3 for f in range(nfields)]
+        with gks.Solver([gks.phys_from_case(cases[q]) for q in which], prec) as s:
+            for f, q in enumerate(which):
+                s.upload(Ws[q], f)
+                s.set_dt(0.02, f)
+            s.step(2)
+            s.sync()
+            for f, q in enumerate(which):
+                assert np.array_equal(s.download(f), alone[q])
