@@ -286,15 +286,14 @@ __device__ __forceinline__ int field_of_warp(const FieldDev *f, int n, long long
 // ---------------------------------------------------------------------------
 constexpr int kZLineWarps = kReconBlock / 32, kZLineCells = 32 + 6;
 
-template <int PREC, int MINB>
-__global__ void __launch_bounds__(kReconBlock, MINB) k_recon_zline(Batch b)
+template <int PREC, bool ENSEMBLE>
+__device__ __forceinline__ void recon_zlines(const Batch &b, double (&tiles)[kZLineWarps][5][kZLineCells])
 {
-    __shared__ double tiles[kZLineWarps][5][kZLineCells];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     double (*tile)[kZLineCells] = tiles[wid];
     const long long stride = (long long)gridDim.x * kZLineWarps;
     for (long long it = b.lo + (long long)blockIdx.x * kZLineWarps + wid; it < b.hi; it += stride) {
-        const FieldDev &f = b.fields[field_of_warp<&FieldDev::zbase>(b.fields, b.nfields, it)];
+        const FieldDev &f = ENSEMBLE ? b.fields[field_of_warp<&FieldDev::zbase>(b.fields, b.nfields, it)] : b.one;
         const int nc = f.nc;
         const unsigned lbase = unsigned(it - f.zbase) * unsigned(nc); // cell (j, i, 0)
         const bool direct = (f.flags & GKS_DIRECT_ENERGY) != 0;
@@ -374,6 +373,20 @@ __global__ void __launch_bounds__(kReconBlock, MINB) k_recon_zline(Batch b)
     }
 }
 
+// FP64 reads a one-field batch's descriptor from the launch parameters (x and y
+// windows and z lines): from memory, every asynchronous copy, a memory barrier
+// to the compiler, has the pointers and constants loaded again.  us per sweep at
+// 256^3, x / y / z: 625 / 554 / 607 -> 599 / 548 / 595; 130^3 111 / 97 / 109 -> 106 /
+// 96 / 105.  Mixed needs more registers with two loops in a kernel (120 -> 138; y
+// 454 -> 469, z 448 -> 457 us) and keeps one.
+template <int PREC, int MINB>
+__global__ void __launch_bounds__(kReconBlock, MINB) k_recon_zline(Batch b)
+{
+    __shared__ double tiles[kZLineWarps][5][kZLineCells];
+    if (PREC == 0 && b.nfields == 1) recon_zlines<PREC, false>(b, tiles);
+    else recon_zlines<PREC, true>(b, tiles);
+}
+
 // ---------------------------------------------------------------------------
 // Reconstruction for the x (DIR 0) and y (DIR 1) sweeps with a sliding
 // window: a work item is a run of consecutive interfaces along the sweep at
@@ -396,17 +409,16 @@ constexpr int kWinRing = 8;
 // p + 3 of the mixed one, besides them.
 __host__ __device__ constexpr int win_prefetch(int prec) { return prec == 0 ? 3 : 2; }
 
-template <int DIR, int PREC, int MINB>
-__global__ void __launch_bounds__(kReconBlock, MINB) k_recon_win(Batch b)
+template <int DIR, int PREC, bool ENSEMBLE>
+__device__ __forceinline__ void recon_runs(const Batch &b, double (&ring)[kWinRing][5][kReconBlock])
 {
     constexpr int PF = win_prefetch(PREC), NR = kWinRing;
     static_assert(NR >= (PREC == 0 ? 4 : 6) + PF && (NR & (NR - 1)) == 0, "the ring holds the live cells and those in flight");
-    __shared__ double ring[NR][5][kReconBlock];
     const int tid = threadIdx.x;
     static_assert(DIR == 0 || DIR == 1, "windowed reconstruction is for the x and y sweeps");
     const long long stride = (long long)gridDim.x * blockDim.x;
     for (long long it = b.lo + (long long)blockIdx.x * blockDim.x + threadIdx.x; it < b.hi; it += stride) {
-        const FieldDev &f = b.fields[field_of_warp<&FieldDev::wbase>(b.fields, b.nfields, it)];
+        const FieldDev &f = ENSEMBLE ? b.fields[field_of_warp<&FieldDev::wbase>(b.fields, b.nfields, it)] : b.one;
         const bool ranged = DIR == 1 && b.wy1 > 0;
         const long long loc = ranged ? it : it - f.wbase;
         if (!ranged && loc >= f.nwin) continue; // alignment padding after the field
@@ -541,6 +553,14 @@ __global__ void __launch_bounds__(kReconBlock, MINB) k_recon_win(Batch b)
         }
         cp_async_wait<0>(); // nothing in flight into the ring before the next item
     }
+}
+
+template <int DIR, int PREC, int MINB>
+__global__ void __launch_bounds__(kReconBlock, MINB) k_recon_win(Batch b)
+{
+    __shared__ double ring[kWinRing][5][kReconBlock];
+    if (PREC == 0 && b.nfields == 1) recon_runs<DIR, PREC, false>(b, ring);
+    else recon_runs<DIR, PREC, true>(b, ring);
 }
 
 // ---------------------------------------------------------------------------
