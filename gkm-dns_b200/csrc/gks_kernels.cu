@@ -1153,8 +1153,11 @@ __global__ void k_maxwave(FieldDev f, unsigned long long *out)
 // Two blocks fit an SM at 256^3, so that one's lines are solved while the
 // other's are moved.
 template <int AXIS, int LW> struct SplineTiles {
-    __host__ __device__ static int tile(int nt) { return AXIS == 2 ? LW * (nt | 1) : nt * LW; }
-    __host__ __device__ static size_t bytes(int nt) { return (3 * (size_t)tile(nt) + 2 * (size_t)nt) * sizeof(double); }
+    __host__ __device__ static constexpr int tile(int nt) { return AXIS == 2 ? LW * (nt | 1) : nt * LW; }
+    __host__ __device__ static constexpr size_t bytes(int nt)
+    {
+        return (3 * (size_t)tile(nt) + 2 * (size_t)nt) * sizeof(double);
+    }
 };
 constexpr int kSplineBlock = 256, kStage = 4; // threads; nodes a thread loads at a time
 
@@ -1597,11 +1600,17 @@ cudaError_t launch_maxwave(const FieldDev &f, unsigned long long *out_bits, int 
     return cudaGetLastError();
 }
 
+// Longest lines: of the 16-line form, and of all (nc = 1024).
+constexpr int kSplineNt16 = 288, kSplineNtMax = 1024 + 6;
+
 template <int AXIS, int LW>
 cudaError_t spline_go(const FieldDev &f, double *scratch, double *partial, double *kout, int max_grid, int *grid, cudaStream_t st)
 {
+    // the limit belongs to the function, which fields of other sizes launch from
+    // other threads: every call sets the same one, that of the longest lines
+    constexpr size_t limit = SplineTiles<AXIS, LW>::bytes(LW == 16 ? kSplineNt16 : kSplineNtMax);
     const size_t bytes = SplineTiles<AXIS, LW>::bytes(f.nc + 6);
-    cudaError_t e = cudaFuncSetAttribute(k_spline<AXIS, LW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaError_t e = cudaFuncSetAttribute(k_spline<AXIS, LW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
     if (e != cudaSuccess) return e;
     // lines: y lines (i, k) of the whole slab, x and z lines of the interior planes
     const int ny = f.yhi - f.ylo;
@@ -1617,7 +1626,7 @@ template <int AXIS>
 cudaError_t spline_axis(const FieldDev &f, double *scratch, double *partial, double *kout, int max_grid, int *grid,
                         cudaStream_t st)
 {
-    if (f.nc + 6 <= 288) return spline_go<AXIS, 16>(f, scratch, partial, kout, max_grid, grid, st);
+    if (f.nc + 6 <= kSplineNt16) return spline_go<AXIS, 16>(f, scratch, partial, kout, max_grid, grid, st);
     return spline_go<AXIS, 8>(f, scratch, partial, kout, max_grid, grid, st);
 }
 

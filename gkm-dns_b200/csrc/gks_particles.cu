@@ -416,7 +416,7 @@ __device__ __forceinline__ void bspline_smem(int N, double *c, const double *__r
 // thread t at row t / 5 and field t % 5 reads without bank conflicts), 30
 // threads run the recurrences, and the rows leave as contiguous runs.
 constexpr int kRowRows = 6, kRowThreads = 128;
-__host__ __device__ inline int row_pitch(int M) { return (kNF * M - kNF + 15) / 16 * 16 + kNF; }
+__host__ __device__ constexpr int row_pitch(int M) { return (kNF * M - kNF + 15) / 16 * 16 + kNF; }
 
 __global__ void __launch_bounds__(kRowThreads) k_prims_rows(FieldDev f, double *coef, const double *__restrict__ w)
 {
@@ -633,11 +633,10 @@ cudaError_t launch_particle_splines(const FieldDev &f, double *coef, const doubl
 {
     const long long nt = f.nc + 6, M = nt + 2;
     if (nt <= kLineShort) {
+        // within the 48 KB any kernel may have without asking for more
+        static_assert(kRowRows * row_pitch(kLineShort + 2) * sizeof(double) <= 49152 && kLineShort * 32 * sizeof(double) <= 49152,
+                      "shared memory of the short lines");
         const size_t rows = (size_t)kRowRows * row_pitch((int)M) * sizeof(double), cols = (size_t)nt * 32 * sizeof(double);
-        cudaError_t e = cudaFuncSetAttribute(k_prims_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rows);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line_cols<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols);
-        if (e == cudaSuccess) e = cudaFuncSetAttribute(k_line_cols<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)cols);
-        if (e != cudaSuccess) return e;
         k_prims_rows<<<(unsigned)((nt * nt + kRowRows - 1) / kRowRows), kRowThreads, rows, st>>>(f, coef, w);
         k_line_cols<1><<<(unsigned)((kNF * nt * M + 31) / 32), 32, cols, st>>>(coef, (int)nt, w);
         k_line_cols<0><<<(unsigned)((kNF * M * M + 31) / 32), 32, cols, st>>>(coef, (int)nt, w);
