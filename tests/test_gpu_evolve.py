@@ -144,3 +144,67 @@ def test_evolve_with_separate_component_arrays(gks):
         rc = gks.load_library().gks_evolve(s._h, 0, ptrs, 1)
         assert rc == 0
     assert np.array_equal(np.stack(comps), plain(gks, case, W0, gks.FP64, dt))
+
+
+def pinned(W):
+    import torch
+
+    host = torch.empty(W.shape, dtype=torch.float64, pin_memory=True).numpy()
+    host[...] = W
+    return host
+
+
+@pytest.mark.parametrize("nc", [56, 64, 104, 128])
+@pytest.mark.parametrize("variant", ["plain", "options", "mixed"])
+def test_slab_form_from_pinned_memory_equals_the_plain_sequence(gks, nc, variant):
+    """The slab-pipelined form with copies that really are asynchronous: its
+    smallest size, two and more slabs, a field above 2^20 cells (one
+    reconstruction buffer in gks_step, three here) and one whose resident steps
+    take the update inside the z flux, which then follow the swap of the state
+    buffers."""
+    prec = gks.MIXED if variant == "mixed" else gks.FP64
+    flags = gks.FIX_ZSWEEP | gks.DIRECT_ENERGY if variant == "options" else 0
+    case = gks_ic.make_dhit(nc, k0=4.0, Mt=0.5, seed=nc)
+    W0 = gks_ic.to_conservative_padded(case)
+    with gks.Solver(gks.phys_from_case(case), prec, flags) as s:
+        s.upload(W0)
+        dt = s.timestep(0.5)
+        host = pinned(W0)
+        ref = W0
+        for _ in range(2):
+            s.evolve(host)
+            ref = plain(gks, case, ref, prec, dt, flags=flags)
+            assert np.array_equal(host, ref)
+        s.step(2)
+        s.sync()
+        assert np.array_equal(s.download(), plain(gks, case, ref, prec, dt, 2, flags))
+
+
+@pytest.mark.parametrize("nc", [24, 64, 104])
+def test_host_step_on_components_in_separate_pieces(gks, nc):
+    """Five separate arrays, and one block page-locked in five pieces, which a
+    single copy over all of it refuses: one copy per component, in the one-piece
+    form and in the slab form."""
+    import ctypes
+
+    lib = gks.load_library()
+    case = gks_ic.make_dhit(nc, k0=4.0, Mt=0.4, seed=nc)
+    W0 = gks_ic.to_conservative_padded(case)
+    with gks.Solver(gks.phys_from_case(case)) as s:
+        s.upload(W0)
+        dt = s.timestep(0.5)
+        want = plain(gks, case, W0, gks.FP64, dt)
+        comps = [np.ascontiguousarray(W0[q]).copy() for q in range(5)]
+        assert lib.gks_evolve(s._h, 0, gks.DP5(*[c.ctypes.data_as(gks.DP) for c in comps]), 1) == 0
+        assert np.array_equal(np.stack(comps), want)
+        W = W0.copy()
+        ptrs = [ctypes.c_void_p(W[q].ctypes.data) for q in range(5)]
+        made = ctypes.c_int()
+        for p in ptrs:
+            assert lib.gks_host_register(p, W[0].nbytes, ctypes.byref(made)) == 0
+        try:
+            s.evolve(W)
+            assert np.array_equal(W, want)
+        finally:
+            for p in ptrs:
+                assert lib.gks_host_unregister(p) == 0
