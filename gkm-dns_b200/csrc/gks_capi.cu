@@ -957,8 +957,10 @@ int gks_upload(gks_ctx *ctx, int f, double *const W[5])
     for (int q = 0; q < 5; ++q)
         if (!W[q]) return fail(ctx, GKS_EINVAL, "null component pointer");
     CK(cudaSetDevice(ctx->device));
-    if ((rc = enqueue_upload(ctx, f, W))) return rc;
-    CK(cudaStreamSynchronize(ctx->stream));
+    rc = enqueue_upload(ctx, f, W);
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream); // after a failure too: no copy from W stays in flight
+    if (rc) return rc;
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamSynchronize(ctx->stream)");
     ctx->fh[f].uploaded = true;
     return GKS_OK;
 }
@@ -971,8 +973,10 @@ int gks_download(gks_ctx *ctx, int f, double *const W[5])
     for (int q = 0; q < 5; ++q)
         if (!W[q]) return fail(ctx, GKS_EINVAL, "null component pointer");
     CK(cudaSetDevice(ctx->device));
-    if ((rc = enqueue_download(ctx, f, W))) return rc;
-    CK(cudaStreamSynchronize(ctx->stream));
+    rc = enqueue_download(ctx, f, W);
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream); // after a failure too: no copy into W stays in flight
+    if (rc) return rc;
+    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaStreamSynchronize(ctx->stream)");
     return GKS_OK;
 }
 
@@ -991,14 +995,20 @@ int gks_evolve(gks_ctx *ctx, int f, double *const W[5], int nsteps)
     if (ctx->nfields == 1 && nsteps == 1 && ctx->fh[f].phys.nc >= kPipeMinNc && !ctx->fh[f].slab)
         return evolve_pipelined(ctx, W);
     // several fields or steps: upload, the captured steps, download, in stream order
-    if ((rc = enqueue_upload(ctx, f, W))) return rc;
+    const bool uploaded = ctx->fh[f].uploaded;
     ctx->fh[f].uploaded = true;
-    for (int g = 0; g < ctx->nfields; ++g)
-        if (!ctx->fh[g].uploaded) return fail(ctx, GKS_ESTATE, "evolve with field " + std::to_string(g) + " not uploaded");
-    if ((rc = gks_step(ctx, nsteps))) return rc;
-    if ((rc = enqueue_download(ctx, f, W))) return rc;
-    CK(cudaStreamSynchronize(ctx->stream));
-    return GKS_OK;
+    rc = enqueue_upload(ctx, f, W);
+    bool resident = rc == GKS_OK;
+    for (int g = 0; g < ctx->nfields && !rc; ++g)
+        if (!ctx->fh[g].uploaded) rc = fail(ctx, GKS_ESTATE, "evolve with field " + std::to_string(g) + " not uploaded");
+    if (!rc) rc = gks_step(ctx, nsteps);
+    if (!rc) rc = enqueue_download(ctx, f, W);
+    // a failure too returns when the copies from and to the caller's memory have ended
+    const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+    if (e != cudaSuccess) resident = false;
+    if (!resident) ctx->fh[f].uploaded = uploaded;
+    if (!rc && e != cudaSuccess) rc = cuda_fail(ctx, e, "cudaStreamSynchronize(ctx->stream)");
+    return rc;
 }
 
 int gks_host_register(void *p, size_t bytes, int *registered)

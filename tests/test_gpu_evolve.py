@@ -208,3 +208,34 @@ def test_host_step_on_components_in_separate_pieces(gks, nc):
         finally:
             for p in ptrs:
                 assert lib.gks_host_unregister(p) == 0
+
+
+@pytest.mark.parametrize("why", ["field", "dt"])
+def test_a_refused_host_step_leaves_no_copy_in_flight(gks, why):
+    """gks_evolve that fails after it has begun its upload (another field of the
+    ensemble not uploaded, or without its dt) has finished with the caller's
+    memory when it returns, and the field it was given is resident, as after
+    gks_upload."""
+    import torch
+
+    cases = [gks_ic.make_dhit(n, k0=4.0, Mt=0.4, seed=n) for n in (128, 12)]
+    Ws = [gks_ic.to_conservative_padded(c) for c in cases]
+    host = pinned(Ws[0])
+    with gks.Solver([gks.phys_from_case(c) for c in cases]) as s:
+        stream = torch.cuda.ExternalStream(s.stream())
+        s.upload(Ws[0])  # staging allocated: the call below only copies
+        dt = s.timestep(0.5)
+        if why == "dt":
+            s.upload(Ws[1], 1)
+        lib, ptrs = gks.load_library(), gks.DP5(*[host[q].ctypes.data_as(gks.DP) for q in range(5)])
+        stream.query()
+        rc = lib.gks_evolve(s._h, 0, ptrs, 1)
+        idle = stream.query()
+        assert rc == -4
+        assert idle
+        assert np.array_equal(s.download(), Ws[0])
+        s.upload(Ws[1], 1)
+        s.timestep(0.5, 1)
+        s.step(1)
+        s.sync()
+        assert np.array_equal(s.download(), plain(gks, cases[0], Ws[0], gks.FP64, dt))
