@@ -811,9 +811,6 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
         d.ksn = 2.0 * d.inv_dx;
         d.kst = 0.5 * d.inv_dx;
         d.hK2 = (p.K + 2) * 0.5;
-        d.igm1 = 1.0 / d.gm1;
-        d.shig = std::sqrt(d.hig);
-        d.rlg = 0.5 / (std::sqrt(pi) * d.shig);
         d.kA4 = p.pr_factor / (p.K + 3);
         d.prm1 = p.pr_factor - 1.0;
         const int kdi[5] = {p.K + 2, 2 * (p.K + 2), p.K + 3, p.K + 4, p.K + 5};

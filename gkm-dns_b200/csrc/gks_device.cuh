@@ -58,11 +58,13 @@ __device__ __forceinline__ f2 fmaxT(f2 a, f2 b) { return f2(fmaxf(a.v.x, b.v.x),
 template <typename T> __device__ __forceinline__ constexpr T cst(double x) { return T(x); }
 template <> __device__ __forceinline__ f2 cst<f2>(double x) { return f2(float(x)); }
 
-// 1/x from the hardware's approximation (rcp.approx.ftz.f64, good to about 20
-// bits) and one cubic step, y (1 + e + e^2) with e = 1 - x y: three fused
-// multiply-adds and no branch, within one unit in the last place for normal x
-// whose reciprocal is normal (__drcp_rn: twice the instructions and a
-// slow-path test).  x = 0, inf or NaN give NaN.
+// 1/x from the hardware's approximation y (rcp.approx.ftz.f64, good to about 20
+// bits) and one third-order step: with e = 1 - x y, 1/x = y / (1 - e), of whose
+// geometric series y (1 + e + e^2) is taken.  Three fused multiply-adds and no
+// branch; e^3 is below the rounding of the last, so nearly always correctly
+// rounded, and within one unit in the last place for 2^-1021 <= |x| < 2^1021
+// (__drcp_rn: twice the instructions and a slow-path test).  x = 0, inf or NaN
+// give NaN.
 __device__ __forceinline__ double rcp_cubic(double x)
 {
     double y;
@@ -71,9 +73,10 @@ __device__ __forceinline__ double rcp_cubic(double x)
     return fma(fma(e, e, e), y, y);
 }
 
-// 1/sqrt(x) likewise: rsqrt.approx.ftz.f64 and one cubic step
-// y (1 + e/2 + 3 e^2/8), e = 1 - x y^2, five FP64 instructions, within about one
-// unit in the last place for normal x > 0; x <= 0, inf or NaN give NaN.
+// 1/sqrt(x) likewise: rsqrt.approx.ftz.f64 and with e = 1 - x y^2 the binomial
+// series of y (1 - e)^(-1/2) to its second order, y (1 + e/2 + 3 e^2/8): five FP64
+// instructions, within one unit in the last place (half for the last rounding,
+// half for that of x y) for 2^-1021 <= x < 2^1021; x <= 0, inf or NaN give NaN.
 __device__ __forceinline__ double rsqrt_cubic(double x)
 {
     double y;
@@ -321,8 +324,7 @@ struct FluxConst {
 // And the FP64 path's (gks_flux64.cuh).
 struct FluxConst64 {
     double dt;
-    double gm1, igm1;            // gamma - 1 and its reciprocal
-    double shig, rlg;            // sqrt(1 / (2 (gamma - 1))), 1 / (2 sqrt(pi) shig)
+    double gm1;                  // gamma - 1
     double ksn, kst;             // slope scales: 2/dx (normal), 1/(2 dx) (transverse)
     double kA4;                  // pr_factor / (K + 3)
     double prm1;                 // pr_factor - 1

@@ -45,36 +45,39 @@ namespace gks {
 // One Maxwellian: state, frame and derived constants.
 struct Gauss {
     double den, rinv, U0, U1, U2;
-    double s;        // variance 1 / (2 lambda)
+    double p, s;     // pressure, variance 1 / (2 lambda)
     double tl;       // 2 lambda
     double kh;       // kA lambda^2
     double k3, k5;   // (K+3) s, (K+5) s
     double x, e2, g; // sqrt(lambda) U0, exp(-x^2), exp(-x^2) / (2 sqrt(pi lambda))
 };
 
-// From the conserved state, with one reciprocal square root: A = rho2p(W),
-// z = 1 / (rho sqrt(A)) gives 1/sqrt(A) = rho z and sqrt(A)/rho = A z, of which
-// 1/rho, s = (gamma - 1) A / rho^2, 2 lambda = 1/s and sqrt(lambda) are products.
+// From the conserved state.  The pressure, whose rounding is most of the error of
+// a slow flow's momentum, is taken with as few roundings as there are: one of
+// rho E - rho U^2 / 2 and one of its product with gamma - 1 (the kinetic part is
+// the smaller one), and goes into the flux as it is.  2 lambda = 1/s and
+// sqrt(lambda) are products of one reciprocal square root y of s = p / rho.
+// Error of the momenta after a step against 64-bit mantissas, rms relative to
+// their largest value, ten fields of 16^3 to 33^3: 3.9e-17; p and 1/rho as products
+// of 1 / (rho sqrt(rho2p(W))): 7.0e-17; the reference's order in double: 5.5e-17.
 __device__ __forceinline__ Gauss gauss(const double W[5], const FluxConst64 &c)
 {
     Gauss m;
     m.den = W[0];
-    const double A = rho2p(W);
-    const double z = rsqrt_cubic(W[0] * (W[0] * A));
-    const double ra = W[0] * z, az = A * z;
-    const double t = W[0] * ra;
-    m.rinv = az * ra;
+    m.rinv = rcp_cubic(W[0]);
     m.U0 = W[1] * m.rinv;
     m.U1 = W[2] * m.rinv;
     m.U2 = W[3] * m.rinv;
-    m.s = (c.gm1 * az) * az;
-    m.tl = (c.igm1 * t) * t;
+    m.p = c.gm1 * fma(-0.5, fma(W[1], m.U0, fma(W[2], m.U1, W[3] * m.U2)), W[4]);
+    m.s = m.p * m.rinv;
+    const double y = rsqrt_cubic(m.s);
+    m.tl = y * y;
     m.kh = (c.kA4 * m.tl) * m.tl;
     m.k3 = c.K3 * m.s;
     m.k5 = c.K5 * m.s;
-    m.x = (c.shig * t) * m.U0;
+    m.x = (0.7071067811865476 * y) * m.U0;
     m.e2 = exp(-m.x * m.x);
-    m.g = (c.rlg * az) * m.e2;
+    m.g = (0.3989422804014327 * (m.s * y)) * m.e2;
     return m;
 }
 
@@ -147,11 +150,12 @@ __device__ __forceinline__ void flux_side(const Src &src, const FluxConst64 &c)
     const double c4 = 0.5 * (r2 + hu);
     {
         const double d0 = m.den * X[0];
-        src.template sum<SIDE>(Src::kW0 + 0, d0);
-        src.template sum<SIDE>(Src::kW0 + 1, m.den * X[1]);
-        src.template sum<SIDE>(Src::kW0 + 2, U1 * d0);
-        src.template sum<SIDE>(Src::kW0 + 3, U2 * d0);
-        src.template sum<SIDE>(Src::kW0 + 4, fma(0.5 * m.den, X[2], c4 * d0));
+        src.template sum<SIDE>(Src::kW0 + 0, m.den, X[0]);
+        src.template sum<SIDE>(Src::kW0 + 1, m.den, X[1]);
+        src.template sum<SIDE>(Src::kW0 + 2, U1, d0);
+        src.template sum<SIDE>(Src::kW0 + 3, U2, d0);
+        src.template sum<SIDE>(Src::kW0 + 4, c4, d0);
+        src.template sum<1>(Src::kW0 + 4, 0.5 * m.den, X[2]);
     }
     const double hU = 0.5 * fma(U0, U0, hu);
     double ax[5], ayz[5], vx, vy, vz, Dt, e0, e1, e2, f0, f1, f2;
@@ -411,12 +415,12 @@ __device__ __forceinline__ void gks_flux64(const Src &src, double tau_n, double 
         const double g2 = fma(p2, h2[2], f2);
         const double g3 = fma(p2, h2[3], f3);
         const double g4 = fma(p2, h2[4], fma(U0, fma(0.5 * U0, f0, f1), f4));
-        const double w0 = p0 * U0, P = p0 * (m.den * s);
+        const double w0 = p0 * U0;
         F[0] = fma(w0, We[0], fma(m.den, g0, src.get(Src::kF + 0)));
-        F[1] = fma(w0, We[1], fma(m.den, g1, src.get(Src::kF + 1))) + P;
+        F[1] = fma(p0, m.p, fma(w0, We[1], fma(m.den, g1, src.get(Src::kF + 1))));
         F[2] = fma(w0, We[2], fma(m.den, fma(U1, g0, g2), src.get(Src::kF + 2)));
         F[3] = fma(w0, We[3], fma(m.den, fma(U2, g0, g3), src.get(Src::kF + 3)));
-        F[4] = fma(w0, We[4], fma(m.den, fma(U1, g2, fma(U2, g3, fma(0.5 * hu, g0, g4))), src.get(Src::kF + 4))) + P * U0;
+        F[4] = fma(w0, We[4] + m.p, fma(m.den, fma(U1, g2, fma(U2, g3, fma(0.5 * hu, g0, g4))), src.get(Src::kF + 4)));
     }
 }
 

@@ -686,6 +686,10 @@ template <int DIR> struct SweepSrc64 {
         }
     }
     template <int SIDE> __device__ __forceinline__ void sum(int i, double v) const { at(i) = SIDE ? at(i) + v : v; }
+    template <int SIDE> __device__ __forceinline__ void sum(int i, double a, double b) const
+    {
+        at(i) = SIDE ? fma(a, b, at(i)) : a * b;
+    }
     __device__ __forceinline__ double get(int i) const { return at(i); }
     __device__ __forceinline__ void put(int i, double v) const { at(i) = v; }
 };
@@ -801,8 +805,7 @@ __device__ __forceinline__ void flux_item64(const FieldDev &f, unsigned c, const
     // collision time mu / p at the left cell (update.cpp:262-264), stored by
     // this step's x-sweep reconstruction
     const double tau_n = __ldg(f.tau[0] + c), tau_d = __ldg(f.tau[1] + c);
-    const FluxConst64 fc = {f.dt,  f.gm1,  f.igm1,  f.shig,  f.rlg,   f.ksn,   f.kst,
-                            f.kA4, f.prm1, f.kd[0], f.kd[1], f.kd[2], f.kd[3], f.kd[4]};
+    const FluxConst64 fc = {f.dt, f.gm1, f.ksn, f.kst, f.kA4, f.prm1, f.kd[0], f.kd[1], f.kd[2], f.kd[3], f.kd[4]};
     gks_flux64(src, tau_n, tau_d, fc, ahead, F);
     unrotate<DIR>(F);
 }

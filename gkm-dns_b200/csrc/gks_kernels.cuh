@@ -56,10 +56,10 @@ struct FieldDev {
     double spl_s;     // 3/h of the spline grid along x and z
     double spl_sy;    // along y (a slab's grid starts at its own first plane)
     // flux constants computed once on the host (no per-interface conversions
-    // or products): 1/(2 (gam-1)), 1/(gam-1), sqrt(hig), 1/(2 sqrt(pi) shig), slope
-    // scales 2/dx and 1/(2 dx), (K+2)/2, kA/4 and pr_factor - 1; K + 2, 2 (K+2),
-    // K + 3, K + 4, K + 5 in double; K + 2, K + 4, (K+2)(K+4), -(K+3) in float
-    double hig, igm1, shig, rlg, ksn, kst, hK2, kA4, prm1;
+    // or products): 1/(2 (gam-1)), slope scales 2/dx and 1/(2 dx), (K+2)/2, kA/4 and
+    // pr_factor - 1; K + 2, 2 (K+2), K + 3, K + 4, K + 5 in double; K + 2, K + 4,
+    // (K+2)(K+4), -(K+3) in float
+    double hig, ksn, kst, hK2, kA4, prm1;
     double kd[5];
     float kf[4];
 };
