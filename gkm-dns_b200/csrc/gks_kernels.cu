@@ -1153,15 +1153,7 @@ __global__ void k_maxwave(FieldDev f, unsigned long long *out)
 //               group of LW threads one contiguous run of LW doubles;
 //   z lines:    LW consecutive (j, i) lines:      tiles [line][node], the
 //               pitch odd so that the lines' threads use distinct banks.
-// Two blocks fit an SM at 256^3, so that one's lines are solved while the
-// other's are moved.
-template <int AXIS, int LW> struct SplineTiles {
-    __host__ __device__ static constexpr int tile(int nt) { return AXIS == 2 ? LW * (nt | 1) : nt * LW; }
-    __host__ __device__ static constexpr size_t bytes(int nt)
-    {
-        return (3 * (size_t)tile(nt) + 2 * (size_t)nt) * sizeof(double);
-    }
-};
+// LW is chosen so that two blocks fit an SM (spline_lines).
 constexpr int kSplineBlock = 256, kStage = 4; // threads; nodes a thread loads at a time
 
 // The line f_p at c[p S], p = 0 .. nt-1, replaced by its slopes.  Nodes move in
@@ -1221,6 +1213,8 @@ template <int S> __device__ __forceinline__ void spline_slopes(double *c, int nt
 }
 
 constexpr int NSUM1 = kStatsSums;
+static_assert(NSUM1 * (kSplineBlock / 32) * sizeof(double) <= spline_bytes(2, 8, 10),
+              "the block sums fit the tiles of the shortest lines");
 
 __device__ __forceinline__ double warp_sum(double v)
 {
@@ -1229,20 +1223,20 @@ __device__ __forceinline__ double warp_sum(double v)
     return v;
 }
 
+// sm: N doubles per warp of shared memory that nothing else uses any more.
 template <int N>
-__device__ __forceinline__ void block_sums(double (&v)[N], double *out)
+__device__ __forceinline__ void block_sums(double (&v)[N], double *sm, double *out)
 {
-    __shared__ double sm[N][32];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
         const double x = warp_sum(v[i]);
-        if (lane == 0) sm[i][wid] = x;
+        if (lane == 0) sm[i * nw + wid] = x;
     }
     __syncthreads();
     if (threadIdx.x < N) {
         double t = 0.0;
-        for (int w = 0; w < nw; ++w) t += sm[threadIdx.x][w];
+        for (int w = 0; w < nw; ++w) t += sm[threadIdx.x * nw + w];
         out[threadIdx.x] = t;
     }
 }
@@ -1311,7 +1305,6 @@ __device__ __forceinline__ void add_sums(const FieldDev &f, long long c, const d
 template <int AXIS, int LW>
 __global__ void __launch_bounds__(kSplineBlock, 2) k_spline(FieldDev f, double *scr, int nsets, double *partial, double *kout)
 {
-    using ST = SplineTiles<AXIS, LW>;
     constexpr bool SUMS = AXIS == 2;
     constexpr int NG = kSplineBlock / LW;    // y / x: threads on one line
     constexpr int NW = kSplineBlock / 32;    // z: warps
@@ -1321,7 +1314,7 @@ __global__ void __launch_bounds__(kSplineBlock, 2) k_spline(FieldDev f, double *
     const int nc = f.nc, nt = AXIS == 0 ? f.ny + 2 * f.yhost : nc + 6;
     const long long n = f.ncell;
     const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    const int tsz = ST::tile(nt), pitch = nt | 1;
+    const int pitch = nt | 1, tsz = AXIS == 2 ? LW * pitch : nt * LW;
     double *cpv = smem + 3 * tsz, *invv = cpv + nt;
     // tile of velocity component a, node, line
     auto T = [&](int a, int node, int line) -> double & {
@@ -1414,7 +1407,7 @@ __global__ void __launch_bounds__(kSplineBlock, 2) k_spline(FieldDev f, double *
         }
         __syncthreads();
     }
-    if constexpr (SUMS) block_sums<NSUM1>(acc, partial + (long long)blockIdx.x * NSUM1);
+    if constexpr (SUMS) block_sums<NSUM1>(acc, smem, partial + (long long)blockIdx.x * NSUM1);
 }
 
 // Sum the per-block partials, one warp per quantity, in a fixed order (so the
@@ -1603,16 +1596,13 @@ cudaError_t launch_maxwave(const FieldDev &f, unsigned long long *out_bits, int 
     return cudaGetLastError();
 }
 
-// Longest lines: of the 16-line form, and of all (nc = 1024).
-constexpr int kSplineNt16 = 288, kSplineNtMax = 1024 + 6;
-
 template <int AXIS, int LW>
 cudaError_t spline_go(const FieldDev &f, double *scratch, double *partial, double *kout, int max_grid, int *grid, cudaStream_t st)
 {
     // the limit belongs to the function, which fields of other sizes launch from
     // other threads: every call sets the same one, that of the longest lines
-    constexpr size_t limit = SplineTiles<AXIS, LW>::bytes(LW == 16 ? kSplineNt16 : kSplineNtMax);
-    const size_t bytes = SplineTiles<AXIS, LW>::bytes(f.nc + 6);
+    constexpr size_t limit = LW == 16 ? kSmemPerSm / 2 - kSmemPerBlock : spline_bytes(AXIS, LW, kSplineNtMax);
+    const size_t bytes = spline_bytes(AXIS, LW, f.nc + 6);
     cudaError_t e = cudaFuncSetAttribute(k_spline<AXIS, LW>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)limit);
     if (e != cudaSuccess) return e;
     // lines: y lines (i, k) of the whole slab, x and z lines of the interior planes
@@ -1623,13 +1613,11 @@ cudaError_t spline_go(const FieldDev &f, double *scratch, double *partial, doubl
     return cudaGetLastError();
 }
 
-// Lines per block: 16 (128 contiguous bytes per row of a y / x tile) up to nt =
-// 288, 8 beyond, so that two blocks fit an SM's shared memory up to nt = 576.
 template <int AXIS>
 cudaError_t spline_axis(const FieldDev &f, double *scratch, double *partial, double *kout, int max_grid, int *grid,
                         cudaStream_t st)
 {
-    if (f.nc + 6 <= kSplineNt16) return spline_go<AXIS, 16>(f, scratch, partial, kout, max_grid, grid, st);
+    if (spline_lines(AXIS, f.nc + 6) == 16) return spline_go<AXIS, 16>(f, scratch, partial, kout, max_grid, grid, st);
     return spline_go<AXIS, 8>(f, scratch, partial, kout, max_grid, grid, st);
 }
 

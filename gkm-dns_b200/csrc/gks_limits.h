@@ -8,7 +8,7 @@
 
 namespace gks {
 
-// Sums the statistics reduction keeps per block (k_sums1).
+// Sums the statistics reduction keeps per block (k_spline's z pass).
 constexpr int kStatsSums = 24;
 // Blocks per SM of the grid-stride helper kernels (gather, scatter, maxwave,
 // check) and of the statistics reduction.
@@ -39,6 +39,31 @@ inline int stats_grid(long long ncell, int block, int nsm)
 inline size_t stats_partial_elems(int nsm)
 {
     return (size_t)(nsm > 0 ? nsm : 1) * kStatsBlocksPerSm * kStatsSums;
+}
+
+// Shared memory of an SM, and what each resident block takes of it besides its own.
+constexpr size_t kSmemPerSm = 233472, kSmemPerBlock = 1024;
+
+// Longest spline line (nc = 1024).
+constexpr int kSplineNtMax = 1024 + 6;
+
+// Shared memory of a block of the statistics' spline passes that holds `lines`
+// lines of nt nodes: three tiles of velocity components (the z pass's pitch is
+// odd) and the two pivot arrays.
+constexpr size_t spline_bytes(int axis, int lines, int nt)
+{
+    return (3 * (size_t)lines * (axis == 2 ? nt | 1 : nt) + 2 * (size_t)nt) * sizeof(double);
+}
+
+// Lines per block: 16 (128 contiguous bytes per row of a y / x tile) where two
+// such blocks fit an SM, so that one's lines are solved while the other's are
+// moved: up to nt = 289; else 8, of which two fit up to nt = 555 (y, x: 556).
+// gks_stats, ps per cell, where a block of the z pass had an SM to itself for its
+// lines / as here: 270^3 90.7 / 75.1, 282^3 91.0 / 75.6, 520^3 106.6 / 85.8, 540^3 109.0 /
+// 88.5 (256^3: 65; 558^3, one block: 123).
+constexpr int spline_lines(int axis, int nt)
+{
+    return 2 * (spline_bytes(axis, 16, nt) + kSmemPerBlock) <= kSmemPerSm ? 16 : 8;
 }
 
 // Device address of a file-scope __device__ array, cached per device and

@@ -632,3 +632,28 @@ def test_many_small_fields_equal_individual_runs(gks, nfields):
             s.sync()
             for f, q in enumerate(which):
                 assert np.array_equal(s.download(f), alone[q])
+
+
+@pytest.mark.parametrize("nc", [275, 283])
+def test_stats_cost_per_cell_has_no_step_at_longer_lines(gks, nc):
+    """Lines a little longer than 256^3's still leave two blocks of every pass on
+    an SM; with one, a cell costs 1.4 times as much."""
+    import time
+
+    def ns_per_cell(n):
+        case = gks_ic.make_dhit(8, k0=2.0, Mt=0.3, seed=1)
+        phys = gks.phys_from_case(case)
+        phys.nc = n
+        W = np.zeros((5,) + (n + 6,) * 3)
+        W[0] = 1.0
+        W[4] = 2.0
+        with gks.Solver(phys) as s:
+            s.upload(W)
+            best = np.inf
+            for _ in range(8):
+                t = time.perf_counter()
+                s.stats_part()
+                best = min(best, time.perf_counter() - t)
+        return best / n**3
+
+    assert ns_per_cell(nc) < 1.2 * ns_per_cell(256)
