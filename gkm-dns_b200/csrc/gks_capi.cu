@@ -210,18 +210,25 @@ gks::LaunchCfg persistent(gks_ctx *ctx, int kind, int dir, int variant, int mult
     return c;
 }
 
-// Untuned defaults: the flux at the 168-register cap (6 blocks of 64 threads
-// per SM), one wave of blocks; the reconstruction with all its blocks launched
-// (a wave of persistent blocks ends unevenly: 256^3 x / y / z, FP64 694 / 627 /
-// 680 -> 670 / 601 / 634 us, mixed 533 / 511 / 501 -> 502 / 465 / 458), at its
-// natural register count but for the FP64 z sweep, which the 96-register cap
-// (20 warps per SM, 40 B spill) serves best (663 at 150 registers).
+// The untuned grid of a variant: the flux and the update one wave of blocks, the
+// reconstruction all its blocks (a wave of persistent blocks ends unevenly: 256^3
+// x / y / z, FP64 694 / 627 / 680 -> 670 / 601 / 634 us when this was chosen, mixed 533 /
+// 511 / 501 -> 502 / 465 / 458).
+gks::LaunchCfg default_launch(gks_ctx *ctx, int kind, int dir, int variant)
+{
+    return persistent(ctx, kind, dir, variant, kind == gks::K_RECON ? 0 : 1);
+}
+
+// Untuned defaults: the flux at the 168-register cap (6 blocks of 64 threads per
+// SM), the reconstruction at its natural register count but for the FP64 z sweep,
+// which the 96-register cap (20 warps per SM, 40 B spill) serves best (663 us at
+// 150 registers against 634).
 void choose_launch(gks_ctx *ctx)
 {
     for (int kind = 0; kind < gks::K_KINDS; ++kind)
         for (int dir = 0; dir < 3; ++dir) {
             const int variant = kind == gks::K_FLUX ? 1 : (kind == gks::K_RECON && dir == 2 && ctx->precision == GKS_FP64 ? 2 : 0);
-            ctx->cfg[kind][dir] = persistent(ctx, kind, dir, variant, kind == gks::K_RECON ? 0 : 1);
+            ctx->cfg[kind][dir] = default_launch(ctx, kind, dir, variant);
         }
 }
 
@@ -1549,7 +1556,7 @@ int gks_set_launch(gks_ctx *ctx, int kind, int dir, int grid, int variant)
     if (variant < 0 || variant >= nvar) return fail(ctx, GKS_EINVAL, "no such kernel variant");
     if (grid < 0) return fail(ctx, GKS_EINVAL, "negative grid");
     CK(cudaSetDevice(ctx->device));
-    gks::LaunchCfg c = persistent(ctx, kind, dir, variant, 1);
+    gks::LaunchCfg c = default_launch(ctx, kind, dir, variant);
     if (grid > 0) c.grid = grid;
     ctx->cfg[kind][dir] = c;
     drop_graph(ctx);

@@ -383,7 +383,7 @@ class Solver:
 
     def set_launch(self, kind: str, d: int, variant: int, grid: int = 0):
         """Pin kernel `kind` ("recon", "flux", "update") of sweep d (0, 1, 2) to a
-        register-cap variant and grid (0: one wave of resident blocks)."""
+        register-cap variant and grid (0: the untuned grid of that variant)."""
         k = ("recon", "flux", "update").index(kind)
         self._ck(self._lib.gks_set_launch(self._h, k, d, grid, variant))
 

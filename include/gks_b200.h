@@ -244,8 +244,10 @@ int gks_get_launch(gks_ctx *ctx, int kind, int dir, int *block, int *grid, int *
 /* Pin the launch configuration of one kernel kind and sweep (for example to
  * restore a tuning saved by a previous run): `variant` indexes the kind's
  * register-cap variants (gks_get_launch reports the one in use), `grid` is the
- * number of blocks of the persistent grid-stride launch, 0 for one wave of
- * resident blocks.  Results do not depend on the configuration. */
+ * number of blocks of the launch (a grid-stride loop), 0 for what an untuned
+ * context launches of that variant: one wave of resident blocks, or, for the
+ * reconstruction, as many as the work needs.  Results do not depend on the
+ * configuration. */
 int gks_set_launch(gks_ctx *ctx, int kind, int dir, int grid, int variant);
 
 /* Peak FMA throughput of the FP64 (GKS_FP64) or FP32 (GKS_MIXED) pipe of

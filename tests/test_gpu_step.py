@@ -657,3 +657,15 @@ def test_stats_cost_per_cell_has_no_step_at_longer_lines(gks, nc):
         return best / n**3
 
     assert ns_per_cell(nc) < 1.2 * ns_per_cell(256)
+
+
+def test_grid_zero_pins_the_default_grid(gks):
+    """gks_set_launch with grid 0 and the default variant is the default launch."""
+    case = gks_ic.make_dhit(128, k0=4.0, Mt=0.3, seed=1)
+    for prec in (gks.FP64, gks.MIXED):
+        with gks.Solver(gks.phys_from_case(case), prec) as s:
+            before = s.launch_config()
+            for kind in ("recon", "flux", "update"):
+                for d in range(3):
+                    s.set_launch(kind, d, before[f"{kind}_{'xyz'[d]}"]["variant"])
+            assert s.launch_config() == before
