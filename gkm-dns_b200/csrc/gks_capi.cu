@@ -313,6 +313,9 @@ int record_step(gks_ctx *ctx)
 // dt (a caller that takes one every step) asks for it again.
 constexpr int kDirectSteps = 16;
 
+// A stream on which no step can be captured: the legacy default stream.
+bool uncapturable(const gks_ctx *ctx) { return ctx->stream == cudaStreamLegacy; }
+
 int build_graph(gks_ctx *ctx)
 {
     drop_graph(ctx);
@@ -901,6 +904,23 @@ int enqueue_download(gks_ctx *ctx, int f, double *const W[5])
     return copy_padded(ctx, f, W, cudaMemcpyDeviceToHost);
 }
 
+int run_steps(gks_ctx *ctx, int nsteps)
+{
+    for (int s = 0; s < nsteps; ++s) {
+        if (!ctx->graph) {
+            const bool direct = ctx->direct < kDirectSteps || uncapturable(ctx);
+            const int rc = direct ? record_step(ctx) : build_graph(ctx);
+            if (rc) return rc;
+            if (direct) {
+                ++ctx->direct;
+                continue;
+            }
+        }
+        CK(cudaGraphLaunch(ctx->graph, ctx->stream));
+    }
+    return GKS_OK;
+}
+
 } // namespace
 
 extern "C" {
@@ -1005,7 +1025,8 @@ int gks_evolve(gks_ctx *ctx, int f, double *const W[5], int nsteps)
     bool resident = rc == GKS_OK;
     for (int g = 0; g < ctx->nfields && !rc; ++g)
         if (!ctx->fh[g].uploaded) rc = fail(ctx, GKS_ESTATE, "evolve with field " + std::to_string(g) + " not uploaded");
-    if (!rc) rc = gks_step(ctx, nsteps);
+    // one field, one step: as the pipelined form, on any stream
+    if (!rc) rc = ctx->nfields == 1 && nsteps == 1 && !ctx->fh[f].slab && uncapturable(ctx) ? run_steps(ctx, 1) : gks_step(ctx, nsteps);
     if (!rc) rc = enqueue_download(ctx, f, W);
     // a failure too returns when the copies from and to the caller's memory have ended
     const cudaError_t e = cudaStreamSynchronize(ctx->stream);
@@ -1082,19 +1103,14 @@ int gks_step(gks_ctx *ctx, int nsteps)
         if (!ctx->fh[f].have_dt) return fail(ctx, GKS_ESTATE, "step before dt of field " + std::to_string(f));
     }
     CK(cudaSetDevice(ctx->device));
-    for (int s = 0; s < nsteps; ++s) {
-        if (!ctx->graph) {
-            const bool direct = ctx->direct < kDirectSteps;
-            const int rc = direct ? record_step(ctx) : build_graph(ctx);
-            if (rc) return rc;
-            if (direct) {
-                ++ctx->direct;
-                continue;
-            }
-        }
-        CK(cudaGraphLaunch(ctx->graph, ctx->stream));
-    }
-    return GKS_OK;
+    // steps are refused from the first on where a later one could not be captured,
+    // or would have to launch its graph into the caller's: they hold this moment's
+    // dt and state buffers
+    if (uncapturable(ctx)) return fail(ctx, GKS_ECUDA, "gks_step on the legacy default stream, which cannot be captured");
+    cudaStreamCaptureStatus capturing;
+    CK(cudaStreamIsCapturing(ctx->stream, &capturing));
+    if (capturing != cudaStreamCaptureStatusNone) return fail(ctx, GKS_ECUDA, "gks_step on a stream that is being captured");
+    return run_steps(ctx, nsteps);
 }
 
 int gks_sync(gks_ctx *ctx)

@@ -145,7 +145,8 @@ int gks_set_dt(gks_ctx *ctx, int f, double dt);
  * (evolveEulerian, update.cpp:194-199): three fused reconstruction + flux
  * sweeps and the conservative update per step; the first few are launched
  * kernel by kernel, then a step is captured as a CUDA graph.  Asynchronous on
- * the context's stream. */
+ * the context's stream.  GKS_ECUDA on a stream that is being captured and on
+ * the legacy default stream (gks_set_stream with cudaStreamLegacy). */
 int gks_step(gks_ctx *ctx, int nsteps);
 
 /* Diagnostics of field f on the current state (synchronises). */

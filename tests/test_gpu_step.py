@@ -669,3 +669,58 @@ def test_grid_zero_pins_the_default_grid(gks):
                 for d in range(3):
                     s.set_launch(kind, d, before[f"{kind}_{'xyz'[d]}"]["variant"])
             assert s.launch_config() == before
+
+
+@pytest.mark.parametrize("steps_before", [0, 20])
+def test_step_is_refused_on_a_stream_being_captured(gks, steps_before):
+    """gks_step into a caller's capture is an error, before a step's own graph
+    exists as well as after; nothing of it enters the caller's graph."""
+    import torch
+
+    case = gks_ic.make_dhit(24, k0=4.0, Mt=0.3, seed=1)
+    W = gks_ic.to_conservative_padded(case)
+    stream, x = torch.cuda.Stream(), torch.zeros(8, device="cuda")
+    with gks.Solver(gks.phys_from_case(case)) as s:
+        s.set_stream(stream.cuda_stream)
+        s.upload(W)
+        s.timestep(0.5)
+        s.step(steps_before)
+        s.sync()
+        before = s.download()
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=stream):
+            x.add_(1.0)
+            with pytest.raises(gks.GksError) as ei:
+                s.step(1)
+        assert ei.value.code == -2
+        graph.replay()
+        torch.cuda.synchronize()
+        assert float(x.sum()) == 8.0
+        assert np.array_equal(s.download(), before)
+        s.step(1)  # outside the capture as ever
+        s.sync()
+        assert not np.array_equal(s.download(), before)
+
+
+def test_step_is_refused_on_the_legacy_stream_and_the_host_step_is_not(gks):
+    """A step cannot be captured on the legacy default stream: gks_step refuses it
+    from the first step on; the one-field host step runs there, whether in one
+    piece or in slabs."""
+    for nc in (20, 60):
+        case = gks_ic.make_dhit(nc, k0=4.0, Mt=0.3, seed=1)
+        W = gks_ic.to_conservative_padded(case)
+        out = []
+        for legacy in (False, True):
+            with gks.Solver(gks.phys_from_case(case)) as s:
+                s.upload(W)
+                s.timestep(0.5)
+                if legacy:
+                    s.set_stream(1)  # cudaStreamLegacy
+                    with pytest.raises(gks.GksError) as ei:
+                        s.step(1)
+                    assert ei.value.code == -2
+                host = W.copy()
+                for _ in range(18):
+                    s.evolve(host)
+                out.append(host)
+        assert np.array_equal(out[0], out[1])
