@@ -188,6 +188,17 @@ int read_err(gks_ctx *ctx, int *word, bool clear)
     return GKS_OK;
 }
 
+// Whether the step's z flux applies the update itself (k_flux_update): one field
+// whose sweeps run one after the other (with concurrent sweeps the x and y fluxes
+// still read the state) and whose z lines fill the warps' 32 lanes (at 250^3,
+// where 2.4 % of them idle, nothing is left of the gain).  us per step,
+// separate / with the flux, runs in turn: FP64 128^3 989 / 971, 256^3 7596 / 7469;
+// mixed 128^3 858 / 845, 256^3 6741 / 6605, 320^3 13265 / 12947, 512^3 55859 / 54205.
+bool update_with_flux(const gks_ctx *ctx)
+{
+    return ctx->nfields == 1 && !ctx->concurrent && !ctx->fh[0].slab && ctx->fh[0].phys.nc % 32 == 0;
+}
+
 // Persistent grid: `mult` times the resident blocks of the kernel, or (mult 0)
 // as many blocks as the work needs, which the hardware hands out as earlier
 // ones end; never more than the work needs.
@@ -197,7 +208,8 @@ gks::LaunchCfg persistent(gks_ctx *ctx, int kind, int dir, int variant, int mult
     c.block = kind == gks::K_UPDATE ? gks::kUpdateBlock : (kind == gks::K_FLUX ? gks::kFluxBlock : gks::kReconBlock);
     c.variant = variant;
     int per_sm = 1;
-    if (gks::max_resident_blocks(kind, dir, ctx->precision, variant, c.block, &per_sm) != cudaSuccess || per_sm < 1)
+    const bool update = kind == gks::K_FLUX && dir == 2 && update_with_flux(ctx);
+    if (gks::max_resident_blocks(kind, dir, ctx->precision, variant, c.block, update, &per_sm) != cudaSuccess || per_sm < 1)
         per_sm = 1;
     long long g = (long long)ctx->nsm * per_sm * mult;
     // threads: one per window run (x / y reconstruction), 32 per z line (z
@@ -258,23 +270,6 @@ std::string tune_key(const gks_ctx *ctx)
 
 int record_slab_step(gks_ctx *ctx);
 
-// Whether the z flux applies the update itself (k_flux_update): one field whose
-// sweeps run one after the other (with concurrent sweeps the x and y fluxes
-// still read the state) and whose z lines fill the warps' 32 lanes (at 250^3,
-// where 2.4 % of them idle, nothing is left of the gain).  us per step,
-// separate / with the flux, runs in turn: FP64 128^3 989 / 971, 256^3 7596 / 7469;
-// mixed 128^3 858 / 845, 256^3 6741 / 6605, 320^3 13265 / 12947, 512^3 55859 / 54205.
-bool update_with_flux(const gks_ctx *ctx)
-{
-    return ctx->nfields == 1 && ctx->fh[0].phys.nc % 32 == 0;
-}
-
-int launch_flux_update(gks_ctx *ctx)
-{
-    CK(gks::launch_flux_update(ctx->batch, ctx->precision, ctx->nsm, ctx->stream));
-    return GKS_OK;
-}
-
 int record_step(gks_ctx *ctx)
 {
     if (ctx->fh[0].slab) return record_slab_step(ctx);
@@ -301,7 +296,10 @@ int record_step(gks_ctx *ctx)
     }
     for (int dir = 0; dir < 3; ++dir) {
         CK(gks::launch_recon(ctx->batch, dir, ctx->precision, ctx->cfg[gks::K_RECON][dir], ctx->stream));
-        if (dir == 2 && update_with_flux(ctx)) return launch_flux_update(ctx);
+        if (dir == 2 && update_with_flux(ctx)) {
+            CK(gks::launch_flux_update(ctx->batch, ctx->precision, ctx->cfg[gks::K_FLUX][2], ctx->stream));
+            return GKS_OK;
+        }
         CK(gks::launch_flux(ctx->batch, dir, ctx->precision, ctx->cfg[gks::K_FLUX][dir], ctx->stream));
     }
     CK(gks::launch_update(ctx->batch, ctx->cfg[gks::K_UPDATE][0], ctx->stream));
@@ -1497,9 +1495,16 @@ int gks_autotune(gks_ctx *ctx, int reps)
     int rc = GKS_OK;
     // time `reps` launches of one candidate after one untimed launch; the
     // reconstruction and flux kernels only write scratch, so repeating them
-    // leaves the state unchanged (the update is not tuned for that reason)
+    // leaves the state unchanged (the update is not tuned for that reason); the z
+    // flux that applies the update writes the new state over the z flux's arrays,
+    // and reports on it to a word that nothing reads
+    gks::Batch scratch = ctx->batch;
+    for (int q = 0; q < 5; ++q) scratch.one.Wout[q] = scratch.one.F[10 + q];
+    scratch.err = reinterpret_cast<int *>(ctx->d_bits);
     auto time_it = [&](int kind, int dir, gks::LaunchCfg c, float *ms) -> cudaError_t {
         auto go = [&]() {
+            if (kind == gks::K_FLUX && dir == 2 && update_with_flux(ctx))
+                return gks::launch_flux_update(scratch, ctx->precision, c, ctx->stream);
             return kind == gks::K_RECON ? gks::launch_recon(ctx->batch, dir, ctx->precision, c, ctx->stream)
                                         : gks::launch_flux(ctx->batch, dir, ctx->precision, c, ctx->stream);
         };

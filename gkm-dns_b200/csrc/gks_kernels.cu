@@ -954,7 +954,8 @@ __global__ void __launch_bounds__(kUpdateBlock) k_update(Batch b)
 }
 
 // ---------------------------------------------------------------------------
-// z flux and update of one field in one kernel, in place.  A warp walks whole z
+// z flux and update of one field in one kernel, in place (or, to be timed, into
+// other arrays, Wout).  A warp walks whole z
 // lines (drawn from the queue of k_flux), 32 interfaces at a time: a lane's
 // lower z flux comes from the lane below by a shuffle, lane 0's from the chunk
 // before (park), and the x and y fluxes of its cell arrive by asynchronous
@@ -1039,7 +1040,7 @@ __global__ void __launch_bounds__(kFluxBlock) __maxnreg__(REGS) k_flux_update(Ba
                     first[q] = d;
                 } else if (k < nc) {
                     w[q] = __dsub_rn(w[q], __dmul_rn(f.inv_dx, __dsub_rn(d, lo)));
-                    f.W[q][c] = w[q];
+                    f.Wout[q][c] = w[q];
                 }
             }
             if (k > 0 && k < nc) bad = !physical(w, f.gm1);
@@ -1050,7 +1051,7 @@ __global__ void __launch_bounds__(kFluxBlock) __maxnreg__(REGS) k_flux_update(Ba
 #pragma unroll
             for (int q = 0; q < 5; ++q) {
                 w[q] = __dsub_rn(f.W[q][lbase], __dmul_rn(f.inv_dx, __dsub_rn(first[q], below[q])));
-                f.W[q][lbase] = w[q];
+                f.Wout[q][lbase] = w[q];
             }
             if (!physical(w, f.gm1)) atomicOr(b.err, 1);
         }
@@ -1507,6 +1508,26 @@ cudaError_t flux_go(Batch b, LaunchCfg cfg, cudaStream_t st)
     return cudaGetLastError();
 }
 
+template <int PREC>
+cudaError_t flux_update_go(const Batch &b, LaunchCfg cfg, cudaStream_t st)
+{
+    const int g = range_grid(cfg.grid, b.one.ncell / b.one.nc, cfg.block / 32);
+    switch (cfg.variant) {
+    case 1: k_flux_update<PREC, kFluxRegs[1]><<<g, cfg.block, 0, st>>>(b); break;
+    case 2: k_flux_update<PREC, kFluxRegs[2]><<<g, cfg.block, 0, st>>>(b); break;
+    default: k_flux_update<PREC, kFluxRegs[0]><<<g, cfg.block, 0, st>>>(b); break;
+    }
+    return cudaGetLastError();
+}
+
+template <int PREC>
+cudaError_t occ_flux_update(int variant, int block, int *n)
+{
+    if (variant == 1) return occ(k_flux_update<PREC, kFluxRegs[1]>, block, n);
+    if (variant == 2) return occ(k_flux_update<PREC, kFluxRegs[2]>, block, n);
+    return occ(k_flux_update<PREC, kFluxRegs[0]>, block, n);
+}
+
 template <int DIR, int PREC>
 cudaError_t occ_kind(int kind, int variant, int block, int *n)
 {
@@ -1555,21 +1576,15 @@ cudaError_t launch_update(const Batch &batch, LaunchCfg cfg, cudaStream_t st)
     return cudaGetLastError();
 }
 
-cudaError_t launch_flux_update(const Batch &b, int prec, int nsm, cudaStream_t st)
+cudaError_t launch_flux_update(const Batch &b, int prec, LaunchCfg cfg, cudaStream_t st)
 {
-    int per_sm = 1;
-    cudaError_t e = prec == 0 ? occ(k_flux_update<0, kFluxRegs[1]>, kFluxBlock, &per_sm) : occ(k_flux_update<1, kFluxRegs[1]>, kFluxBlock, &per_sm);
-    if (e != cudaSuccess) return e;
-    const long long lines = b.one.ncell / b.one.nc;
-    const int g = range_grid(nsm * std::max(per_sm, 1), lines, kFluxBlock / 32);
-    if (prec == 0) k_flux_update<0, kFluxRegs[1]><<<g, kFluxBlock, 0, st>>>(b);
-    else k_flux_update<1, kFluxRegs[1]><<<g, kFluxBlock, 0, st>>>(b);
-    return cudaGetLastError();
+    return prec == 0 ? flux_update_go<0>(b, cfg, st) : flux_update_go<1>(b, cfg, st);
 }
 
-cudaError_t max_resident_blocks(int kind, int dir, int prec, int variant, int block, int *n)
+cudaError_t max_resident_blocks(int kind, int dir, int prec, int variant, int block, bool update, int *n)
 {
     if (kind == K_UPDATE) return occ(k_update, block, n);
+    if (update) return prec == 0 ? occ_flux_update<0>(variant, block, n) : occ_flux_update<1>(variant, block, n);
     return prec == 0 ? occ_dir<0>(kind, dir, variant, block, n) : occ_dir<1>(kind, dir, variant, block, n);
 }
 

@@ -131,11 +131,13 @@ inline long long batch_items(const Batch &b, int kind, int dir)
 cudaError_t launch_recon(const Batch &b, int dir, int prec, LaunchCfg cfg, cudaStream_t st);
 cudaError_t launch_flux(const Batch &b, int dir, int prec, LaunchCfg cfg, cudaStream_t st);
 cudaError_t launch_update(const Batch &b, LaunchCfg cfg, cudaStream_t st);
-// The z flux and the update of a one-field batch together, in place (Wout == W).
-cudaError_t launch_flux_update(const Batch &b, int prec, int nsm, cudaStream_t st);
+// The z flux and the update of a one-field batch together (the new state to Wout,
+// which may be W); cfg is that of the z flux.
+cudaError_t launch_flux_update(const Batch &b, int prec, LaunchCfg cfg, cudaStream_t st);
 
-// Resident blocks per SM of a kernel kind / variant (for persistent grids).
-cudaError_t max_resident_blocks(int kind, int dir, int prec, int variant, int block, int *blocks_per_sm);
+// Resident blocks per SM of a kernel kind / variant (for persistent grids); with
+// `update`, of the z flux that applies the update.
+cudaError_t max_resident_blocks(int kind, int dir, int prec, int variant, int block, bool update, int *blocks_per_sm);
 
 // Layout conversion of one field: padded host layout (5 x nty x nt^2, contiguous,
 // nt = nc + 6, nty = ny + 2 yhost) <-> device layout.  gather fills the device

@@ -239,7 +239,10 @@ int gks_time_stages(gks_ctx *ctx, int reps, double *ms);
 int gks_autotune(gks_ctx *ctx, int reps);
 
 /* The launch configuration in use: kind 0 reconstruction, 1 flux, 2 update;
- * dir 0..2 = x, y, z. */
+ * dir 0..2 = x, y, z.  Where gks_step applies the update inside the z flux (one
+ * field of more than 2^20 cells whose nc is a multiple of 32), that kernel runs
+ * with the z flux's configuration, which is also the one the tuner times; the
+ * update's then holds for gks_evolve and gks_time_stages only. */
 int gks_get_launch(gks_ctx *ctx, int kind, int dir, int *block, int *grid, int *variant);
 
 /* Pin the launch configuration of one kernel kind and sweep (for example to

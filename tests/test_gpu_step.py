@@ -724,3 +724,60 @@ def test_step_is_refused_on_the_legacy_stream_and_the_host_step_is_not(gks):
                     s.evolve(host)
                 out.append(host)
         assert np.array_equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+def test_z_flux_with_update_runs_the_pinned_launch(gks, prec):
+    """Where gks_step takes the update inside the z flux, the z flux's launch
+    configuration holds for that kernel: one block takes far longer than a wave
+    of them."""
+    import torch
+
+    case = gks_ic.make_dhit(128, k0=4.0, Mt=0.3, seed=2)
+    with gks.Solver(gks.phys_from_case(case), gks.FP64 if prec == "fp64" else gks.MIXED) as s:
+        s.upload(gks_ic.to_conservative_padded(case))
+        s.timestep(0.5)
+        stream = torch.cuda.ExternalStream(s.stream())
+
+        def ms():
+            s.step(1)
+            s.sync()
+            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            ev[0].record(stream)
+            s.step(1)
+            ev[1].record(stream)
+            s.sync()
+            return ev[0].elapsed_time(ev[1])
+
+        wave = ms()
+        s.set_launch("flux", 2, s.launch_config()["flux_z"]["variant"], grid=1)
+        assert ms() > 10 * wave
+
+
+@pytest.mark.parametrize("prec", ["fp64", "mixed"])
+@pytest.mark.parametrize("flags", [0, 1, 2, 3])
+def test_z_flux_with_update_in_every_variant_and_tuned(gks, prec, flags):
+    """The z flux that applies the update: every register cap, a grid that is no
+    multiple of anything, every option, against the stages launched one by one;
+    the tuner, which times that kernel, leaves the state as it was."""
+    case = gks_ic.make_dhit(128, k0=4.0, Mt=0.5, seed=5)
+    W = gks_ic.to_conservative_padded(case)
+    with gks.Solver(gks.phys_from_case(case), gks.FP64 if prec == "fp64" else gks.MIXED, flags) as s:
+        s.upload(W)
+        s.timestep(0.5)
+        s.time_stages(2)
+        s.sync()
+        want = s.download()
+        for variant, grid in ((0, 0), (1, 101), (2, 0)):
+            s.set_launch("flux", 2, variant, grid=grid)
+            s.upload(W)
+            s.step(2)
+            s.sync()
+            assert np.array_equal(s.download(), want)
+        s.upload(W)
+        s.autotune(1)
+        s.sync()
+        assert np.array_equal(s.download(), W)
+        s.step(2)
+        s.sync()
+        assert np.array_equal(s.download(), want)
