@@ -77,7 +77,7 @@ struct gks_ctx {
     size_t stage_out_elems = 0;
     cudaStream_t h2d = nullptr, d2h = nullptr;
     std::vector<cudaEvent_t> ev_in, ev_out;
-    double *d_partial = nullptr;
+    double *d_partial = nullptr; // one allocation with the four below
     double *d_sums = nullptr;
     unsigned long long *d_bits = nullptr;
     int *d_err = nullptr;
@@ -714,9 +714,7 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
         return rc;
     };
     if (cudaGetDevice(&ctx->device) != cudaSuccess) return bail(GKS_ECUDA);
-    cudaDeviceProp prop;
-    if (cudaGetDeviceProperties(&prop, ctx->device) != cudaSuccess) return bail(GKS_ECUDA);
-    ctx->nsm = prop.multiProcessorCount;
+    if (cudaDeviceGetAttribute(&ctx->nsm, cudaDevAttrMultiProcessorCount, ctx->device) != cudaSuccess) return bail(GKS_ECUDA);
     if (cudaStreamCreateWithFlags(&ctx->stream, cudaStreamNonBlocking) != cudaSuccess) return bail(GKS_ECUDA);
     ctx->own_stream = true;
 
@@ -747,7 +745,10 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
         const long long r0 = (5 * n + 1) & ~1LL, nrec = ctx->concurrent ? 30 : 10;
         const size_t elems = (size_t)(r0 + (nrec + 17) * n);
         if (cudaMalloc(&h.mem, elems * sizeof(double)) != cudaSuccess) return bail(GKS_ENOMEM);
-        if (cudaMemset(h.mem, 0, elems * sizeof(double)) != cudaSuccess) return bail(GKS_ECUDA);
+        // (the y and z sweeps' own reconstruction buffers are written before they are read)
+        if (cudaMemset(h.mem, 0, (r0 + 10 * n) * sizeof(double)) != cudaSuccess ||
+            cudaMemset(h.mem + r0 + nrec * n, 0, 17 * n * sizeof(double)) != cudaSuccess)
+            return bail(GKS_ECUDA);
         FieldDev &d = h.dev;
         memset(&d, 0, sizeof(d));
         for (int q = 0; q < 5; ++q) d.W[q] = d.Wout[q] = h.mem + q * n;
@@ -840,14 +841,14 @@ int create_ctx(gks_ctx **out, int nfields, const gks_phys *phys, int precision, 
     for (int f = 0; f < nfields; ++f)
         if (cudaMemcpy(ctx->d_fields + f, &ctx->fh[f].dev, sizeof(FieldDev), cudaMemcpyHostToDevice) != cudaSuccess)
             return bail(GKS_ECUDA);
-    if (cudaMalloc(&ctx->d_partial, gks::stats_partial_elems(ctx->nsm) * sizeof(double)) != cudaSuccess)
-        return bail(GKS_ENOMEM);
-    if (cudaMalloc(&ctx->d_sums, 32 * sizeof(double)) != cudaSuccess) return bail(GKS_ENOMEM);
-    if (cudaMalloc(&ctx->d_bits, sizeof(unsigned long long)) != cudaSuccess) return bail(GKS_ENOMEM);
-    if (cudaMalloc(&ctx->d_err, sizeof(int)) != cudaSuccess) return bail(GKS_ENOMEM);
-    if (cudaMemset(ctx->d_err, 0, sizeof(int)) != cudaSuccess) return bail(GKS_ECUDA);
-    if (cudaMalloc(&ctx->d_queue, 6 * sizeof(unsigned)) != cudaSuccess) return bail(GKS_ENOMEM);
-    if (cudaMemset(ctx->d_queue, 0, 6 * sizeof(unsigned)) != cudaSuccess) return bail(GKS_ECUDA);
+    // the small buffers in one allocation, each from a 256-byte line of its own
+    const size_t line = 32, partial = (gks::stats_partial_elems(ctx->nsm) + line - 1) / line * line;
+    if (cudaMalloc(&ctx->d_partial, (partial + 4 * line) * sizeof(double)) != cudaSuccess) return bail(GKS_ENOMEM);
+    ctx->d_sums = ctx->d_partial + partial;
+    ctx->d_bits = reinterpret_cast<unsigned long long *>(ctx->d_sums + line);
+    ctx->d_err = reinterpret_cast<int *>(ctx->d_sums + 2 * line);
+    ctx->d_queue = reinterpret_cast<unsigned *>(ctx->d_sums + 3 * line);
+    if (cudaMemset(ctx->d_bits, 0, 3 * line * sizeof(double)) != cudaSuccess) return bail(GKS_ECUDA);
     ctx->batch.queue = ctx->d_queue;
     ctx->batch.fields = ctx->d_fields;
     ctx->batch.nfields = nfields;
@@ -958,10 +959,6 @@ void gks_destroy(gks_ctx *ctx)
     if (ctx->h2d) cudaStreamDestroy(ctx->h2d);
     if (ctx->d2h) cudaStreamDestroy(ctx->d2h);
     if (ctx->d_partial) cudaFree(ctx->d_partial);
-    if (ctx->d_sums) cudaFree(ctx->d_sums);
-    if (ctx->d_bits) cudaFree(ctx->d_bits);
-    if (ctx->d_err) cudaFree(ctx->d_err);
-    if (ctx->d_queue) cudaFree(ctx->d_queue);
     for (int i = 0; i < 2; ++i) {
         if (ctx->side[i]) cudaStreamDestroy(ctx->side[i]);
         if (ctx->fork[i]) cudaEventDestroy(ctx->fork[i]);

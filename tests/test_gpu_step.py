@@ -781,3 +781,27 @@ def test_z_flux_with_update_in_every_variant_and_tuned(gks, prec, flags):
         s.step(2)
         s.sync()
         assert np.array_equal(s.download(), want)
+
+
+@pytest.mark.parametrize("sizes", [[24], [101], [10, 33]])
+def test_captured_sweeps_side_by_side_equal_the_stages(gks, sizes):
+    """A small context's captured step runs its sweeps side by side; the first
+    steps and the stages one by one run them in turn: the same bits, also across a
+    new dt, which has the step captured again."""
+    cases = [gks_ic.make_dhit(n, k0=min(4.0, n / 4), Mt=0.4, seed=n) for n in sizes]
+    for prec in (gks.FP64, gks.MIXED):
+        out = []
+        for staged in (False, True):
+            with gks.Solver([gks.phys_from_case(c) for c in cases], prec) as s:
+                for f, c in enumerate(cases):
+                    s.upload(gks_ic.to_conservative_padded(c), f)
+                for dt in (0.01, 0.005):
+                    for f in range(len(cases)):
+                        s.set_dt(dt, f)
+                    if staged:
+                        s.time_stages(20)
+                    else:
+                        s.step(20)
+                s.sync()
+                out.append([s.download(f) for f in range(len(cases))])
+        assert all(np.array_equal(a, b) for a, b in zip(*out))
