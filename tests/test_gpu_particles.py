@@ -247,3 +247,18 @@ def test_particles_at_group_edges(gks, oracle, nc, n):
         s.particles_locate(x0, y0, z0)
         s.particles_props()
         assert np.array_equal(s.particles_get(), want)
+
+
+def test_particles_after_the_slab_form_of_the_host_step(gks, oracle):
+    """gks_evolve of a field that goes up in slabs swaps the state's buffers: the
+    particles then see the new state."""
+    case, W, x0, y0, z0 = setup(60, 4, 500)
+    with gks.Solver(gks.phys_from_case(case)) as s:
+        s.upload(W)
+        s.timestep(0.5)
+        s.particles_locate(x0, y0, z0)
+        host = W.copy()
+        s.evolve(host)
+        s.particles_props()
+        _, want = oracle_records(oracle, case, host, x0, y0, z0)
+        assert np.array_equal(s.particles_get(), want)
