@@ -224,8 +224,8 @@ gks::LaunchCfg persistent(gks_ctx *ctx, int kind, int dir, int variant, int mult
 
 // The untuned grid of a variant: the flux and the update one wave of blocks, the
 // reconstruction all its blocks (a wave of persistent blocks ends unevenly: 256^3
-// x / y / z, FP64 694 / 627 / 680 -> 670 / 601 / 634 us when this was chosen, mixed 533 /
-// 511 / 501 -> 502 / 465 / 458).
+// x / y / z, one wave against all blocks, FP64 672 / 612 / 657 against 595 / 547 / 592 us,
+// mixed 578 / 517 / 541 against 506 / 453 / 448).
 gks::LaunchCfg default_launch(gks_ctx *ctx, int kind, int dir, int variant)
 {
     return persistent(ctx, kind, dir, variant, kind == gks::K_RECON ? 0 : 1);
@@ -233,8 +233,7 @@ gks::LaunchCfg default_launch(gks_ctx *ctx, int kind, int dir, int variant)
 
 // Untuned defaults: the flux at the 168-register cap (6 blocks of 64 threads per
 // SM), the reconstruction at its natural register count but for the FP64 z sweep,
-// which the 96-register cap (20 warps per SM, 40 B spill) serves best (663 us at
-// 150 registers against 634).
+// which the 96-register cap (20 warps per SM, 40 B spill) serves best (594 us at 256^3 against 603 and 602).
 void choose_launch(gks_ctx *ctx)
 {
     for (int kind = 0; kind < gks::K_KINDS; ++kind)

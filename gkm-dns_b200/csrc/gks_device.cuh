@@ -58,6 +58,19 @@ __device__ __forceinline__ f2 fmaxT(f2 a, f2 b) { return f2(fmaxf(a.v.x, b.v.x),
 template <typename T> __device__ __forceinline__ constexpr T cst(double x) { return T(x); }
 template <> __device__ __forceinline__ f2 cst<f2>(double x) { return f2(float(x)); }
 
+// Asynchronous 8-byte copy global -> shared (cp.async), its groups and waits.
+__device__ __forceinline__ void cp_async8(double *smem, const double *gmem)
+{
+    const unsigned a = unsigned(__cvta_generic_to_shared(smem));
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a), "l"(gmem) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait()
+{
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
+}
+
 // 1/x from the hardware's approximation y (rcp.approx.ftz.f64, good to about 20
 // bits) and one third-order step: with e = 1 - x y, 1/x = y / (1 - e), of whose
 // geometric series y (1 + e + e^2) is taken.  Three fused multiply-adds and no
@@ -102,7 +115,8 @@ __device__ __forceinline__ double rsqrt_cubic(double x)
 // indicators and weight products are formed once for the two states: about 75
 // operations per cell and component instead of the 134 of an interface whose
 // two sides are formed from cell values (FP64 reconstruction at 256^3: x 952
-// -> 704, y 893 -> 629, z 955 -> 683 us).  The two states stay independent
+// -> 704, y 893 -> 629, z 955 -> 683 us, with the launch forms of gks_kernels.cu 597 /
+// 547 / 592).  The two states stay independent
 // (d[0] enters only the right one, d[5] only the left one), so that a range
 // of interfaces can be reconstructed from the cells its own stencils reach.
 __device__ __forceinline__ void weno_cell(const double (&d)[6], double &dl, double &dr)

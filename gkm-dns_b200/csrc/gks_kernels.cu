@@ -239,19 +239,6 @@ __device__ __forceinline__ void interface_states(const SG &s, bool direct, doubl
     wr[4] = energy(wr, wr[4], wl[0] * r, icT);
 }
 
-// Asynchronous 8-byte copy global -> shared (cp.async), its groups and waits.
-__device__ __forceinline__ void cp_async8(double *smem, const double *gmem)
-{
-    const unsigned a = unsigned(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(a), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait()
-{
-    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
-}
-
 // The last field whose range (FieldDev::*BASE) starts at or before item `it`, the
 // same item range for all 32 lanes: each round splits the fields left into 32
 // parts, a lane looking at the start of one, so up to 32 fields take one load's

@@ -32,6 +32,7 @@
 // q of particle a at q * n + a, so that a warp's accesses are coalesced):
 // position (y, x, z) = the reference's pos[0..2], DEN, U[0..2] = (u, v, w),
 // P, and the gradients (d/dy, d/dx, d/dz) of DEN, u, v, w and P.
+#include "gks_device.cuh"
 #include "gks_kernels.cuh"
 #include "../../include/gks_b200.h"
 
@@ -293,21 +294,6 @@ __global__ void __launch_bounds__(kZThreads) k_prims_zlines(FieldDev f, double *
     }
 }
 
-// Asynchronous 8-byte copy global -> shared, its groups and waits.
-__device__ __forceinline__ void cp_async8(double *smem, const double *gmem)
-{
-    const unsigned a = unsigned(__cvta_generic_to_shared(smem));
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\
-" ::"r"(a), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\
-" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait()
-{
-    asm volatile("cp.async.wait_group %0;\
-" ::"n"(N) : "memory");
-}
-
 // ---------------------------------------------------------------------------
 // Short lines stay in shared memory between their two recurrences, so that a
 // pass reads and writes the array once, and an SM holds enough of them (100 of
@@ -487,7 +473,7 @@ __device__ __forceinline__ void bspline_weights(double t, double b[8])
 // along z innermost).  Bound: latency of random reads, 16 rows of 160 B a
 // particle (4.3 GB of DRAM traffic for 2^20 particles at 256^3).  Measured there:
 // a thread per particle (254 registers, 8 warps per SM) 1.65 ms, this form
-// 0.69 ms; visiting the particles tile by tile of the grid 0.88 ms and a sort
+// 0.71 ms; visiting the particles tile by tile of the grid 0.88 ms and a sort
 // (their records are then scattered).
 constexpr int kPropWarps = 4, kPropParticles = 6;
 
