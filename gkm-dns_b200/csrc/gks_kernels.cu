@@ -363,7 +363,7 @@ __device__ __forceinline__ void recon_zlines(const Batch &b, double (&tiles)[kZL
 // FP64 reads a one-field batch's descriptor from the launch parameters (x and y
 // windows and z lines): from memory, every asynchronous copy, a memory barrier
 // to the compiler, has the pointers and constants loaded again.  us per sweep at
-// 256^3, x / y / z: 625 / 554 / 607 -> 599 / 548 / 595; 130^3 111 / 97 / 109 -> 106 /
+// 256^3, x / y / z: 625 / 554 / 607 -> 597 / 547 / 592; 130^3 111 / 97 / 109 -> 106 /
 // 96 / 105.  Mixed needs more registers with two loops in a kernel (120 -> 138; y
 // 454 -> 469, z 448 -> 457 us) and keeps one.
 template <int PREC, int MINB>
@@ -833,8 +833,8 @@ __device__ __forceinline__ void flux_item(const FieldDev &f, unsigned c, FluxPar
 // the next ones come from a counter in global memory, asked for one chunk
 // ahead.  (With equal static shares the schedulers run some warps ahead of
 // others and an SM's last fifth passes at falling occupancy: 9.7 of 12 warps
-// active on average, 11.8 with the queue; 1677 -> 1572 us per sweep at 256^3,
-// 1548 with a loop of its own for one field and for an ensemble.  The mixed
+// active on average, 11.9 with the queue; 1677 -> 1572 us per sweep at 256^3,
+// 1543 with a loop of its own for one field and for an ensemble.  The mixed
 // kernel gains nothing, 1466 -> 1515 us.)  The warp that is last to find the
 // queue empty sets the counters back to zero for the next launch.
 template <int DIR, bool ENSEMBLE>
@@ -1285,7 +1285,7 @@ __device__ __forceinline__ void add_sums(const FieldDev &f, long long c, const d
 // pass, last, adds every cell's terms straight from its tiles and the six
 // slopes before (partial: NSUM1 sums per block; kout: the shifts K), one wave
 // of blocks over all sets of lines.  HBM: 56 B a cell and pass for y and x, 88 B
-// for z and the sums (3.4 GB at 256^3, 0.51 ms); measured 275 + 272 + 532 us, a
+// for z and the sums (3.4 GB at 256^3, 0.51 ms); measured 274 + 269 + 524 us, a
 // block's load, solve and store phases only partly covered by the other's.
 // Before: a warp per line (affine-map scans, 40 instructions a node) and sums of
 // their own, 327 + 317 + 267 + 362 us.  Measured alternatives: 8 lines and 128
