@@ -637,7 +637,7 @@ def test_many_small_fields_equal_individual_runs(gks, nfields):
 @pytest.mark.parametrize("nc", [275, 283])
 def test_stats_cost_per_cell_has_no_step_at_longer_lines(gks, nc):
     """Lines a little longer than 256^3's still leave two blocks of every pass on
-    an SM; with one, a cell costs 1.4 times as much."""
+    an SM (a cell costs 1.17-1.19 times as much as at 256^3); with one, 1.4 times."""
     import time
 
     def ns_per_cell(n):
@@ -656,7 +656,7 @@ def test_stats_cost_per_cell_has_no_step_at_longer_lines(gks, nc):
                 best = min(best, time.perf_counter() - t)
         return best / n**3
 
-    assert ns_per_cell(nc) < 1.2 * ns_per_cell(256)
+    assert ns_per_cell(nc) < 1.3 * ns_per_cell(256)
 
 
 def test_grid_zero_pins_the_default_grid(gks):
